@@ -136,7 +136,7 @@ struct __align__(16) Slot4 {
     uint64_t w0, w1, w2, w3;
     uint32_t count;
     uint32_t state;
-    uint64_t mark;  // merged-histogram mark (hist_* kernels)
+    uint64_t mark;  // unused, zero: keeps the slot a multiple of 16 bytes
 };
 struct __align__(32) Slot2 {
     uint64_t w0, w1;
@@ -1878,13 +1878,17 @@ __global__ void __launch_bounds__(EXP_THREADS) export_write_bits(const void* tab
 // Device form of tool/histogram_tool.cpp "precise"
 // (tool/HighFrequencyInsertThreadPool.h:150-177,
 // tool/LowFrequencyQueryThreadPool.h:375-432): exact count of a key = its
-// table count + [key in low.bin].  Pass 1 walks the packed low.bin keys,
-// looks each up in its bucket's table, marks the slot (pad field) and adds
-// count+1 (or 1) to the histogram; pass 2 adds every unmarked table key with
-// its table count.  Histogram bins are aggregated per CTA in shared memory
-// (HIST_SMEM bins; larger counts go straight to global atomics).
+// table count + [key in low.bin].  A key is in low.bin at most once, so the
+// histogram is a sum in any order: +1 at its count for every table key; for
+// every low.bin key +1 at count 1 when no table holds it, else -1 at its
+// table count and +1 at the next.  Nothing is written to the tables.  Keys in
+// low.bin order visit a bucket's table at random, so a low.bin key is looked
+// up where its table slice is at hand: in shared memory, window by window,
+// after a windowed count (hist_window in kc_window.cuh), else in L2.
+// Histogram bins are aggregated per CTA in shared memory (HIST_SMEM bins;
+// larger counts go straight to global atomics).
 
-constexpr int HIST_SMEM = 1024;
+constexpr int HIST_SMEM = 512;
 
 // Key of low.bin record r (layout of src/ExportWriter.h:522-550, read back as
 // tool/ExportReader.h:355-391 does).  Records of a multiple of 8 bytes
@@ -1909,175 +1913,291 @@ __device__ __forceinline__ typename KeyOf<NW>::T unpack_low(const uint8_t* low, 
     return key;
 }
 
+// The same with at most NW + 1 aligned word loads for any record size: the
+// buffer must be readable for 8 (NW + 1) bytes from the word a record starts
+// in (the context's packed low.bin buffer keeps 64 bytes after its last one).
 template <int NW>
-__device__ __forceinline__ bool table_find(const typename SlotOf<NW>::T* tab, uint64_t mask, uint64_t h,
-                                           const typename KeyOf<NW>::T& key, uint64_t* where) {
-    const uint64_t i0 = (h >> 17) & mask;
-    for (uint64_t p = 0; p <= mask; ++p) {
-        const uint64_t i = (i0 + p) & mask;
-        const typename SlotOf<NW>::T& s = tab[i];
-        bool empty, eq;
-        if constexpr (NW == 1) {
-            empty = s.key == EMPTY;
-            eq = s.key == key;
-        } else if constexpr (NW == 2) {
-            empty = s.w0 == EMPTY && s.w1 == EMPTY;
-            eq = s.w0 == key.w0 && s.w1 == key.w1;
-        } else {
-            empty = s.state != SLOT_READY;  // after the count every used slot is ready
-            eq = !empty && s.w0 == key.w0 && s.w1 == key.w1 && s.w2 == key.w2 && s.w3 == key.w3;
+__device__ __forceinline__ typename KeyOf<NW>::T load_low(const uint8_t* __restrict__ low, uint64_t r, uint32_t P,
+                                                          uint32_t full, uint32_t tail_bytes) {
+    uint64_t w[NW];
+    const uint64_t a = r * P;
+    const uint64_t* q = reinterpret_cast<const uint64_t*>(low) + (a >> 3);
+    const uint32_t sh = (uint32_t)(a & 7) * 8;
+    if (P == 8 * NW) {
+#pragma unroll
+        for (int i = 0; i < NW; ++i) w[i] = __ldcs(q + i);
+    } else {
+        uint64_t x[NW + 1];
+#pragma unroll
+        for (int i = 0; i <= NW; ++i) x[i] = __ldg(q + i);
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            const uint64_t v = sh ? (x[i] >> sh) | (x[i + 1] << (64 - sh)) : x[i];
+            w[i] = (uint32_t)i < full ? v : ((uint32_t)i == full && tail_bytes ? v << (64 - 8 * tail_bytes) : 0ull);
         }
-        if (eq) {
-            *where = i;
-            return true;
-        }
-        if (empty) return false;
     }
-    return false;
+    if constexpr (NW == 1) return w[0];
+    else if constexpr (NW == 2) return Key2{w[0], w[1]};
+    else return Key4{w[0], w[1], w[2], w[3]};
 }
 
-__device__ __forceinline__ void hist_add(uint32_t* sh, unsigned long long* gh, uint64_t merged, uint32_t lo,
+// Table lookups.  A key is stored at most PROBE_LIMIT - 1 cells after its
+// first one, with no EMPTY cell in between.
+template <int NW>
+struct Cell {  // what one probe reads
+    typename KeyOf<NW>::T key;
+    uint32_t count;  // 256-bit cells: read only when the key matches
+    bool used;
+};
+template <int NW>
+__device__ __forceinline__ Cell<NW> read_cell_all(const typename SlotOf<NW>::T* s) {
+    Cell<NW> c;
+    if constexpr (NW == 1) {
+        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(s));
+        c.key = ((uint64_t)v.y << 32) | v.x;
+        c.count = v.z;
+        c.used = c.key != EMPTY;
+    } else if constexpr (NW == 2) {
+        const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2*>(s));
+        c.key = Key2{v.x, v.y};
+        c.count = 0;
+        c.used = !(v.x == EMPTY && v.y == EMPTY);
+    } else {
+        const ulonglong2 a = __ldcg(reinterpret_cast<const ulonglong2*>(s));
+        const ulonglong2 b = __ldcg(reinterpret_cast<const ulonglong2*>(s) + 1);
+        const uint2 t = __ldcg(reinterpret_cast<const uint2*>(s) + 4);
+        c.key = Key4{a.x, a.y, b.x, b.y};
+        c.count = t.x;
+        c.used = t.y == SLOT_READY;  // after the count every used slot is ready
+    }
+    return c;
+}
+__device__ __forceinline__ bool same_key(uint64_t a, uint64_t b) { return a == b; }
+__device__ __forceinline__ bool same_key(const Key2& a, const Key2& b) { return a.w0 == b.w0 && a.w1 == b.w1; }
+__device__ __forceinline__ bool same_key(const Key4& a, const Key4& b) {
+    return a.w0 == b.w0 && a.w1 == b.w1 && a.w2 == b.w2 && a.w3 == b.w3;
+}
+
+// `add` keys of exact count `merged` (add may be -1: bins and totals are
+// two's complement sums).
+__device__ __forceinline__ void hist_add(uint32_t* sh, unsigned long long* gh, uint64_t merged, int add, uint32_t lo,
                                          uint32_t hi) {
-    // the active lanes of the warp that share a shared-memory bin add once
-    // (nearly every low.bin key lands in the bin of count 1, and shared-memory
-    // atomics on one address are serialised)
-    const bool in = merged >= lo && merged <= hi;
+    if (merged < lo || merged > hi) return;
     const uint64_t bin = merged - lo;
-    const uint32_t key = in && bin < HIST_SMEM ? (uint32_t)bin : 0xFFFFFFFFu;
-    const uint32_t same = __match_any_sync(__activemask(), key);
-    if (key != 0xFFFFFFFFu) {
-        if ((int)(__ffs(same) - 1) == (int)(threadIdx.x & 31)) atomicAdd(sh + key, (uint32_t)__popc(same));
-    } else if (in) {
-        atomicAdd(gh + bin, 1ull);
-    }
+    if (bin < HIST_SMEM) atomicAdd(sh + bin, (uint32_t)add);
+    else atomicAdd(gh + bin, (unsigned long long)(long long)add);
+}
+__device__ __forceinline__ void hist_flush(const uint32_t* sh, unsigned long long* gh, uint32_t lo, uint32_t hi) {
+    for (int i = threadIdx.x; i < HIST_SMEM; i += blockDim.x)
+        if (sh[i] && (uint64_t)lo + i <= hi) atomicAdd(gh + i, (unsigned long long)(long long)(int)sh[i]);
 }
 
-template <int NW>
-__global__ void hist_clear_marks(void* table, uint64_t n_slots) {
-    using S = typename SlotOf<NW>::T;
-    S* t = reinterpret_cast<S*>(table);
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_slots; i += (uint64_t)gridDim.x * blockDim.x) {
-        if constexpr (NW == 1) t[i].pad = 0;
-        else if constexpr (NW == 2) t[i].pad[0] = 0;
-        else t[i].mark = 0;
+// Table placement of a bucket in 16 bytes.
+struct TabRef {
+    uint64_t off, mask;
+};
+// The buckets' table placements in shared memory when there are at most 256
+// of them (a lookup per key through L1 otherwise).
+struct TabRefs {
+    const BucketMeta* meta;
+    const TabRef* sm;
+    __device__ __forceinline__ TabRef operator()(uint32_t b) const {
+        return sm ? sm[b] : TabRef{__ldg(&meta[b].tab_off), __ldg(&meta[b].tab_mask)};
     }
+};
+constexpr uint32_t TABREF_SMEM = 256;
+__device__ __forceinline__ TabRefs tab_refs(const BucketMeta* meta, uint32_t n_buckets, TabRef* sm) {
+    if (n_buckets > TABREF_SMEM) return TabRefs{meta, nullptr};
+    for (uint32_t b = threadIdx.x; b < n_buckets; b += blockDim.x) sm[b] = TabRef{meta[b].tab_off, meta[b].tab_mask};
+    return TabRefs{meta, sm};  // the caller's __syncthreads publishes sm
 }
 
+// Items a lane of the lookup kernels resolves side by side: the next record
+// and the first cell of each are in flight together.
 template <int NW>
-__global__ void hist_low_pass(const uint8_t* low, uint64_t n_low, uint32_t k, const BucketMeta* meta,
-                              uint32_t bucket_shift, void* table, uint32_t lo, uint32_t hi,
-                              unsigned long long* gh) {
+constexpr int lookup_items() {
+    return NW == 4 ? 1 : 2;
+}
+
+// Calls found(key, count) for every low.bin record [r0, r1) that its bucket's
+// table holds and returns how many this thread found.  A warp probes in
+// lockstep rounds (the vote ends a round for all its lanes): left to itself
+// the compiler lets lanes that leave the probe loop early run the rest of it
+// apart, which cost 940 warp instructions per 32 keys of 128 bits where the
+// rounds take about 200.
+template <int NW, class F>
+__device__ __forceinline__ uint32_t lookup_low(const uint8_t* __restrict__ low, uint64_t r0, uint64_t r1, uint32_t k,
+                                               uint32_t bucket_shift, const TabRefs& refs,
+                                               const typename SlotOf<NW>::T* __restrict__ table, F found) {
     using K = typename KeyOf<NW>::T;
     using S = typename SlotOf<NW>::T;
-    __shared__ uint32_t sh[HIST_SMEM];
-    for (int i = threadIdx.x; i < HIST_SMEM; i += blockDim.x) sh[i] = 0;
-    __syncthreads();
-    const uint32_t full = k / 32, tail_bits = 2 * (k % 32), tail_bytes = (tail_bits + 7) / 8;
-    const uint32_t P = full * 8 + tail_bytes;
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_low; r += (uint64_t)gridDim.x * blockDim.x) {
-        const K key = unpack_low<NW>(low, r, P, full, tail_bytes);
-        const BucketMeta m = meta[key_hi(key) >> bucket_shift];
-        S* tab = reinterpret_cast<S*>(table) + m.tab_off;
-        uint64_t at;
-        uint64_t merged = 1;
-        if (table_find<NW>(tab, m.tab_mask, hash_key(key), key, &at)) {
-            merged = (uint64_t)tab[at].count + 1;
-            if constexpr (NW == 1) tab[at].pad = 1;
-            else if constexpr (NW == 2) tab[at].pad[0] = 1;
-            else tab[at].mark = 1;
+    constexpr int IT = lookup_items<NW>();
+    const uint32_t full = k / 32, tail_bytes = (2 * (k % 32) + 7) / 8, P = full * 8 + tail_bytes;
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t n = 0;
+    // r: the warp's first record of the round
+    for (uint64_t r = r0 + (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); r < r1; r += step * IT) {
+        K key[IT];
+        const S* tab[IT];
+        uint32_t at[IT], mask[IT];
+        Cell<NW> c[IT];
+        uint32_t todo = 0, hit = 0;
+#pragma unroll
+        for (int j = 0; j < IT; ++j) {
+            const uint64_t i = r + j * step + lane;
+            if (i < r1) {
+                key[j] = load_low<NW>(low, i, P, full, tail_bytes);
+                todo |= 1u << j;
+            }
         }
-        hist_add(sh, gh, merged, lo, hi);
+#pragma unroll
+        for (int j = 0; j < IT; ++j)
+            if ((todo >> j) & 1u) {
+                const TabRef t = refs((uint32_t)(key_hi(key[j]) >> bucket_shift));
+                tab[j] = table + t.off;
+                mask[j] = (uint32_t)t.mask;  // a bucket holds fewer than 2^32 cells
+                at[j] = (uint32_t)(hash_key(key[j]) >> 17) & mask[j];
+                c[j] = read_cell_all<NW>(tab[j] + at[j]);
+            }
+        for (uint32_t p = 0;; ++p) {
+#pragma unroll
+            for (int j = 0; j < IT; ++j) {
+                if (!((todo >> j) & 1u)) continue;
+                const bool eq = c[j].used && same_key(c[j].key, key[j]);
+                if (eq) hit |= 1u << j;
+                if (eq || !c[j].used || p >= min((uint32_t)PROBE_LIMIT - 1, mask[j])) todo &= ~(1u << j);
+            }
+            if (!__any_sync(0xffffffffu, todo != 0)) break;  // warp-uniform
+#pragma unroll
+            for (int j = 0; j < IT; ++j)
+                if ((todo >> j) & 1u) {
+                    at[j] = (at[j] + 1) & mask[j];
+                    c[j] = read_cell_all<NW>(tab[j] + at[j]);
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < IT; ++j)
+            if ((hit >> j) & 1u) {
+                if constexpr (NW == 2) c[j].count = __ldcg(&tab[j][at[j]].count);
+                found(key[j], c[j].count);
+                ++n;
+            }
+        __syncwarp();
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < HIST_SMEM; i += blockDim.x)
-        if (sh[i]) atomicAdd(gh + i, (unsigned long long)sh[i]);
+    return n;
 }
 
+// Sum of v over the block, added to *out by one thread.
+__device__ __forceinline__ void block_add(unsigned long long* out, long long v, unsigned long long* s_sum) {
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0 && v) atomicAdd(s_sum, (unsigned long long)v);
+    __syncthreads();
+    if (threadIdx.x == 0 && *s_sum) atomicAdd(out, *s_sum);
+}
+
+// First low.bin record of output segment `seg` of a batch whose segments'
+// record offsets are prefix[0..nsegs) and that holds n_low records.
+__device__ __forceinline__ uint64_t low_at(const uint64_t* prefix, uint64_t nsegs, uint64_t seg, uint64_t n_low) {
+    return seg < nsegs ? prefix[seg] : n_low;
+}
+
+// Low.bin records of the segments from first_seg on (0 without a prefix: all
+// n_low records): histogram changes of those some table holds, +1 at count 1
+// for the others.  extra -= the number found (distinct keys = low.bin keys +
+// table keys - found).
 template <int NW>
-__global__ void hist_table_pass(const void* table, const ExportChunk* chunks, uint64_t n_chunks, uint32_t lo, uint32_t hi,
-                                unsigned long long* gh, unsigned long long* unmarked) {
+__global__ void __launch_bounds__(256, 6) hist_low_pass(const uint8_t* low, uint64_t n_low, const uint64_t* prefix,
+                                                        uint64_t nsegs, uint64_t first_seg, uint32_t k,
+                                                        const BucketMeta* meta, uint32_t n_buckets,
+                                                        uint32_t bucket_shift, const void* table, uint32_t lo,
+                                                        uint32_t hi, unsigned long long* gh,
+                                                        unsigned long long* extra) {
+    __shared__ uint32_t sh[HIST_SMEM];
+    __shared__ TabRef s_ref[TABREF_SMEM];
+    __shared__ unsigned long long s_found;
+    for (int i = threadIdx.x; i < HIST_SMEM; i += blockDim.x) sh[i] = 0;
+    if (threadIdx.x == 0) s_found = 0;
+    const TabRefs refs = tab_refs(meta, n_buckets, s_ref);
+    __syncthreads();
+    const uint64_t r0 = prefix ? low_at(prefix, nsegs, first_seg, n_low) : 0;
+    const uint32_t n = lookup_low<NW>(low, r0, n_low, k, bucket_shift, refs,
+                                      reinterpret_cast<const typename SlotOf<NW>::T*>(table),
+                                      [&](const typename KeyOf<NW>::T&, uint32_t count) {
+                                          hist_add(sh, gh, count, -1, lo, hi);
+                                          hist_add(sh, gh, (uint64_t)count + 1, 1, lo, hi);
+                                      });
+    block_add(extra, -(long long)n, &s_found);  // synchronises the block: sh is complete
+    hist_flush(sh, gh, lo, hi);
+    // the records no table holds: all minus those found, at count 1
+    if (threadIdx.x == 0 && lo <= 1) {
+        const long long all = blockIdx.x == 0 ? (long long)(n_low - r0) : 0;
+        const long long add = all + (long long)s_found;  // s_found = -(found by this block)
+        if (add) atomicAdd(gh + (1 - lo), (unsigned long long)add);
+    }
+}
+
+// Every table key at its table count; extra += the number of table keys.
+template <int NW>
+__global__ void __launch_bounds__(256) hist_table_pass(const void* table, const ExportChunk* chunks, uint64_t n_chunks,
+                                                       uint32_t lo, uint32_t hi, unsigned long long* gh,
+                                                       unsigned long long* extra) {
     using S = typename SlotOf<NW>::T;
     __shared__ uint32_t sh[HIST_SMEM];
-    __shared__ unsigned long long s_un;
+    __shared__ unsigned long long s_used;
     for (int i = threadIdx.x; i < HIST_SMEM; i += blockDim.x) sh[i] = 0;
-    if (threadIdx.x == 0) s_un = 0;
+    if (threadIdx.x == 0) s_used = 0;
     __syncthreads();
-    uint32_t un = 0;
-    for (uint64_t c = blockIdx.x; c < n_chunks; c += gridDim.x)
-    for (uint32_t q = threadIdx.x; q < chunks[c].n_slots; q += blockDim.x) {
-        const S s = reinterpret_cast<const S*>(table)[chunks[c].slot_begin + q];
-        bool used, marked;
-        if constexpr (NW == 1) {
-            used = s.key != EMPTY;
-            marked = s.pad != 0;
-        } else if constexpr (NW == 2) {
-            used = !(s.w0 == EMPTY && s.w1 == EMPTY);
-            marked = s.pad[0] != 0;
-        } else {
-            used = s.state == SLOT_READY;
-            marked = s.mark != 0;
-        }
-        if (used && !marked) {
-            ++un;
-            hist_add(sh, gh, s.count, lo, hi);
+    uint32_t n = 0;
+    for (uint64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
+        const ExportChunk ch = chunks[c];
+        const S* t = reinterpret_cast<const S*>(table) + ch.slot_begin;
+#pragma unroll 4
+        for (uint32_t q = threadIdx.x; q < ch.n_slots; q += blockDim.x) {
+            const S s = t[q];
+            if (slot_used<NW>(s)) {
+                ++n;
+                hist_add(sh, gh, s.count, 1, lo, hi);
+            }
         }
     }
-    for (int o = 16; o; o >>= 1) un += __shfl_xor_sync(0xffffffffu, un, o);
-    if ((threadIdx.x & 31) == 0 && un) atomicAdd(&s_un, (unsigned long long)un);
-    __syncthreads();
-    for (int i = threadIdx.x; i < HIST_SMEM; i += blockDim.x)
-        if (sh[i]) atomicAdd(gh + i, (unsigned long long)sh[i]);
-    if (threadIdx.x == 0 && s_un) atomicAdd(unmarked, s_un);
+    block_add(extra, (long long)n, &s_used);
+    hist_flush(sh, gh, lo, hi);
 }
 
-// Per model bucket (key word 0 >> 52) loads of the last result: low keys,
-// looked up in their table (marked as in hist_low_pass), then every table
-// key.  distinct = low keys + unmarked table keys; kmers = occurrences.
+// Per model bucket (key word 0 >> 52) loads of the last result, as the
+// histogram's sums: distinct = low.bin keys + table keys - low.bin keys found
+// in a table; kmers = low.bin keys + the table keys' counts.
 // model buckets of the sizing loads (the top 12 bits of the key)
 constexpr uint32_t KC_LOADS_BINS = 4096;
 // dynamic shared memory of loads_low_pass / loads_table_pass
-constexpr size_t loads_low_smem() { return KC_LOADS_BINS * (8 + 4); }
-constexpr size_t loads_table_smem() { return KC_LOADS_BINS * (8 + 4 + 4); }
+constexpr size_t loads_low_smem() { return KC_LOADS_BINS * (4 + 4); }
+constexpr size_t loads_table_smem() { return KC_LOADS_BINS * (8 + 4); }
 
 template <int NW>
-__global__ void loads_low_pass(const uint8_t* low, uint64_t n_low, uint32_t k, const BucketMeta* meta,
-                               uint32_t bucket_shift, void* table, unsigned long long* distinct,
-                               unsigned long long* kmers) {
+__global__ void __launch_bounds__(512) loads_low_pass(const uint8_t* low, uint64_t n_low, uint32_t k,
+                                                      const BucketMeta* meta, uint32_t n_buckets,
+                                                      uint32_t bucket_shift, const void* table,
+                                                      unsigned long long* distinct, unsigned long long* kmers) {
     // per-CTA totals per model bucket in shared memory (consecutive low keys
     // share their model bucket, so global atomics would serialise on it),
     // added to the global totals once per CTA
     extern __shared__ unsigned long long ld_smem[];
-    unsigned long long* s_kmers = ld_smem;                                        // [KC_LOADS_BINS]
-    uint32_t* s_distinct = reinterpret_cast<uint32_t*>(ld_smem + KC_LOADS_BINS);  // [KC_LOADS_BINS]
-    for (uint32_t i = threadIdx.x; i < KC_LOADS_BINS; i += blockDim.x) {
-        s_kmers[i] = 0;
-        s_distinct[i] = 0;
-    }
+    uint32_t* s_low = reinterpret_cast<uint32_t*>(ld_smem);  // [KC_LOADS_BINS]
+    uint32_t* s_found = s_low + KC_LOADS_BINS;               // [KC_LOADS_BINS]
+    __shared__ TabRef s_ref[TABREF_SMEM];
+    for (uint32_t i = threadIdx.x; i < 2 * KC_LOADS_BINS; i += blockDim.x) s_low[i] = 0;
+    const TabRefs refs = tab_refs(meta, n_buckets, s_ref);
     __syncthreads();
-    using K = typename KeyOf<NW>::T;
-    using S = typename SlotOf<NW>::T;
-    const uint32_t full = k / 32, tail_bits = 2 * (k % 32), tail_bytes = (tail_bits + 7) / 8;
-    const uint32_t P = full * 8 + tail_bytes;
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_low; r += (uint64_t)gridDim.x * blockDim.x) {
-        const K key = unpack_low<NW>(low, r, P, full, tail_bytes);
-        const BucketMeta m = meta[key_hi(key) >> bucket_shift];
-        S* tab = reinterpret_cast<S*>(table) + m.tab_off;
-        uint64_t at;
-        unsigned long long occ = 1;
-        if (table_find<NW>(tab, m.tab_mask, hash_key(key), key, &at)) {
-            occ += tab[at].count;
-            if constexpr (NW == 1) tab[at].pad = 1;
-            else if constexpr (NW == 2) tab[at].pad[0] = 1;
-            else tab[at].mark = 1;
-        }
-        const uint32_t bin = (uint32_t)(key_hi(key) >> 52);
-        atomicAdd(s_distinct + bin, 1u);
-        atomicAdd(s_kmers + bin, occ);
-    }
+    lookup_low<NW>(low, 0, n_low, k, bucket_shift, refs, reinterpret_cast<const typename SlotOf<NW>::T*>(table),
+                   [&](const typename KeyOf<NW>::T& key, uint32_t) { atomicAdd(s_found + (key_hi(key) >> 52), 1u); });
+    const uint32_t full = k / 32, tail_bytes = (2 * (k % 32) + 7) / 8, P = full * 8 + tail_bytes;
+    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_low; r += (uint64_t)gridDim.x * blockDim.x)
+        atomicAdd(s_low + (key_hi(load_low<NW>(low, r, P, full, tail_bytes)) >> 52), 1u);
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < KC_LOADS_BINS; i += blockDim.x) {
-        if (s_distinct[i]) atomicAdd(distinct + i, (unsigned long long)s_distinct[i]);
-        if (s_kmers[i]) atomicAdd(kmers + i, s_kmers[i]);
+        if (s_low[i] != s_found[i]) atomicAdd(distinct + i, (unsigned long long)s_low[i] - s_found[i]);
+        if (s_low[i]) atomicAdd(kmers + i, (unsigned long long)s_low[i]);
     }
 }
 
@@ -2085,12 +2205,10 @@ template <int NW>
 __global__ void loads_table_pass(const void* table, const ExportChunk* chunks, uint64_t n_chunks,
                                  unsigned long long* distinct, unsigned long long* tkeys, unsigned long long* kmers) {
     extern __shared__ unsigned long long ld_smem[];
-    unsigned long long* s_kmers = ld_smem;                                        // [KC_LOADS_BINS]
-    uint32_t* s_distinct = reinterpret_cast<uint32_t*>(ld_smem + KC_LOADS_BINS);  // [KC_LOADS_BINS]
-    uint32_t* s_tkeys = s_distinct + KC_LOADS_BINS;                               // [KC_LOADS_BINS]
+    unsigned long long* s_kmers = ld_smem;                                     // [KC_LOADS_BINS]
+    uint32_t* s_tkeys = reinterpret_cast<uint32_t*>(ld_smem + KC_LOADS_BINS);  // [KC_LOADS_BINS]
     for (uint32_t i = threadIdx.x; i < KC_LOADS_BINS; i += blockDim.x) {
         s_kmers[i] = 0;
-        s_distinct[i] = 0;
         s_tkeys[i] = 0;
     }
     __syncthreads();
@@ -2098,34 +2216,20 @@ __global__ void loads_table_pass(const void* table, const ExportChunk* chunks, u
     for (uint64_t c = blockIdx.x; c < n_chunks; c += gridDim.x)
     for (uint32_t q = threadIdx.x; q < chunks[c].n_slots; q += blockDim.x) {
         const S s = reinterpret_cast<const S*>(table)[chunks[c].slot_begin + q];
+        if (!slot_used<NW>(s)) continue;
         uint64_t hi;
-        bool used, marked;
-        if constexpr (NW == 1) {
-            used = s.key != EMPTY;
-            marked = s.pad != 0;
-            hi = s.key;
-        } else if constexpr (NW == 2) {
-            used = !(s.w0 == EMPTY && s.w1 == EMPTY);
-            marked = s.pad[0] != 0;
-            hi = s.w0;
-        } else {
-            used = s.state == SLOT_READY;
-            marked = s.mark != 0;
-            hi = s.w0;
-        }
-        if (!used) continue;
-        const uint32_t bin = (uint32_t)(hi >> 52);
-        atomicAdd(s_tkeys + bin, 1u);
-        if (!marked) {
-            atomicAdd(s_distinct + bin, 1u);
-            atomicAdd(s_kmers + bin, (unsigned long long)s.count);
-        }
+        if constexpr (NW == 1) hi = s.key;
+        else hi = s.w0;
+        atomicAdd(s_tkeys + (hi >> 52), 1u);
+        atomicAdd(s_kmers + (hi >> 52), (unsigned long long)s.count);
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < KC_LOADS_BINS; i += blockDim.x) {
-        if (s_tkeys[i]) atomicAdd(tkeys + i, (unsigned long long)s_tkeys[i]);
-        if (s_distinct[i]) atomicAdd(distinct + i, (unsigned long long)s_distinct[i]);
-        if (s_kmers[i]) atomicAdd(kmers + i, s_kmers[i]);
+        if (s_tkeys[i]) {
+            atomicAdd(tkeys + i, (unsigned long long)s_tkeys[i]);
+            atomicAdd(distinct + i, (unsigned long long)s_tkeys[i]);
+            atomicAdd(kmers + i, s_kmers[i]);
+        }
     }
 }
 
