@@ -408,29 +408,46 @@ struct Seg {
     uint32_t nls;    // bit j set: byte j is '\n'
 };
 
-// Four bytes at a time: base test (A/C/G/T/U after folding case) by the
-// exact zero-byte test of x ^ letter, newline likewise, 2-bit code by the
-// ((c >> 1) ^ (c >> 2)) & 3 identity (A=0 C=1 G=2 T/U=3, either case).
+// Byte selection of the PRMT instruction: byte i of the result is byte
+// (sel >> 4i) & 7 of the eight bytes y:x.
+KC_HD uint32_t byte_perm(uint32_t x, uint32_t y, uint32_t sel) {
+#ifdef __CUDA_ARCH__
+    return __byte_perm(x, y, sel);
+#else
+    const uint64_t v = ((uint64_t)y << 32) | x;
+    uint32_t r = 0;
+    for (int i = 0; i < 4; ++i) r |= (uint32_t)((v >> (8 * ((sel >> (4 * i)) & 7))) & 0xFF) << (8 * i);
+    return r;
+#endif
+}
+
+// Four bytes at a time.  The 2-bit code of a base is ((c >> 1) ^ (c >> 2)) & 3
+// (A=0 C=1 G=2 T/U=3, either case); any byte has such a code, and it is a base
+// when it equals the letter of its code: the letter is looked up by byte
+// permutation, case (0x20) is ignored, and for code 3 bit 0 too (T = 0x54,
+// U = 0x55).  Newlines by the exact zero-byte test.
 KC_HD Seg classify(const uint32_t (&w)[8], uint64_t valid_bytes) {
     Seg s{0, 0, 0};
-    uint32_t chi = 0, clo = 0;  // codes of bytes 0..15 (chi) and 16..31 (clo)
+    uint32_t prod[8];  // the word's four codes in byte 3
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const uint32_t x = w[i];
-        const uint32_t u = x & 0xDFDFDFDFu;
-        const uint32_t isb = zero_bytes(u ^ 0x41414141u) | zero_bytes(u ^ 0x43434343u) | zero_bytes(u ^ 0x47474747u) |
-                             zero_bytes(u ^ 0x54545454u) | zero_bytes(u ^ 0x55555555u);
-        const uint32_t isn = zero_bytes(x ^ 0x0A0A0A0Au);
-        s.bases |= gather_bit7(isb) << (4 * i);
-        s.nls |= gather_bit7(isn) << (4 * i);
+        const uint32_t code4 = ((x >> 1) ^ (x >> 2)) & 0x03030303u;
         // codes of bytes 4i..4i+3 -> 8 bits, byte 4i in the high pair: the
         // 2-bit fields at 0, 8, 16, 24 times 2^30 + 2^20 + 2^10 + 1 land at
         // 30, 28, 26, 24 (the other products fall below bit 22 or out)
-        const uint32_t code4 = ((x >> 1) ^ (x >> 2)) & 0x03030303u;
-        const uint32_t c8 = (code4 * 0x40100401u) >> 24;
-        if (i < 4) chi |= c8 << (24 - 8 * i);
-        else clo |= c8 << (24 - 8 * (i - 4));
+        prod[i] = code4 * 0x40100401u;
+        // the codes as selector nibbles 0..3
+        const uint32_t sel = byte_perm(code4 | (code4 >> 4), 0u, 0x20u) & 0xFFFFu;
+        const uint32_t letter = byte_perm(0x54474341u, 0u, sel);  // A C G T
+        const uint32_t care = byte_perm(0xDEDFDFDFu, 0u, sel);
+        const uint32_t isb = zero_bytes((x ^ letter) & care);
+        const uint32_t isn = zero_bytes(x ^ 0x0A0A0A0Au);
+        s.bases |= gather_bit7(isb) << (4 * i);
+        s.nls |= gather_bit7(isn) << (4 * i);
     }
+    const uint32_t chi = byte_perm(byte_perm(prod[2], prod[3], 0x37u), byte_perm(prod[0], prod[1], 0x37u), 0x5410u);
+    const uint32_t clo = byte_perm(byte_perm(prod[6], prod[7], 0x37u), byte_perm(prod[4], prod[5], 0x37u), 0x5410u);
     s.codes = ((uint64_t)chi << 32) | clo;
     if (valid_bytes < 32) {
         const uint32_t keep = valid_bytes ? (0xFFFFFFFFu >> (32 - (uint32_t)valid_bytes)) : 0u;
@@ -500,22 +517,38 @@ KC_HD uint32_t runs_at_least5(uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3
     return (uint32_t)x2;
 }
 
-// Bits of the 32 bytes that lie on sequence lines (line index = 1 mod 4),
-// line0 = line index of byte 0, nls = newline bits.
-__device__ __forceinline__ uint32_t sequence_mask(uint32_t line0, uint32_t nls) {
-    uint32_t seq = 0, start = 0, line = line0, m = nls;
-    for (;;) {
-        const uint32_t end = m ? (uint32_t)__ffs(m) : 32u;  // bytes [start, end) share `line`
-        if ((line & 3u) == 1u && end > start) {
-            const uint32_t hi = end >= 32 ? 0xFFFFFFFFu : ((1u << end) - 1u);
-            seq |= hi & ~((1u << start) - 1u);
-        }
-        if (!m) break;
-        start = end;
-        m &= m - 1;
-        ++line;
+// runs_at_least for k <= 32: the k bytes ending at byte j of the segment with
+// base bits `cur` lie in it and the segment before it (`prev`).
+KC_HD uint32_t runs_at_least2(uint32_t prev, uint32_t cur, uint32_t k) {
+    uint64_t R = ((uint64_t)cur << 32) | prev;
+    uint32_t have = 1;
+    while (2 * have <= k) {
+        R &= R << have;
+        have *= 2;
     }
-    return seq;
+    if (have < k) R &= R << (k - have);
+    return (uint32_t)(R >> 32);
+}
+
+// Bit j: parity of the bits 0..j of x.
+KC_HD uint32_t prefix_parity(uint32_t x) {
+    x ^= x << 1;
+    x ^= x << 2;
+    x ^= x << 4;
+    x ^= x << 8;
+    return x ^ (x << 16);
+}
+
+// Bits of the 32 bytes that lie on sequence lines (line index = 1 mod 4),
+// line0 = line index of byte 0, nls = newline bits.  The number of newlines
+// before a byte, mod 4, bit by bit: its low bit is their parity, its high bit
+// the parity of those that found the low bit set.
+KC_HD uint32_t sequence_mask(uint32_t line0, uint32_t nls) {
+    const uint32_t low = prefix_parity(nls) << 1;
+    const uint32_t high = prefix_parity(nls & low) << 1;
+    const uint32_t want = 1u - line0;  // mod 4
+    const uint32_t w0 = (want & 1u) ? ~0u : 0u, w1 = (want & 2u) ? ~0u : 0u;
+    return ~(low ^ w0) & ~(high ^ w1);
 }
 
 // Reverse the order of the nb two-bit bases in the low 2*nb bits of x.
@@ -613,6 +646,91 @@ KC_HD uint32_t bucket_of_window(uint64_t lo, uint64_t hi, uint32_t k, uint32_t B
     return topF < topC ? topF : topC;
 }
 
+// ---- canonical keys from two base streams
+//
+// Both orientations of a window are contiguous in a stream of 2-bit codes:
+// C (complemented, read order) in the stream of complemented codes, first base
+// first; F (not complemented, newest base first) in the stream of codes in
+// reverse order.  A tile keeps both as 32-bit words (16 bases, first one in
+// the high bits), so a left-aligned key word is one funnel shift of two
+// adjacent words, with no bit reversal or left alignment per key.
+constexpr int TILE_SEGS = EXT_TILE / 32 + HALO_SEGS;  // segments of a tile with its halo
+constexpr int C_WORDS = 2 * TILE_SEGS + 8;            // a window may read 7 words past its last base's
+constexpr int STREAM_WORDS = C_WORDS + 2 * TILE_SEGS; // C stream, then F stream
+
+KC_HD uint32_t funnel_l(uint32_t hi, uint32_t lo, uint32_t sh) {  // high word of (hi:lo) << sh, sh < 32
+#ifdef __CUDA_ARCH__
+    return __funnelshift_l(lo, hi, sh);
+#else
+    return sh ? (hi << sh) | (lo >> (32 - sh)) : hi;
+#endif
+}
+
+// The codes of segment t (0 = the first halo segment) into both streams.
+KC_HD void stream_put(uint32_t* sw, int t, uint64_t codes) {
+    sw[2 * t] = ~(uint32_t)(codes >> 32);
+    sw[2 * t + 1] = ~(uint32_t)codes;
+    const uint64_t r = rev_bases(codes);
+    uint32_t* f = sw + C_WORDS + 2 * (TILE_SEGS - 1 - t);
+    f[0] = (uint32_t)(r >> 32);
+    f[1] = (uint32_t)r;
+}
+
+// Where a k-base window that ends at byte e of the tile (halo not counted)
+// starts in the streams.
+struct StreamPos {
+    uint32_t c, cs, f, fs;  // first word and bit shift of C, of F
+};
+KC_HD StreamPos stream_pos(uint32_t e, uint32_t k) {
+    const uint32_t b0 = e + HALO + 1 - k;         // its first base in the C stream (k <= HALO)
+    const uint32_t q = (uint32_t)EXT_TILE - 1 - e;  // its newest base in the F stream
+    return StreamPos{b0 >> 4, 2 * (b0 & 15), (uint32_t)C_WORDS + (q >> 4), 2 * (q & 15)};
+}
+
+// Bits of 32-bit key word w that belong to a k-base key.
+KC_HD uint32_t key_mask(uint32_t w, uint32_t k) {
+    const int n = (int)(2 * k) - 32 * (int)w;
+    return n >= 32 ? ~0u : (n <= 0 ? 0u : ~0u << (32 - n));
+}
+
+// The first 32 bits of the canonical key (what its bucket is taken from):
+// the smaller of the orientations' first words, whichever orientation the
+// rest decides for.
+KC_HD uint32_t top_of_window(const uint32_t* sw, const StreamPos& p, uint32_t mask0) {
+    const uint32_t f = funnel_l(sw[p.f], sw[p.f + 1], p.fs) & mask0;
+    const uint32_t c = funnel_l(sw[p.c], sw[p.c + 1], p.cs) & mask0;
+    return f < c ? f : c;
+}
+
+// The canonical key: the orientation with the smaller word at the first
+// difference (bits past the key can differ only when all of its bits agree,
+// and then either will do).
+template <int NW>
+KC_HD void key_of_window(const uint32_t* sw, const StreamPos& p, uint32_t k, uint64_t (&key)[NW]) {
+    const uint32_t n = (2 * k + 31) / 32;  // 32-bit words that hold key bits
+    bool f_less = true;
+    for (uint32_t w = 0; w < n; ++w) {
+        const uint32_t f = funnel_l(sw[p.f + w], sw[p.f + w + 1], p.fs);
+        const uint32_t c = funnel_l(sw[p.c + w], sw[p.c + w + 1], p.cs);
+        f_less = f < c;
+        if (f != c) break;
+    }
+    const uint32_t* s = sw + (f_less ? p.f : p.c);
+    const uint32_t sh = f_less ? p.fs : p.cs;
+    uint32_t prev = s[0];
+#pragma unroll
+    for (int w = 0; w < 2 * NW; ++w) {
+        uint32_t v = 0;
+        if ((uint32_t)w < n) {
+            const uint32_t next = s[w + 1];
+            v = funnel_l(prev, next, sh) & key_mask(w, k);
+            prev = next;
+        }
+        if (w & 1) key[w / 2] |= v;
+        else key[w / 2] = (uint64_t)v << 32;
+    }
+}
+
 // Canonical k-mer extraction over one 8 KiB tile per CTA.
 //
 // Emission rule (reference: src/FastqReader.h:140-308 + src/FastqParser.h:
@@ -623,53 +741,83 @@ KC_HD uint32_t bucket_of_window(uint64_t lo, uint64_t hi, uint32_t k, uint32_t B
 //
 // Phase A, per thread (32 bytes): classify, then a bit-parallel emit mask:
 //   run of >= k bases ending at byte j (shift-AND doubling over the bases
-//   of this and the two preceding segments) AND byte j on a sequence line.
-// Phase C, per position: round r covers bytes [256r, 256r+256) of the tile,
-//   so a warp owns one 32-byte segment per round -- warps over quality and
-//   header bytes skip uniformly.  The window comes from the segment's codes
-//   and its two predecessors (shared memory; the two before the tile are the
-//   64-byte halo).
-// HIST: per-bucket totals via the bucket-only path.  SCATTER: bucket-only
-// histogram, one reservation per bucket per CTA, then full keys written to
-// routed[base[bucket] + rank].
-// Keys of one SCATTER tile staged in shared memory (bucket-sorted) before
-// they are written out as contiguous runs; keys beyond this go out directly.
-// (3840 keys for 64-bit keys: an 8 KiB tile of 150 bp FASTQ holds ~3150, and
-// 4 CTAs of the scatter still fit one SM's shared memory)
-template <int NW>
-__host__ __device__ constexpr int stage_keys() {
-    return NW == 1 ? 3840 : (NW == 2 ? 2048 : 1024);
-}
+//   of this and the preceding segments) AND byte j on a sequence line; the
+//   segments that emit are listed, and their codes go to the two streams.
+// Phase C, per listed segment: one warp, lane j the window ending at byte j.
+//
+// HIST: per-bucket totals (bucket = top bits of the canonical key, from the
+// streams' first words).  SCATTER (256 buckets): every key takes its rank
+// from its bucket's shared-memory counter, one reservation per bucket per CTA
+// places the tile's runs in the routed array, and the keys are written in
+// bucket order, as contiguous runs.
+//   64-bit keys are staged in arrival order and indexed in bucket order.
+//   128- and 256-bit keys, and tiles with more 64-bit keys than the staging
+//   area holds, only index their positions: the first pass needs the bucket
+//   alone, and the key is built from the streams when it is written, once.
+//   (Staging 128-bit keys in 48 KB held 2048 of the 2300 keys of a tile of
+//   150 bp reads at k = 63; the tiles that did not fit built every key twice.)
+//
+// The kernel is bound by instruction issue (the integer pipe), not by its
+// bytes.  Before, each key came from 64-bit shifts and bit reversals of its
+// segment's codes, and tiles walked all their segments: 10 M reads of 150 bp
+// at k = 31 9.5 -> 7.4 ms, 6 M at k = 63 10.4 -> 4.6, 1 M of 250 bp at
+// k = 101 5.2 -> 2.2.
+
+// 64-bit keys of one tile staged in shared memory: an 8 KiB tile of 150 bp
+// FASTQ holds ~3150 at k = 31, and 4 CTAs fit one SM's shared memory.
+constexpr int STAGE_KEYS = 3824;
+constexpr int ROUTE_BUCKETS = 256;  // buckets of SCATTER, one per thread
+static_assert(ROUTE_BUCKETS == EXT_THREADS, "a thread reserves its bucket's run");
 
 // Dynamic shared memory of extract_kernel.
 template <int NW, int MODE>
 __host__ __device__ constexpr size_t extract_smem_bytes(uint32_t n_buckets) {
-    return (size_t)n_buckets * (8 + 4 + 4 + 4) + (MODE == SCATTER ? (size_t)stage_keys<NW>() * (8 * NW + 2 + 2) : 0);
+    if (MODE == HIST) return (size_t)n_buckets * 4;
+    // u64 gdelta[256] | u32 hist[256] | u32 loff[256] | staged keys (u64 key,
+    // u16 rank, u16 order) or positions (u16 rank, u16 order, u8 bucket)
+    const size_t staged = NW == 1 ? (size_t)STAGE_KEYS * 12 : 0, byplace = (size_t)EXT_TILE * 5;
+    return (size_t)ROUTE_BUCKETS * 16 + (staged > byplace ? staged : byplace);
+}
+
+// Inclusive scan of one value per thread over the CTA; *total = its sum.
+// warp_sums: a buffer of its own per use (one barrier, no reuse).
+__device__ __forceinline__ uint32_t tile_scan(uint32_t v, uint32_t* warp_sums, uint32_t* total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
+    }
+    if (lane == 31) warp_sums[warp] = v;
+    __syncthreads();
+    uint32_t before = 0, sum = 0;
+#pragma unroll
+    for (int w = 0; w < EXT_THREADS / 32; ++w) {
+        const uint32_t t = warp_sums[w];
+        before += w < warp ? t : 0u;
+        sum += t;
+    }
+    *total = sum;
+    return v + before;
 }
 
 template <int NW, int MODE>
 __global__ void __launch_bounds__(EXT_THREADS, EXT_MIN_CTAS) extract_kernel(ExtractArgs a) {
-    // dynamic smem: u64 base[nb] | u32 hist[nb] | u32 fill[nb] | u32 loff[nb]
-    //               | SCATTER: K keys[stage] | u16 rank_or_bucket[stage] | u16 order[stage]
-    extern __shared__ unsigned long long ext_smem[];
-    // segment t of the tile is seg_*[t + HALO_SEGS]; the HALO_SEGS before it
-    // hold the halo bytes (zero where there is nothing to read)
-    __shared__ uint64_t seg_codes[EXT_THREADS + HALO_SEGS];
-    __shared__ uint32_t seg_bases[EXT_THREADS + HALO_SEGS];
-    __shared__ uint32_t seg_emit[EXT_THREADS];
-    __shared__ uint32_t seg_first[EXT_THREADS];  // arrival index of the segment's first k-mer
-    __shared__ uint32_t warp_sums[EXT_THREADS / 32];
-    using K = typename KeyOf<NW>::T;
-    constexpr int STAGE = stage_keys<NW>();
-    unsigned long long* bbase = ext_smem;
-    uint32_t* hist = reinterpret_cast<uint32_t*>(ext_smem + a.n_buckets);
-    uint32_t* fill = hist + a.n_buckets;
-    uint32_t* loff = fill + a.n_buckets;
-    K* skeys = reinterpret_cast<K*>(loff + a.n_buckets + (a.n_buckets & 1));  // 8-byte aligned
-    uint16_t* sbkt = reinterpret_cast<uint16_t*>(skeys + STAGE);  // two-pass: bucket; one pass: rank
-    uint16_t* sorder = sbkt + STAGE;                               // one pass: arrival index by bucket order
+    extern __shared__ __align__(16) uint8_t ext_smem[];
+    __shared__ uint32_t sw[STREAM_WORDS];
+    // emitting segments: emit mask << 32 | first arrival index << 8 | segment
+    __shared__ uint64_t seg_list[EXT_THREADS];
+    __shared__ uint32_t sums[3][EXT_THREADS / 32];
+    __shared__ uint32_t hist_bases[MODE == HIST ? TILE_SEGS : 1];
+    uint64_t* gdelta = reinterpret_cast<uint64_t*>(ext_smem);
+    uint32_t* hist = MODE == HIST ? reinterpret_cast<uint32_t*>(ext_smem)
+                                  : reinterpret_cast<uint32_t*>(gdelta + ROUTE_BUCKETS);
+    uint32_t* loff = hist + ROUTE_BUCKETS;
+    uint8_t* area = reinterpret_cast<uint8_t*>(loff + ROUTE_BUCKETS);
+    // base bits of the segments: phase A only, in the staging area
+    uint32_t* seg_bases = MODE == HIST ? hist_bases : reinterpret_cast<uint32_t*>(area);
 
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t tile = a.tile_list ? (uint64_t)a.tile_list[blockIdx.x]
                                       : (uint64_t)blockIdx.x * (a.tile_stride > 1 ? a.tile_stride : 1u);
     uint64_t tile_start = tile * EXT_TILE;
@@ -688,238 +836,169 @@ __global__ void __launch_bounds__(EXT_THREADS, EXT_MIN_CTAS) extract_kernel(Extr
         bucket_off = (uint64_t)t.set * a.n_buckets;
     }
     const uint64_t seg_start = tile_start + (uint64_t)tid * EXT_BPT;
-    const uint32_t B = 64 - a.bucket_shift;
+    const uint32_t tile_line0 = (uint32_t)a.tile_line[tile];
 
-    for (uint32_t b = tid; b < a.n_buckets; b += EXT_THREADS) {
-        hist[b] = 0;
-        fill[b] = 0;
-    }
+    for (uint32_t b = tid; b < (MODE == HIST ? a.n_buckets : (uint32_t)ROUTE_BUCKETS); b += EXT_THREADS) hist[b] = 0;
 
     // ---- phase A: classify own segment (+ the halo segments)
     uint32_t w[8];
     const uint64_t valid = seg_start < n_end ? n_end - seg_start : 0;
     load32(a.buf + seg_start, valid, w);
     const Seg s = classify(w, valid);
-    seg_codes[tid + HALO_SEGS] = s.codes;
+    stream_put(sw, tid + HALO_SEGS, s.codes);
     seg_bases[tid + HALO_SEGS] = s.bases;
     if (tid < HALO_SEGS) {
         uint32_t hw[8];
-        const bool readable = halo_ok;
-        load32(a.buf + (int64_t)tile_start - HALO + 32 * tid, readable ? 32 : 0, hw);
-        const Seg h = classify(hw, readable ? 32 : 0);
-        seg_codes[tid] = h.codes;
+        load32(a.buf + (int64_t)tile_start - HALO + 32 * tid, halo_ok ? 32 : 0, hw);
+        const Seg h = classify(hw, halo_ok ? 32 : 0);
+        stream_put(sw, tid, h.codes);
         seg_bases[tid] = h.bases;
     }
-    uint32_t nl_total;
-    const uint32_t nl_before = block_exclusive_scan<EXT_THREADS>(__popc(s.nls), warp_sums, &nl_total);
-    (void)nl_total;  // the scan synchronised the block: seg_* are visible
-    const uint32_t line0 = (uint32_t)a.tile_line[tile] + nl_before;
+    if (tid < C_WORDS - 2 * TILE_SEGS) sw[2 * TILE_SEGS + tid] = 0;  // read past the last window, masked out
+    uint32_t total;
+    const uint32_t nl = (uint32_t)__popc(s.nls);
+    const uint32_t line0 = tile_line0 + tile_scan(nl, sums[0], &total) - nl;  // the scan publishes seg_bases
 
     uint32_t emit = 0;
-    if (s.bases) {
-        const uint32_t seq = sequence_mask(line0, s.nls);
-        if (seq & s.bases) {
-            const uint32_t* sb = seg_bases + tid + HALO_SEGS;  // sb[0] = this segment
-            if constexpr (NW == 4) {
-                emit = runs_at_least5(sb[-4], sb[-3], sb[-2], sb[-1], s.bases, k) & seq;
-            } else {
-                const u128 X = ((u128)s.bases << 64) | ((u128)sb[-1] << 32) | (u128)sb[-2];
-                emit = (uint32_t)(runs_at_least(X, k) >> 64) & seq;
-            }
+    const uint32_t seq = s.bases ? sequence_mask(line0, s.nls) : 0u;
+    if (seq & s.bases) {
+        const uint32_t* sb = seg_bases + tid + HALO_SEGS;  // sb[0] = this segment
+        if constexpr (NW == 1) {
+            emit = runs_at_least2(sb[-1], s.bases, k) & seq;
+        } else if constexpr (NW == 4) {
+            emit = runs_at_least5(sb[-4], sb[-3], sb[-2], sb[-1], s.bases, k) & seq;
+        } else {
+            const u128 X = ((u128)s.bases << 64) | ((u128)sb[-1] << 32) | (u128)sb[-2];
+            emit = (uint32_t)(runs_at_least(X, k) >> 64) & seq;
         }
     }
-    seg_emit[tid] = emit;
-    uint32_t n_tile;  // k-mers of the tile; the scan also publishes seg_emit
-    seg_first[tid] = block_exclusive_scan<EXT_THREADS>(__popc(emit), warp_sums, &n_tile);
-    __syncthreads();  // every segment's seg_first is read by another warp below
-    if (!n_tile) {
-        return;  // nothing to count in this tile (HIST adds nothing; SCATTER reserves nothing)
-    }
+    // k-mers (low half) and emitting segments (high half) up to this segment
+    const uint32_t mine = (uint32_t)__popc(emit) | (emit ? 1u << 16 : 0u);
+    const uint32_t upto = tile_scan(mine, sums[1], &total);
+    const uint32_t n_tile = total & 0xFFFFu, n_segs = total >> 16;
+    if (!n_tile) return;  // block-uniform: nothing to count in this tile (SCATTER reserves nothing)
+    if (emit)
+        seg_list[(upto >> 16) - 1] = ((uint64_t)emit << 32) | (((upto & 0xFFFFu) - (uint32_t)__popc(emit)) << 8) | (uint32_t)tid;
+    __syncthreads();
 
     // ---- phase C
-    const int lane = tid & 31;
-    const int warp = tid >> 5;
     const uint32_t lt = (1u << lane) - 1u;
-    // canonical key and routing bucket of the window ending at byte `lane` of segment t
-    auto full_key = [&](int t, K& key, uint32_t& bucket) {
-        const uint64_t* sc = seg_codes + t + HALO_SEGS;  // sc[0] = segment t
-        uint64_t lo, hi, w2 = 0, w3 = 0;
-        if constexpr (NW == 4) window_at4(sc[-4], sc[-3], sc[-2], sc[-1], sc[0], (uint32_t)lane, lo, hi, w2, w3);
-        else window_at(sc[-2], sc[-1], sc[0], (uint32_t)lane, lo, hi);
-        if constexpr (NW == 1) {
-            const uint64_t km = k >= 32 ? ~0ull : ((1ull << (2 * k)) - 1ull);
-            key = canonical1(lo & km, k);
-            bucket = (uint32_t)(key >> a.bucket_shift);
-        } else if constexpr (NW == 2) {
-            const uint32_t hb = 2 * k - 64;
-            const uint64_t hmask = hb >= 64 ? ~0ull : ((1ull << hb) - 1ull);
-            key = canonical2(hi & hmask, lo, k);
-            bucket = (uint32_t)(key.w0 >> a.bucket_shift);
-        } else {
-            key = canonical4(lo, hi, w2, w3, k);
-            bucket = (uint32_t)(key.w0 >> a.bucket_shift);
-        }
-    };
-    // reserve each bucket's run in the routed array (bbase) and the local
-    // offsets of the bucket-sorted staging area (loff), from hist
-    auto reserve = [&]() {
-        const uint32_t per = (a.n_buckets + EXT_THREADS - 1) / EXT_THREADS;
-        uint32_t sum = 0;
-        for (uint32_t q = 0; q < per; ++q) {
-            const uint32_t b = tid * per + q;
-            if (b < a.n_buckets) {
-                const uint32_t c = hist[b];
-                const uint64_t rb = bucket_off + b;  // the region (of this set)
-                unsigned long long base = c ? atomicAdd(a.bucket_cursor + rb, (unsigned long long)c) : 0ull;
-                if (a.region_end && c && base + c > a.region_end[rb]) {
-                    // the run does not fit the region: it goes whole to the
-                    // overflow area.  If that is full too, the batch is routed
-                    // again (error bit 1) and the run lands, in bounds, at the
-                    // overflow area's start (at least 65536 keys >= one run).
-                    atomicMin(a.region_fill + rb, base);
-                    // a multi-set batch has an overflow area per set
-                    unsigned long long* const ocur = a.set_ovf_cursor ? a.set_ovf_cursor + set : a.overflow_cursor;
-                    const uint64_t oend = a.set_ovf_cursor ? a.set_ovf_end[set] : a.overflow_end;
-                    const uint64_t ostart = a.set_ovf_cursor ? a.set_ovf_start[set] : a.overflow_start;
-                    const unsigned long long ob = atomicAdd(ocur, (unsigned long long)c);
-                    if (ob + c <= oend) {
-                        base = ob;
-                    } else {
-                        base = ostart;
-                        atomicOr(a.error, 2u);
-                    }
-                }
-                bbase[b] = base;
-                sum += c;
-            }
-        }
-        uint32_t run = block_exclusive_scan<EXT_THREADS>(sum, warp_sums, nullptr);
-        for (uint32_t q = 0; q < per; ++q) {
-            const uint32_t b = tid * per + q;
-            if (b < a.n_buckets) {
-                loff[b] = run;
-                run += hist[b];
-            }
-        }
-        __syncthreads();
-    };
+    const uint32_t mask0 = key_mask(0, k);
+    // lane `lane` of segment t: the window's place for t = 0 plus 2t words
+    const StreamPos lane_pos = stream_pos((uint32_t)lane, k);
+    auto pos_of = [&](uint32_t t) { return StreamPos{lane_pos.c + 2 * t, lane_pos.cs, lane_pos.f - 2 * t, lane_pos.fs}; };
 
-    if (MODE == SCATTER && n_tile <= (uint32_t)STAGE) {
-        // One extraction pass: the bucket's shared-memory counter gives each
-        // key its rank in the bucket and builds the tile histogram at once;
-        // keys are staged in arrival order, then indexed in bucket order and
-        // written out as contiguous runs.
-#pragma unroll 1
-        for (int r = 0; r < EXT_BPT; ++r) {
-            const int t = r * (EXT_THREADS / 32) + warp;
-            const uint32_t em = seg_emit[t];
-            if (!em) continue;  // warp-uniform
-            if (!((em >> lane) & 1u)) continue;
-            K key;
-            uint32_t bucket;
-            full_key(t, key, bucket);
-            const uint32_t arr = seg_first[t] + __popc(em & lt);
-            if (arr >= n_tile) {  // cannot happen; reported, never written
-                atomicOr(a.error, 1u);
-                continue;
-            }
-            const uint32_t rnk = atomicAdd(hist + bucket, 1u);
-            skeys[arr] = key;
-            sbkt[arr] = (uint16_t)rnk;
+    if constexpr (MODE == HIST) {
+        const uint32_t shift = a.bucket_shift - 32;  // of the key's first 32 bits
+        for (uint32_t i = warp; i < n_segs; i += EXT_THREADS / 32) {
+            const uint64_t e = seg_list[i];
+            if (((uint32_t)(e >> 32) >> lane) & 1u)
+                atomicAdd(hist + (top_of_window(sw, pos_of((uint32_t)e & 0xFFu), mask0) >> shift), 1u);
         }
         __syncthreads();
-        reserve();
-        for (uint32_t i = tid; i < n_tile; i += EXT_THREADS) {
-            const uint32_t b = (uint32_t)(key_hi(skeys[i]) >> a.bucket_shift);
-            const uint32_t pos = loff[b] + sbkt[i];
-            if (sbkt[i] < hist[b] && pos < n_tile) sorder[pos] = (uint16_t)i;
-            else atomicOr(a.error, 1u);
-        }
-        __syncthreads();
-        K* out = reinterpret_cast<K*>(a.routed);
-        for (uint32_t p = tid; p < n_tile; p += EXT_THREADS) {
-            const uint32_t i = sorder[p];
-            if (i >= n_tile) {
-                atomicOr(a.error, 1u);
-                continue;
-            }
-            const K key = skeys[i];
-            const uint32_t b = (uint32_t)(key_hi(key) >> a.bucket_shift);
-            if (p - loff[b] < hist[b]) out[bbase[b] + (p - loff[b])] = key;  // inside the bucket's reservation
-            else atomicOr(a.error, 1u);
+        for (uint32_t b = tid; b < a.n_buckets; b += EXT_THREADS) {
+            const uint32_t c = hist[b];
+            if (c) atomicAdd(a.bucket_count + bucket_off + b, (unsigned long long)c);
         }
         return;
     }
 
-    // Two passes (histogram, then keys; and the HIST kernel's only pass):
-    // tiles with more k-mers than the staging area holds
-#pragma unroll 1
-    for (int pass = 0; pass < (MODE == SCATTER ? 2 : 1); ++pass) {
-        if (pass == 1) reserve();
-#pragma unroll 1
-        for (int r = 0; r < EXT_BPT; ++r) {
-            const int t = r * (EXT_THREADS / 32) + warp;  // segment owned by this warp this round
-            const uint32_t em = seg_emit[t];
-            if (!em) continue;  // warp-uniform
-            if (!((em >> lane) & 1u)) continue;
-            const uint64_t* sc = seg_codes + t + HALO_SEGS;  // sc[0] = segment t
-            uint64_t lo, hi, w2 = 0, w3 = 0;
-            if constexpr (NW == 4) window_at4(sc[-4], sc[-3], sc[-2], sc[-1], sc[0], (uint32_t)lane, lo, hi, w2, w3);
-            else window_at(sc[-2], sc[-1], sc[0], (uint32_t)lane, lo, hi);
-            if (pass == 0 && NW == 4) {
-                // 256-bit keys: the bucket from the full canonical key
-                const Key4 key4 = canonical4(lo, hi, w2, w3, k);
-                atomicAdd(hist + (uint32_t)(key4.w0 >> a.bucket_shift), 1u);
-            } else if (pass == 0) {
-                if (NW == 1) {
-                    const uint64_t km = k >= 32 ? ~0ull : ((1ull << (2 * k)) - 1ull);
-                    lo &= km;
-                } else {
-                    const uint32_t hb = 2 * k - 64;
-                    hi &= hb >= 64 ? ~0ull : ((1ull << hb) - 1ull);
-                }
-                atomicAdd(hist + bucket_of_window(lo, hi, k, B), 1u);
+    // Reserve bucket tid's run in the routed array, and the runs' offsets in
+    // the tile's bucket order (loff): position p of that order, in bucket b,
+    // belongs at routed[gdelta[b] + p].
+    auto reserve = [&]() {
+        const uint32_t c = hist[tid];
+        const uint64_t rb = bucket_off + tid;  // the region (of this set)
+        unsigned long long base = c ? atomicAdd(a.bucket_cursor + rb, (unsigned long long)c) : 0ull;
+        if (a.region_end && c && base + c > a.region_end[rb]) {
+            // the run does not fit the region: it goes whole to the
+            // overflow area.  If that is full too, the batch is routed
+            // again (error bit 1) and the run lands, in bounds, at the
+            // overflow area's start (at least 65536 keys >= one run).
+            atomicMin(a.region_fill + rb, base);
+            // a multi-set batch has an overflow area per set
+            unsigned long long* const ocur = a.set_ovf_cursor ? a.set_ovf_cursor + set : a.overflow_cursor;
+            const uint64_t oend = a.set_ovf_cursor ? a.set_ovf_end[set] : a.overflow_end;
+            const uint64_t ostart = a.set_ovf_cursor ? a.set_ovf_start[set] : a.overflow_start;
+            const unsigned long long ob = atomicAdd(ocur, (unsigned long long)c);
+            if (ob + c <= oend) {
+                base = ob;
             } else {
-                K key;
-                uint32_t bucket;
-                full_key(t, key, bucket);
-                const uint32_t rnk = atomicAdd(fill + bucket, 1u);
-                if (rnk < hist[bucket]) {
-                    const uint32_t sidx = loff[bucket] + rnk;
-                    if (sidx < (uint32_t)STAGE) {
-                        skeys[sidx] = key;
-                        sbkt[sidx] = (uint16_t)bucket;
-                    } else {
-                        reinterpret_cast<K*>(a.routed)[bbase[bucket] + rnk] = key;
-                    }
-                } else {
-                    atomicOr(a.error, 1u);  // never write outside the reservation
-                }
+                base = ostart;
+                atomicOr(a.error, 2u);
             }
+        }
+        uint32_t sum;
+        const uint32_t off = tile_scan(c, sums[2], &sum) - c;
+        loff[tid] = off;
+        gdelta[tid] = base - off;
+        if (sum != n_tile) atomicOr(a.error, 1u);  // cannot happen: every listed k-mer was ranked once
+        __syncthreads();
+    };
+
+    if (NW == 1 && n_tile <= (uint32_t)STAGE_KEYS) {
+        uint64_t* skeys = reinterpret_cast<uint64_t*>(area);
+        uint16_t* rank = reinterpret_cast<uint16_t*>(skeys + STAGE_KEYS);
+        uint16_t* order = rank + STAGE_KEYS;
+        const uint32_t mask1 = key_mask(1, k);
+        for (uint32_t i = warp; i < n_segs; i += EXT_THREADS / 32) {
+            const uint64_t e = seg_list[i];
+            const uint32_t em = (uint32_t)(e >> 32);
+            if (!((em >> lane) & 1u)) continue;
+            const StreamPos p = pos_of((uint32_t)e & 0xFFu);
+            const uint32_t f1 = sw[p.f + 1], c1 = sw[p.c + 1];
+            const uint64_t F = ((uint64_t)funnel_l(sw[p.f], f1, p.fs) << 32) | funnel_l(f1, sw[p.f + 2], p.fs);
+            const uint64_t C = ((uint64_t)funnel_l(sw[p.c], c1, p.cs) << 32) | funnel_l(c1, sw[p.c + 2], p.cs);
+            const uint64_t key = (F < C ? F : C) & (((uint64_t)mask0 << 32) | mask1);
+            const uint32_t arr = ((uint32_t)e >> 8) + (uint32_t)__popc(em & lt);  // < n_tile
+            rank[arr] = (uint16_t)atomicAdd(hist + (uint32_t)(key >> 56), 1u);
+            skeys[arr] = key;
         }
         __syncthreads();
-        if (MODE == SCATTER && pass == 1) {
-            // staged keys out as contiguous runs: consecutive slots of one
-            // bucket go to consecutive routed positions
-            uint32_t total = 0;
-            for (uint32_t b = tid; b < a.n_buckets; b += EXT_THREADS) total += hist[b];
-            for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-            if ((tid & 31) == 0) warp_sums[tid >> 5] = total;
-            __syncthreads();
-            total = 0;
-            for (int w = 0; w < EXT_THREADS / 32; ++w) total += warp_sums[w];
-            const uint32_t staged = min(total, (uint32_t)STAGE);
-            K* out = reinterpret_cast<K*>(a.routed);
-            for (uint32_t i = tid; i < staged; i += EXT_THREADS) {
-                const uint32_t b = sbkt[i];
-                out[bbase[b] + (i - loff[b])] = skeys[i];
-            }
+        reserve();
+        for (uint32_t i = tid; i < n_tile; i += EXT_THREADS)
+            order[loff[(uint32_t)(skeys[i] >> 56)] + rank[i]] = (uint16_t)i;
+        __syncthreads();
+        uint64_t* out = reinterpret_cast<uint64_t*>(a.routed);
+        for (uint32_t p = tid; p < n_tile; p += EXT_THREADS) {
+            const uint64_t key = skeys[order[p]];
+            out[gdelta[(uint32_t)(key >> 56)] + p] = key;
         }
+        return;
     }
-    if (MODE == HIST) {
-        for (uint32_t b = tid; b < a.n_buckets; b += EXT_THREADS) {
-            const uint32_t c = hist[b];
-            if (c) atomicAdd(a.bucket_count + bucket_off + b, (unsigned long long)c);
+
+    {
+        uint16_t* rank = reinterpret_cast<uint16_t*>(area);
+        uint16_t* order = rank + EXT_TILE;
+        uint8_t* bkt = reinterpret_cast<uint8_t*>(order + EXT_TILE);
+        for (uint32_t i = warp; i < n_segs; i += EXT_THREADS / 32) {
+            const uint64_t e = seg_list[i];
+            if (!(((uint32_t)(e >> 32) >> lane) & 1u)) continue;
+            const uint32_t t = (uint32_t)e & 0xFFu, at = 32 * t + lane;
+            const uint32_t b = top_of_window(sw, pos_of(t), mask0) >> 24;
+            rank[at] = (uint16_t)atomicAdd(hist + b, 1u);
+            bkt[at] = (uint8_t)b;
+        }
+        __syncthreads();
+        reserve();
+        for (uint32_t i = warp; i < n_segs; i += EXT_THREADS / 32) {
+            const uint64_t e = seg_list[i];
+            if (!(((uint32_t)(e >> 32) >> lane) & 1u)) continue;
+            const uint32_t at = 32 * ((uint32_t)e & 0xFFu) + lane;
+            order[loff[bkt[at]] + rank[at]] = (uint16_t)at;
+        }
+        __syncthreads();
+        for (uint32_t p = tid; p < n_tile; p += EXT_THREADS) {
+            uint64_t key[NW];
+            key_of_window<NW>(sw, stream_pos(order[p], k), k, key);
+            const uint64_t at = gdelta[(uint32_t)(key[0] >> 56)] + p;
+            if constexpr (NW == 1) {
+                reinterpret_cast<uint64_t*>(a.routed)[at] = key[0];
+            } else {
+                ulonglong2* out = reinterpret_cast<ulonglong2*>(a.routed) + at * (NW / 2);
+#pragma unroll
+                for (int q = 0; q < NW / 2; ++q) out[q] = make_ulonglong2(key[2 * q], key[2 * q + 1]);
+            }
         }
     }
 }
@@ -2107,7 +2186,7 @@ __device__ __forceinline__ uint64_t low_at(const uint64_t* prefix, uint64_t nseg
 // for the others.  extra -= the number found (distinct keys = low.bin keys +
 // table keys - found).
 template <int NW>
-__global__ void __launch_bounds__(256, 6) hist_low_pass(const uint8_t* low, uint64_t n_low, const uint64_t* prefix,
+__global__ void __launch_bounds__(256, 5) hist_low_pass(const uint8_t* low, uint64_t n_low, const uint64_t* prefix,
                                                         uint64_t nsegs, uint64_t first_seg, uint32_t k,
                                                         const BucketMeta* meta, uint32_t n_buckets,
                                                         uint32_t bucket_shift, const void* table, uint32_t lo,
