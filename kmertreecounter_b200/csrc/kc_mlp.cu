@@ -8,7 +8,8 @@
 // All three layers and their gradients are one GEMM kernel on the tensor
 // cores (mma.sync.m16n8k16 BF16 x BF16 -> FP32) with strided operands (so
 // the transposed products of the backward pass need no copies) and fused
-// epilogues (bias, ReLU, BF16 cast).  FP32 master weights and Adam state;
+// epilogues (bias, ReLU, BF16 cast), and its form for the long contractions
+// over a batch of rows.  FP32 master weights and Adam state;
 // BF16 copies feed the forward pass.  The network is ~6.6 M parameters and
 // runs once per input file, far below the size at which tcgen05 tiles would
 // change anything measurable.
@@ -126,6 +127,121 @@ __global__ void __launch_bounds__(G_THREADS) gemm_bf16(GemmArgs g) {
             }
 }
 
+// ---- long contractions over few rows
+//
+// The forward products and dX = dY W^T have at most a batch of rows and
+// K = 512..8192: one 64 x 64 tile per CTA left 8 CTAs loading element by
+// element, 129..256 dependent steps each (0.2-0.4 ms a product).  Here a CTA
+// takes 16 columns and 64 rows; its warps are 16 x 8 tiles and the operands
+// arrive in 128-deep chunks, four in flight (cp.async, 16 bytes a copy).  The
+// k16 steps of a tile keep their order, so results are the same bits as the
+// 64 x 64 kernel's; splitting K would fill more SMs but round differently.
+// Bound by the chain of dependent MMAs (K / 16) of a tile.  A training step of
+// 32 rows with its copies: 1.66 -> 0.43 ms.
+constexpr int C_M = 64, C_N = 16, C_K = 128, C_STAGES = 4;
+constexpr int C_PITCH = C_K + 8;    // [row][k] chunks: rows of 272 bytes
+constexpr int C_BPITCH = C_N + 8;   // [k][column] chunks of B: rows of 48 bytes
+constexpr int C_A = C_M * C_PITCH;  // elements
+constexpr int C_B = C_K * C_BPITCH > C_N * C_PITCH ? C_K * C_BPITCH : C_N * C_PITCH;
+constexpr size_t C_SMEM = (size_t)C_STAGES * (C_A + C_B) * sizeof(__nv_bfloat16);
+
+__device__ __forceinline__ void copy16(void* smem, const void* gmem, bool valid) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
+    const int n = valid ? 16 : 0;  // the rest of the 16 bytes is zero-filled
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem), "r"(n) : "memory");
+}
+
+// A: row-major, ldA; B: BT ? columns contiguous in k (element (k, n) at
+// B[n * ldb + k]) : rows contiguous in n (B[k * ldb + n]).  ldA, ldb, K (and
+// N without BT) are multiples of 8 and the arrays 16-byte aligned.
+template <bool BT>
+__global__ void __launch_bounds__(256) gemm_chain(GemmArgs g, long lda, long ldb) {
+    extern __shared__ __align__(16) uint8_t c_smem[];
+    __nv_bfloat16* sa = reinterpret_cast<__nv_bfloat16*>(c_smem);
+    __nv_bfloat16* sb = sa + C_STAGES * C_A;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int m0 = blockIdx.y * C_M, n0 = blockIdx.x * C_N;
+    const int wm = (warp >> 1) * 16, wn = (warp & 1) * 8;
+    const int rows = min(C_M, ((g.M - m0 + 15) / 16) * 16);  // staged rows (the launch has 2 warps per 16)
+    const int chunks = (g.K + C_K - 1) / C_K;
+    auto stage = [&](int c) {
+        if (c < chunks) {
+            __nv_bfloat16* da = sa + (c % C_STAGES) * C_A;
+            __nv_bfloat16* db = sb + (c % C_STAGES) * C_B;
+            const int k0 = c * C_K;
+            for (int e = tid; e < rows * (C_K / 8); e += blockDim.x) {
+                const int m = e / (C_K / 8), k = (e % (C_K / 8)) * 8;
+                const bool ok = m0 + m < g.M && k0 + k < g.K;
+                copy16(da + m * C_PITCH + k, ok ? g.A + (long)(m0 + m) * lda + k0 + k : g.A, ok);
+            }
+            for (int e = tid; e < C_K * C_N / 8; e += blockDim.x) {
+                if (BT) {
+                    const int n = e / (C_K / 8), k = (e % (C_K / 8)) * 8;
+                    const bool ok = n0 + n < g.N && k0 + k < g.K;
+                    copy16(db + n * C_PITCH + k, ok ? g.B + (long)(n0 + n) * ldb + k0 + k : g.B, ok);
+                } else {
+                    const int k = e / (C_N / 8), n = (e % (C_N / 8)) * 8;
+                    const bool ok = n0 + n < g.N && k0 + k < g.K;
+                    copy16(db + k * C_BPITCH + n, ok ? g.B + (long)(k0 + k) * ldb + n0 + n : g.B, ok);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int c = 0; c < C_STAGES - 1; ++c) stage(c);
+    for (int c = 0; c < chunks; ++c) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(C_STAGES - 2) : "memory");
+        __syncthreads();  // chunk c is staged; chunk c - 1 is no longer read
+        stage(c + C_STAGES - 1);
+        const __nv_bfloat16* ta = sa + (c % C_STAGES) * C_A + wm * C_PITCH;
+        const __nv_bfloat16* tb = sb + (c % C_STAGES) * C_B;
+#pragma unroll
+        for (int kk = 0; kk < C_K; kk += 16) {
+            uint32_t a[4], b[2];
+            const uint32_t pa =
+                (uint32_t)__cvta_generic_to_shared(ta + (lane & 15) * C_PITCH + kk + (lane >> 4) * 8);
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                         : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
+                         : "r"(pa)
+                         : "memory");
+            const int l = lane & 15;  // lanes 0..15 address the two 8 x 8 halves of B
+            if (BT) {
+                const uint32_t pb =
+                    (uint32_t)__cvta_generic_to_shared(tb + (wn + (l & 7)) * C_PITCH + kk + (l >> 3) * 8);
+                asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n"
+                             : "=r"(b[0]), "=r"(b[1])
+                             : "r"(pb)
+                             : "memory");
+            } else {
+                const uint32_t pb = (uint32_t)__cvta_generic_to_shared(tb + (kk + l) * C_BPITCH + wn);
+                asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
+                             : "=r"(b[0]), "=r"(b[1])
+                             : "r"(pb)
+                             : "memory");
+            }
+            asm volatile(
+                "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
+                "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                : "+f"(acc[0]), "+f"(acc[1]), "+f"(acc[2]), "+f"(acc[3])
+                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+        }
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int m = m0 + wm + (lane >> 2) + (r >= 2 ? 8 : 0);
+        const int n = n0 + wn + (lane & 3) * 2 + (r & 1);
+        if (m >= g.M || n >= g.N) continue;
+        float v = acc[r];
+        if (g.epi == EPI_BIAS || g.epi == EPI_BIAS_RELU) v += g.bias[n];
+        if (g.epi == EPI_BIAS_RELU) v = fmaxf(v, 0.f);
+        g.C[(long)m * g.ldc + n] = v;
+        if (g.Cb) g.Cb[(long)m * g.ldc + n] = __float2bfloat16(v);
+    }
+}
+
 __global__ void to_bf16(const float* x, __nv_bfloat16* y, long n) {
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
         y[i] = __float2bfloat16(x[i]);
@@ -217,6 +333,17 @@ cudaError_t dalloc(T** p, long n) {
 void gemm(cudaStream_t st, const __nv_bfloat16* A, long sa0, long sa1, const __nv_bfloat16* B, long sb0, long sb1,
           float* C, __nv_bfloat16* Cb, long ldc, const float* bias, int M, int N, int K, int epi) {
     GemmArgs g{A, B, C, Cb, bias, M, N, K, sa0, sa1, sb0, sb1, ldc, epi};
+    // rows of A contiguous in k, 16-byte copies possible, and a contraction
+    // long enough for the chunks (the weight gradients contract a batch)
+    const bool bt = sb0 == 1;
+    if (sa1 == 1 && sa0 % 8 == 0 && K % 8 == 0 && K >= C_K &&
+        (bt ? sb1 % 8 == 0 : sb1 == 1 && sb0 % 8 == 0 && N % 8 == 0)) {
+        const dim3 grid((N + C_N - 1) / C_N, (M + C_M - 1) / C_M);
+        const int warps = 2 * ((std::min(M, C_M) + 15) / 16);
+        if (bt) gemm_chain<true><<<grid, warps * 32, C_SMEM, st>>>(g, sa0, sb1);
+        else gemm_chain<false><<<grid, warps * 32, C_SMEM, st>>>(g, sa0, sb0);
+        return;
+    }
     dim3 grid((N + GN - 1) / GN, (M + GM - 1) / GM);
     gemm_bf16<<<grid, G_THREADS, 0, st>>>(g);
 }
@@ -323,7 +450,8 @@ int kc_mlp_create(int in, int hid, int out, int max_batch, uint64_t seed, kc_mlp
         g_mlp_err = "stream creation failed";
         return KC_ERR_DEVICE;
     }
-    bool ok = true;
+    bool ok = cudaFuncSetAttribute(gemm_chain<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C_SMEM) == cudaSuccess &&
+              cudaFuncSetAttribute(gemm_chain<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C_SMEM) == cudaSuccess;
     for (int l = 0; l < 3; ++l) {
         m->nW[l] = (long)dims[l] * dims[l + 1];
         m->nb[l] = dims[l + 1];
