@@ -360,6 +360,8 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) count_window(WindowArgs a) {
     unsigned long long* s_key = reinterpret_cast<unsigned long long*>(win_smem);
     uint32_t* s_cnt = reinterpret_cast<uint32_t*>(win_smem + (size_t)WIN_CELLS * 8);
     uint32_t* s_pad = s_cnt + WIN_CELLS;
+    __shared__ uint32_t s_full;  // a key of this window has met a full probe window
+    if (threadIdx.x == 0) s_full = 0;
 
     const uint32_t r = a.order[a.order_base + blockIdx.x];
     const WinInfo wi = a.wins[r];
@@ -451,6 +453,7 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) count_window(WindowArgs a) {
             if (!reps) continue;
             bool done = false;
             for (uint32_t p = 0; p < limit; ++p) {
+                if (p && p % PROBE_CHECK == 0 && *reinterpret_cast<volatile uint32_t*>(&s_full)) break;
                 const uint32_t c = single ? (uint32_t)((local + p) & M) : local + p;
                 unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&s_key[c]);
                 if (cur == EMPTY) {
@@ -466,6 +469,7 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) count_window(WindowArgs a) {
             if (!done) {
                 fail_bits |= 1u << j;
                 mult[j] = reps;  // occurrences still to add after the table grows
+                s_full = 1u;
                 a.bucket_overflow[wi.bucket] = 1u;
             }
         }
