@@ -1088,7 +1088,8 @@ int count_and_pack(kc_context* c, uint64_t n_keys, uint32_t ext_err) {
     }
     {
         Stage st(c, KC_STAGE_PACK_LOW);
-        kc::pack_low<NW><<<resident_grid(c, kc::pack_low<NW>, 256, ceil_div(nsegs, 256)), 256, 0, c->stream>>>(
+        auto pack = c->packed_bytes % 8 ? kc::pack_low<NW, false> : kc::pack_low<NW, true>;
+        pack<<<resident_grid(c, pack, 256, ceil_div(nsegs, 256)), 256, 0, c->stream>>>(
             c->routed.p, c->tile_low.as<uint32_t>(), c->tile_low_prefix.as<uint64_t>(), nsegs, c->cfg.k, low_dst,
             low_base);
     }

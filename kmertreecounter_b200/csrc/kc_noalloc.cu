@@ -267,8 +267,8 @@ int run(const kc_config* g, const uint8_t* d_fastq, uint64_t n, uint8_t* d_low, 
     if ((ts * sizeof(SlotT) + nch * sizeof(kc::ExportChunk) + 256) > tab_cap * sizeof(SlotT))
         return err(KC_ERR_OVERFLOW, "no-alloc scratch exhausted at export");
     if (nsegs)
-        kc::pack_low<NW><<<std::min<uint64_t>(cdiv(nsegs, 256), 148 * 4), 256, 0, st>>>(routed, seg_low, seg_prefix,
-                                                                                       nsegs, k, d_low, 0);
+        (kc_packed_bytes(k) % 8 ? kc::pack_low<NW, false> : kc::pack_low<NW, true>)<<<
+            std::min<uint64_t>(cdiv(nsegs, 256), 148 * 4), 256, 0, st>>>(routed, seg_low, seg_prefix, nsegs, k, d_low, 0);
 
     // root records grouped by root id
     NKS(cudaMemcpyAsync(chunks, h_chunks, nch * sizeof(kc::ExportChunk), cudaMemcpyHostToDevice, st));
