@@ -132,6 +132,7 @@ struct kc_context {
     cudaStream_t side = nullptr;
     cudaEvent_t ev_side_in = nullptr, ev_init = nullptr;
     bool init_pending = false;
+    bool init_deferred = false;  // tables not initialised: the windowed count of the first batch writes every cell
     uint32_t nw = 1, bucket_bits = 8, n_buckets = 256, bucket_shift = 56;
     int sm_count = 148;
     uint64_t slot_bytes = 16, record_bytes = 16, packed_bytes = 8;
@@ -437,6 +438,24 @@ int device_scan(kc_context* c, const TI* in, uint64_t n, TO* out, uint64_t base,
     return KC_OK;
 }
 
+// Windows pay a read and a write of every table cell per batch: worth it from
+// 2 keys per cell, e.g. a whole input in one pass, not for the host path's
+// batches against the whole input's tables.
+bool windows_pay(const kc_context* c, uint64_t n_keys) {
+    return c->window_count && n_keys >= 2 * c->table_slots_used;
+}
+
+// Initialisation put off in the hope of a windowed count, when the batch is
+// counted by the global kernel after all.
+int init_now(kc_context* c) {
+    if (!c->init_deferred) return KC_OK;
+    c->init_deferred = false;
+    Stage st(c, KC_STAGE_INIT);
+    kc::init_slots<1><<<c->sm_count * 8, 256, 0, c->stream>>>(c->table.p, c->table_slots_used);
+    CK(cudaGetLastError());
+    return KC_OK;
+}
+
 // Allocate filter and tables from per-bucket k-mer totals of the first batch
 // (batch_bytes of FASTQ; 0 when no extraction follows).
 int size_structures(kc_context* c, const std::vector<uint64_t>& kb, double scale, uint64_t batch_bytes) {
@@ -497,10 +516,17 @@ int size_structures(kc_context* c, const std::vector<uint64_t>& kb, double scale
         // the count joins it.  Otherwise it runs first at full width: 48 GB
         // of 128-bit tables behind a 2 GiB batch slowed that batch's
         // extraction and still held up the count.
+        //
+        // 64-bit keys that will be counted in windows (their number estimated
+        // from the histogram) need none: the windowed count starts its cells
+        // EMPTY and writes them all.
         const uint64_t init_bytes = bw * sizeof(uint64_t) + ts * c->slot_bytes;
+        uint64_t batch_keys = 0;
+        for (uint32_t b = 0; b < nb; ++b) batch_keys += kb[b];
+        c->init_deferred = c->nw == 1 && windows_pay(c, batch_keys);
         const bool beside = init_bytes < 4 * batch_bytes;
         cudaStream_t is = c->stream;
-        if (beside) {
+        if (beside && !c->init_deferred) {
             // after the work queued before this batch's extraction (recorded
             // before it when sizing follows the extraction's launch)
             if (!c->side_in_ready) CK(cudaEventRecord(c->ev_side_in, c->stream));
@@ -508,16 +534,18 @@ int size_structures(kc_context* c, const std::vector<uint64_t>& kb, double scale
             is = c->side;
         }
         c->side_in_ready = false;
-        Stage st(c, KC_STAGE_INIT, bw ? 2 : 1, is);
-        const int ig = c->sm_count * (beside ? 2 : 8);
-        if (bw) kc::zero16<<<ig, 256, 0, is>>>(c->bloom.as<uint4>(), bw / 2);  // bw: a sum of powers of two >= 256
-        if (c->nw == 1) kc::init_slots<1><<<ig, 256, 0, is>>>(c->table.p, ts);
-        else if (c->nw == 2) kc::init_slots<2><<<ig, 256, 0, is>>>(c->table.p, ts);
-        else kc::init_slots<4><<<ig, 256, 0, is>>>(c->table.p, ts);
-        CK(cudaGetLastError());
-        if (beside) {
-            CK(cudaEventRecord(c->ev_init, c->side));
-            c->init_pending = true;
+        if (!c->init_deferred) {
+            Stage st(c, KC_STAGE_INIT, bw ? 2 : 1, is);
+            const int ig = c->sm_count * (beside ? 2 : 8);
+            if (bw) kc::zero16<<<ig, 256, 0, is>>>(c->bloom.as<uint4>(), bw / 2);  // bw: a sum of powers of two >= 256
+            if (c->nw == 1) kc::init_slots<1><<<ig, 256, 0, is>>>(c->table.p, ts);
+            else if (c->nw == 2) kc::init_slots<2><<<ig, 256, 0, is>>>(c->table.p, ts);
+            else kc::init_slots<4><<<ig, 256, 0, is>>>(c->table.p, ts);
+            CK(cudaGetLastError());
+            if (beside) {
+                CK(cudaEventRecord(c->ev_init, c->side));
+                c->init_pending = true;
+            }
         }
     }
     CK(c->overflow.ensure(nb * sizeof(uint32_t)));
@@ -810,6 +838,8 @@ int window_count(kc_context* c, uint64_t& n_keys) {
     a.seg_low = c->tile_low.as<uint32_t>();
     a.seg_fail = c->tile_fail.as<uint32_t>();
     a.bucket_overflow = c->overflow.as<uint32_t>();
+    a.fresh = c->init_deferred;
+    c->init_deferred = false;
     {
         Stage st(c, KC_STAGE_COUNT_ROUTED, 2);
         for (uint32_t ph = 0; ph < 2; ++ph) {
@@ -1035,15 +1065,15 @@ int count_and_pack(kc_context* c, uint64_t n_keys, uint32_t ext_err) {
     if constexpr (NW == 1) {
         // 64-bit keys count in shared-memory windows while every bucket's
         // filter sits in its table's cells (no table has grown yet)
-        // (windows pay a read and a write of every table cell per batch:
-        // worth it from 2 keys per cell, e.g. a whole input in one pass,
-        // not for the host path's batches against the whole input's tables)
-        if (c->window_count && n_keys >= 2 * c->table_slots_used && (c->win_ready || build_windows(c))) {
+        if (windows_pay(c, n_keys) && (c->win_ready || build_windows(c))) {
             if ((rc = window_count(c, n_keys))) return rc;
             windowed = true;
         }
     }
-    if (!windowed) launch_count<NW>(c, n_keys, 1);
+    if (!windowed) {
+        CKR(init_now(c));
+        launch_count<NW>(c, n_keys, 1);
+    }
     const uint64_t nsegs = ceil_div(n_keys, SEG);
     CK(cudaGetLastError());
     if ((rc = rehash_loop<NW>(c, n_keys))) return rc;
@@ -1212,6 +1242,7 @@ int begin_run(kc_context* c, uint64_t total_bytes) {
     c->have_result = false;
     c->batch_result = false;
     c->win_result = false;
+    c->init_deferred = false;
     c->expected_total_bytes = total_bytes;
     c->ev_used = 0;
     c->spans.clear();
