@@ -119,6 +119,9 @@ inline uint64_t pow2_at_least(uint64_t x) { return std::bit_ceil(std::max<uint64
 
 }  // namespace
 
+// Routed keys of a multi-set pass from which it is counted in windows.
+constexpr uint64_t SETS_WINDOW_KEYS = 4ull << 20;
+
 // Histogram bins kept in the context between kc_histogram calls.
 constexpr uint64_t HIST_KEEP_BYTES = 256ull << 10;
 
@@ -671,8 +674,7 @@ int rehash_loop(kc_context* c, uint64_t n_keys) {
 // table have parted (a table that grew after an overflow keeps its old cells
 // as the filter): the windowed count needs the filter word in the first probe
 // cell of the key's own table.
-bool build_windows(kc_context* c) {
-    const uint32_t nb = c->n_buckets;
+bool build_windows(kc_context* c, uint32_t nb) {
     c->h_bucket_win.assign(nb, kc::BucketWin{});
     c->h_win_info.clear();
     for (uint32_t b = 0; b < nb; ++b) {
@@ -732,15 +734,17 @@ void launch_count_range(kc_context* c, uint64_t off, uint64_t n, int use_filter)
 // windows first, then the spilled keys with count_routed.  `routed` then
 // holds the window-grouped keys with per-segment first occurrences and
 // overflowed keys as count_routed leaves them, and n_keys becomes its length.
-int window_count(kc_context* c, uint64_t& n_keys) {
+// A multi-set batch (sets.n sets, nb = 256 buckets each) takes exact ranges:
+// a spill area would mix the sets' keys.
+int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets = {nullptr, 0}) {
     const uint64_t nw = c->n_wins;
     if (!c->win_ready) {
-        CK(c->bucket_win.ensure(c->n_buckets * sizeof(kc::BucketWin)));
+        CK(c->bucket_win.ensure(nb * sizeof(kc::BucketWin)));
         CK(c->win_info.ensure(nw * sizeof(kc::WinInfo)));
         CK(c->win_order.ensure(nw * sizeof(uint32_t)));
         CK(cudaMemcpyAsync(c->win_order.p, c->h_win_order.data(), nw * sizeof(uint32_t), cudaMemcpyHostToDevice,
                            c->stream));
-        CK(cudaMemcpyAsync(c->bucket_win.p, c->h_bucket_win.data(), c->n_buckets * sizeof(kc::BucketWin),
+        CK(cudaMemcpyAsync(c->bucket_win.p, c->h_bucket_win.data(), nb * sizeof(kc::BucketWin),
                            cudaMemcpyHostToDevice, c->stream));
         CK(cudaMemcpyAsync(c->win_info.p, c->h_win_info.data(), nw * sizeof(kc::WinInfo), cudaMemcpyHostToDevice,
                            c->stream));
@@ -758,7 +762,7 @@ int window_count(kc_context* c, uint64_t& n_keys) {
     const uint64_t cchunks = ceil_div(n_keys, kc::SUB_CHUNK);
     const uint64_t small_grid = std::min<uint64_t>(ceil_div(nw, 256), (uint64_t)c->sm_count * 8);
     // sampled ranges need enough sampled chunks per window to be worth it
-    uint32_t stride = cchunks >= 64ull * 16 ? 16u : 1u;
+    uint32_t stride = cchunks >= 64ull * 16 && !sets.n ? 16u : 1u;
     uint64_t total = 0, spill_start = 0, spill_used = 0;
     for (;;) {
         CKR(fill_dev(c, c->win_count.p, nw * sizeof(uint32_t), 0));
@@ -767,7 +771,7 @@ int window_count(kc_context* c, uint64_t& n_keys) {
             const uint64_t g = ceil_div(cchunks, stride);
             if (g)
                 kc::subroute_count<<<g, kc::SUB_THREADS, 0, c->stream>>>(
-                    c->routed.as<uint64_t>(), n_keys, meta, bwin, c->bucket_shift, stride, c->win_count.as<uint32_t>());
+                    c->routed.as<uint64_t>(), n_keys, meta, bwin, c->bucket_shift, stride, sets, c->win_count.as<uint32_t>());
             kc::window_caps<<<small_grid, 256, 0, c->stream>>>(c->win_count.as<uint32_t>(), nw, stride,
                                                                 c->win_padded.as<uint32_t>());
             CK(cudaGetLastError());
@@ -803,9 +807,10 @@ int window_count(kc_context* c, uint64_t& n_keys) {
             sa.spill_end = arr;
             sa.spill_full = d_spill_full;
             sa.out = c->routed2.as<uint64_t>();
+            sa.sets = sets;
             if (n_keys)
-                kc::subroute_scatter<<<ceil_div(n_keys, kc::SCAT_CHUNK), kc::SCAT_THREADS, kc::scatter_smem_bytes(),
-                                       c->stream>>>(sa);
+                (sets.n ? kc::subroute_scatter<true> : kc::subroute_scatter<false>)<<<
+                    ceil_div(n_keys, kc::SCAT_CHUNK), kc::SCAT_THREADS, kc::scatter_smem_bytes(), c->stream>>>(sa);
             CK(cudaGetLastError());
         }
         uint32_t full = 0;
@@ -1065,8 +1070,8 @@ int count_and_pack(kc_context* c, uint64_t n_keys, uint32_t ext_err) {
     if constexpr (NW == 1) {
         // 64-bit keys count in shared-memory windows while every bucket's
         // filter sits in its table's cells (no table has grown yet)
-        if (windows_pay(c, n_keys) && (c->win_ready || build_windows(c))) {
-            if ((rc = window_count(c, n_keys))) return rc;
+        if (windows_pay(c, n_keys) && (c->win_ready || build_windows(c, c->n_buckets))) {
+            if ((rc = window_count(c, n_keys, c->n_buckets))) return rc;
             windowed = true;
         }
     }
@@ -1555,8 +1560,8 @@ int kc_create(const kc_config* cfg, kc_context** out) {
     cudaFuncSetAttribute(kc::loads_table_pass<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::loads_table_smem());
     cudaFuncSetAttribute(kc::loads_table_pass<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::loads_table_smem());
     cudaFuncSetAttribute(kc::loads_table_pass<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::loads_table_smem());
-    cudaFuncSetAttribute(kc::subroute_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kc::scatter_smem_bytes());
+    for (auto k : {kc::subroute_scatter<false>, kc::subroute_scatter<true>})
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::scatter_smem_bytes());
     if ((e = cudaGetLastError()) != cudaSuccess) {
         delete c;
         return fail(KC_ERR_DEVICE, "kernel attribute setup failed: %s", cudaGetErrorString(e));
@@ -2277,7 +2282,7 @@ int count_sets_impl(kc_context* c, const uint8_t* buf, const kc_set_desc* sets, 
     CK(c->tile_prefix.ensure(std::max<uint64_t>(nt, 1) * sizeof(uint64_t)));
     CK(c->scalars.ensure(64));
     uint64_t* d_scal = c->scalars.as<uint64_t>();
-    CK(cudaMemsetAsync(c->scalars.as<uint32_t>() + 12, 0, sizeof(uint32_t), c->stream));
+    CK(cudaMemsetAsync(c->scalars.as<uint32_t>() + 12, 0, 2 * sizeof(uint32_t), c->stream));
     if (nt) CK(cudaMemcpyAsync(c->set_tiles.p, tiles.data(), nt * sizeof(kc::SetTile), cudaMemcpyHostToDevice, c->stream));
     const kc::SetTile* d_tiles = c->set_tiles.as<kc::SetTile>();
     int rc;
@@ -2389,8 +2394,13 @@ route_again:
                 words = pow2_at_least(std::max<uint64_t>((uint64_t)(kb * g.bloom_bits / 64.0), 64));
                 slots = pow2_at_least(std::max<uint64_t>((uint64_t)(kb * g.repeat_ratio / g.table_load), 64));
             }
-            c->h_meta[(uint64_t)s * NB + b] = kc::BucketMeta{bw, words - 1, ts, slots - 1};
-            bw += words;
+            if (NW == 1) {  // the filter words are the cells' pad fields, as for one input
+                slots = std::max<uint64_t>(slots, 2 * words);
+                c->h_meta[q] = kc::BucketMeta{ts, slots - 1, ts, slots - 1};
+            } else {
+                c->h_meta[q] = kc::BucketMeta{bw, words - 1, ts, slots - 1};
+                bw += words;
+            }
             ts += slots;
         }
         ovf_start[s] = pos;
@@ -2398,22 +2408,34 @@ route_again:
         ovf_end[s] = pos;
         set_key1[s] = pos;
     }
-    const uint64_t n_keys = ceil_div(pos, SEG) * SEG;
+    uint64_t n_keys = ceil_div(pos, SEG) * SEG;
     for (uint32_t s = 0; s < n_sets; ++s) set_next[s] = (s + 1 < n_sets) ? set_key0[s + 1] : n_keys;
     c->K = K;
-    c->bloom_words = bw;
+    c->bloom_words = NW == 1 ? ts / 2 : bw;
     c->table_slots_used = ts;
     CK(c->bloom.ensure(bw * sizeof(uint64_t)));
     CK(c->table.ensure(ts * c->slot_bytes + ts * c->slot_bytes / 4));  // room for a few in-place growths
     CK(c->meta.ensure(nbk * sizeof(kc::BucketMeta)));
     CK(c->overflow.ensure(nbk * sizeof(uint32_t)));
-    const uint64_t nsegs = n_keys / SEG;
+    // 64-bit keys of a large pass are counted in windows (the rule for one
+    // input; SETS_WINDOW_KEYS keys pay for the extra launches and the exact
+    // window counts) while the second key buffer fits the device: 48 sets of
+    // 10k-300k reads, 543 M k-mers, 34.6 ms by the global count, 22.3 in windows
+    bool windowed = NW == 1 && n_keys >= SETS_WINDOW_KEYS && windows_pay(c, n_keys) && build_windows(c, (uint32_t)nbk);
+    if (windowed && c->routed2.ensure((n_keys + c->n_wins * kc::WIN_SEG) * sizeof(KeyT)) != cudaSuccess) {
+        cudaGetLastError();
+        windowed = false;
+    }
+    c->win_ready = false;
+    c->init_deferred = windowed;
+    uint64_t nsegs = n_keys / SEG;
     CK(c->routed.ensure(std::max<uint64_t>(ceil_div(n_keys, CT) * CT, 1) * sizeof(KeyT)));
     CK(c->tile_low.ensure(std::max<uint64_t>(nsegs, 1) * sizeof(uint32_t)));
     CK(c->tile_fail.ensure(std::max<uint64_t>(nsegs, 1) * sizeof(uint32_t)));
     CK(c->tile_low_prefix.ensure(std::max<uint64_t>(nsegs, 1) * sizeof(uint64_t)));
-    CK(c->set_info.ensure((size_t)n_sets * 9 * sizeof(uint64_t) + 64));
-    uint64_t* d_seg = c->set_info.as<uint64_t>();              // set_seg_start[n_sets]
+    CK(c->set_info.ensure((size_t)n_sets * 10 * sizeof(uint64_t) + 64));
+    uint64_t* d_key0 = c->set_info.as<uint64_t>();             // windows: set_key0[n_sets]
+    uint64_t* d_seg = d_key0 + n_sets;                         // set_seg_start[n_sets]
     uint64_t* d_end = d_seg + n_sets;                          // set_key1
     uint64_t* d_next = d_end + n_sets;                         // next set's first key
     uint64_t* d_low = d_next + n_sets;                         // low count per set
@@ -2451,8 +2473,8 @@ route_again:
     }
     {
         Stage st(c, KC_STAGE_INIT, 1);
-        CK(cudaMemsetAsync(c->bloom.p, 0, bw * sizeof(uint64_t), c->stream));
-        kc::init_slots<NW><<<c->sm_count * 8, 256, 0, c->stream>>>(c->table.p, ts);
+        if (bw) CK(cudaMemsetAsync(c->bloom.p, 0, bw * sizeof(uint64_t), c->stream));
+        if (!windowed) kc::init_slots<NW><<<c->sm_count * 8, 256, 0, c->stream>>>(c->table.p, ts);
         CK(cudaMemsetAsync(c->overflow.p, 0, nbk * sizeof(uint32_t), c->stream));
     }
     CK(cudaGetLastError());
@@ -2472,9 +2494,11 @@ route_again:
     ca.n_sets = n_sets;
     ca.set_buckets = NB;
     ca.use_filter = 1;
-    const uint64_t cgrid = ceil_div(n_keys, (uint64_t)CT * kc::CNT_SEGS_PER_WARP);
+    ca.filter_in_table = NW == 1;
+    ca.error = c->scalars.as<uint32_t>() + 13;
+    uint64_t cgrid = ceil_div(n_keys, (uint64_t)CT * kc::CNT_SEGS_PER_WARP);
 
-    // scatter -> gap fill(s) -> count as one graph.  The context keeps the
+    // scatter -> gap fill(s) -> count (unless in windows) as one graph.  The context keeps the
     // instantiated graph of each shape: a later call captures its own
     // launches (the same kernels, new arguments and grids) and updates the
     // instantiated graph of its shape in place (cudaGraphExecUpdate),
@@ -2494,12 +2518,12 @@ route_again:
                 c->region_end.as<unsigned long long>(), (uint32_t)nbk);
         // and after each set's keys (its overflow area's unused part, the alignment gap)
         kc::fill_set_gaps<NW><<<n_sets, 256, 0, c->stream>>>(c->routed.p, d_ovc, d_next, n_sets);
-        if (cgrid) kc::count_routed<NW><<<cgrid, kc::CNT_THREADS, 0, c->stream>>>(ca);
+        if (cgrid && !windowed) kc::count_routed<NW><<<cgrid, kc::CNT_THREADS, 0, c->stream>>>(ca);
         const cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
         if (ce != cudaSuccess) return fail(KC_ERR_DEVICE, "graph capture failed: %s", cudaGetErrorString(ce));
         cudaError_t e = cudaSuccess;
         bool updated = false;
-        const int nodes = (nt ? 1 : 0) + (any_sampled ? 1 : 0) + 1 + (cgrid ? 1 : 0);
+        const int nodes = (nt ? 1 : 0) + (any_sampled ? 1 : 0) + 1 + (cgrid && !windowed ? 1 : 0);
         const int key = NW * 16 + nodes + (any_sampled ? 8 : 0);
         int slot = -1;
         for (int i = 0; i < kc_context::SETS_EXECS; ++i)
@@ -2550,6 +2574,22 @@ route_again:
         }
         c->K = K;
     }
+    if constexpr (NW == 1) {
+        if (windowed) {
+            CK(cudaMemcpyAsync(d_key0, set_key0.data(), n_sets * sizeof(uint64_t), cudaMemcpyHostToDevice, c->stream));
+            if ((rc = window_count(c, n_keys, (uint32_t)nbk, kc::SetSpan{d_key0, n_sets}))) return rc;
+            c->win_ready = false;
+            nsegs = n_keys / SEG;
+            kc::set_window_segs<<<std::max<uint64_t>(1, ceil_div(n_sets, 256)), 256, 0, c->stream>>>(
+                c->bucket_win.as<kc::BucketWin>(), c->win_start.as<uint64_t>(), n_sets, d_seg);
+            CK(cudaGetLastError());
+            ca.routed = c->routed.p;
+            ca.n_keys = n_keys;
+            ca.seg_low = c->tile_low.as<uint32_t>();
+            ca.seg_fail = c->tile_fail.as<uint32_t>();
+            cgrid = ceil_div(n_keys, (uint64_t)CT * kc::CNT_SEGS_PER_WARP);
+        }
+    }
 
     // overflowed tables: grow x4, move, retry only the failed keys
     for (int round = 0;; ++round) {
@@ -2582,10 +2622,11 @@ route_again:
     CK(cudaGetLastError());
     std::vector<uint64_t> lows(n_sets);
     CK(cudaMemcpyAsync(lows.data(), d_low, n_sets * sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream));
-    uint32_t ext_err = 0;
-    CK(cudaMemcpyAsync(&ext_err, c->scalars.as<uint32_t>() + 12, sizeof ext_err, cudaMemcpyDeviceToHost, c->stream));
+    uint32_t err[2] = {0, 0};  // extraction and count error words
+    CK(cudaMemcpyAsync(err, c->scalars.as<uint32_t>() + 12, sizeof err, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    if (ext_err) return fail(KC_ERR_DEVICE, "internal error: routing bucket disagreed with its reservation");
+    if (err[0]) return fail(KC_ERR_DEVICE, "internal error: routing bucket disagreed with its reservation");
+    if (err[1]) return fail(KC_ERR_DEVICE, "internal error: a 256-bit table slot was never published");
     std::vector<uint64_t> lowbase(n_sets);
     uint64_t lb = 0, total_low = 0;
     for (uint32_t s = 0; s < n_sets; ++s) {  // each set's low.bin bytes start 16-byte aligned

@@ -91,6 +91,22 @@ __device__ __forceinline__ uint32_t window_of(uint64_t key, uint32_t bucket_shif
     return w.range_base + (w.zshift >= WIN_SINGLE ? 0u : (uint32_t)(cell >> w.zshift));
 }
 
+// The sets of a multi-set batch: set s's keys start at start[s] and use the
+// 256 buckets from 256 s on.  n = 0: one input.
+struct SetSpan {
+    const uint64_t* start;
+    uint32_t n;
+};
+__device__ __forceinline__ uint32_t first_bucket(const SetSpan& sets, uint64_t i) {
+    uint32_t lo = 0, hi = sets.n;  // the last set that starts at or before key i
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) / 2;
+        if (__ldg(sets.start + mid) <= i) lo = mid;
+        else hi = mid;
+    }
+    return lo * 256;
+}
+
 // Smallest bucket of the chunk's keys (EMPTY keys skipped); 0xFFFFFFFF if none.
 __device__ __forceinline__ uint32_t chunk_min_bucket(const uint64_t (&k)[SUB_ITEMS], uint32_t bucket_shift,
                                                      uint32_t* s_min) {
@@ -113,7 +129,8 @@ __device__ __forceinline__ uint32_t chunk_min_bucket(const uint64_t (&k)[SUB_ITE
 __global__ void __launch_bounds__(SUB_THREADS) subroute_count(const uint64_t* __restrict__ keys, uint64_t n,
                                                              const BucketMeta* __restrict__ meta,
                                                              const BucketWin* __restrict__ bw, uint32_t bucket_shift,
-                                                             uint32_t chunk_stride, uint32_t* __restrict__ win_count) {
+                                                             uint32_t chunk_stride, SetSpan sets,
+                                                             uint32_t* __restrict__ win_count) {
     __shared__ uint32_t hist[SUB_BINS];
     __shared__ uint32_t s_min;
     const uint64_t c0 = (uint64_t)blockIdx.x * chunk_stride * SUB_CHUNK;
@@ -125,7 +142,27 @@ __global__ void __launch_bounds__(SUB_THREADS) subroute_count(const uint64_t* __
         const uint64_t i = c0 + (uint64_t)j * SUB_THREADS + threadIdx.x;
         k[j] = i < n ? __ldcs(keys + i) : EMPTY;
     }
+    bool split = false;  // a chunk that lies in several sets: every key by itself
+    if (sets.n) {
+        const uint32_t first = first_bucket(sets, c0);
+        split = first != first_bucket(sets, min(c0 + SUB_CHUNK, n) - 1);
+        if (!split) {
+            meta += first;
+            bw += first;
+        }
+    }
     __syncthreads();
+    if (split) {
+#pragma unroll 1
+        for (int j = 0; j < SUB_ITEMS; ++j) {
+            const uint64_t i = c0 + (uint64_t)j * SUB_THREADS + threadIdx.x;
+            const uint64_t key = i < n ? keys[i] : EMPTY;
+            if (key == EMPTY) continue;
+            const uint32_t b = first_bucket(sets, i);
+            atomicAdd(&win_count[window_of(key, bucket_shift, WinCache{0xFFFFFFFFu, {}, 0}, meta + b, bw + b)], 1u);
+        }
+        return;  // block-uniform
+    }
     const uint32_t bmin = chunk_min_bucket(k, bucket_shift, &s_min);
     if (bmin == 0xFFFFFFFFu) return;  // block-uniform: no key in this chunk
     const WinCache wc{bmin, bw[bmin], __ldg(&meta[bmin].tab_mask)};
@@ -156,6 +193,13 @@ __global__ void window_caps(const uint32_t* __restrict__ cnt, uint64_t n, uint32
         }
         cap[i] = (uint32_t)min((c + (WIN_SEG - 1)) & ~(uint64_t)(WIN_SEG - 1), (uint64_t)0xFFFFFFC0u);
     }
+}
+
+// First output segment of every set: that of its first window.
+__global__ void set_window_segs(const BucketWin* __restrict__ bw, const uint64_t* __restrict__ start, uint32_t n_sets,
+                                uint64_t* __restrict__ seg) {
+    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n_sets; s += gridDim.x * blockDim.x)
+        seg[s] = start[bw[256 * s].range_base] / WIN_SEG;
 }
 
 // cursor = start; end = start + cap, for every window.
@@ -189,6 +233,7 @@ struct ScatterArgs {
     uint64_t spill_end;
     uint32_t* spill_full;            // set when the spill area overflowed
     uint64_t* out;
+    SetSpan sets;
 };
 
 // Keys into their window's range.  A chunk of 4096 keys is counted per
@@ -206,6 +251,7 @@ struct ScatterArgs {
 // genome shape (1163 M keys, 18.6 GB): 6.84 -> 5.94 ms, 0.48 of the copy
 // bandwidth, by the 32-bit window, five barriers instead of eight and one
 // addition per key written.
+template <bool SETS>
 __global__ void __launch_bounds__(SCAT_THREADS, 3) subroute_scatter(ScatterArgs a) {
     extern __shared__ __align__(16) uint8_t sc_smem[];
     uint64_t* stage = reinterpret_cast<uint64_t*>(sc_smem);
@@ -250,16 +296,30 @@ __global__ void __launch_bounds__(SCAT_THREADS, 3) subroute_scatter(ScatterArgs 
     __syncthreads();
     const uint32_t top_shift = a.bucket_shift - 32;
     const uint32_t bmin = s_min >> top_shift, bmax = s_max >> top_shift;
-    const BucketWin bwin = a.bw[bmin];
-    const uint64_t bmask = __ldg(&a.meta[bmin].tab_mask);
+    const BucketMeta* meta = a.meta;
+    const BucketWin* bw = a.bw;
+    bool split = false;  // a chunk that lies in several sets: every key's own set, bins from the first one's windows on
+    if constexpr (SETS) {
+        const uint32_t first = first_bucket(a.sets, c0);
+        split = first != first_bucket(a.sets, min(c0 + SCAT_CHUNK, a.n) - 1);
+        meta += first;
+        bw += first;
+    }
+    const BucketWin bwin = bw[split ? 0 : bmin];
+    const uint64_t bmask = __ldg(&meta[bmin].tab_mask);
     const uint32_t r0 = bwin.range_base;
+    const WinCache wc{split ? 0xFFFFFFFFu : bmin, bwin, bmask};
+    auto general_window = [&](uint64_t key, int j) {
+        if (!SETS || !split) return window_of(key, a.bucket_shift, wc, meta, bw);
+        const uint32_t b = first_bucket(a.sets, c0 + (uint64_t)j * SCAT_THREADS + tid);
+        return window_of(key, a.bucket_shift, wc, a.meta + b, a.bw + b);
+    };
     // per key: staged bin (high 16 bits) and place inside it (low 16), or
     // FAR for a window outside the staged span (placed one by one later)
     constexpr uint32_t FAR = 0xFFFFFFFFu;
     uint32_t slot[SCAT_ITEMS];
     uint32_t bins = SCAT_BINS;
-    const bool uniform = bmin == bmax && bmin != (0xFFFFFFFFu >> top_shift);
-    const WinCache wc{bmin, bwin, bmask};
+    const bool uniform = !split && bmin == bmax && bmin != (0xFFFFFFFFu >> top_shift);
     if (uniform) {
         // windows of at most 2^32 cells: 32-bit arithmetic
         const uint32_t wmask = bwin.zshift >= WIN_SINGLE ? 0u : (uint32_t)bmask;
@@ -274,7 +334,7 @@ __global__ void __launch_bounds__(SCAT_THREADS, 3) subroute_scatter(ScatterArgs 
         for (int j = 0; j < SCAT_ITEMS; ++j) {
             slot[j] = FAR;
             if (k[j] == EMPTY) continue;
-            const uint32_t l = window_of(k[j], a.bucket_shift, wc, a.meta, a.bw) - r0;
+            const uint32_t l = general_window(k[j], j) - r0;
             if (l < (uint32_t)SCAT_BINS) slot[j] = (l << 16) | atomicAdd(&hist[l], 1u);
         }
     }
@@ -327,7 +387,7 @@ __global__ void __launch_bounds__(SCAT_THREADS, 3) subroute_scatter(ScatterArgs 
             stage[pos] = k[j];
             stage_bin[pos] = (uint16_t)l;
         } else if (k[j] != EMPTY) {  // far window: one key at a time
-            const uint32_t w = window_of(k[j], a.bucket_shift, wc, a.meta, a.bw);
+            const uint32_t w = general_window(k[j], j);
             const unsigned long long g = atomicAdd(&a.win_cursor[w], 1ull);
             if (g < a.win_end[w]) {
                 a.out[g] = k[j];
