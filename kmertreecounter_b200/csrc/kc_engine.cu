@@ -122,6 +122,11 @@ inline uint64_t pow2_at_least(uint64_t x) { return std::bit_ceil(std::max<uint64
 // Routed keys of a multi-set pass from which it is counted in windows.
 constexpr uint64_t SETS_WINDOW_KEYS = 4ull << 20;
 
+// A last batch whose keys (packed) and tables take at most this much is packed
+// and exported without waiting for its counts (count_and_pack): the bounds of
+// both outputs are allocated.  1000 reads: three waits of ~12 us in 260.
+constexpr uint64_t SMALL_BYTES = 32ull << 20;
+
 // Histogram bins kept in the context between kc_histogram calls.
 constexpr uint64_t HIST_KEEP_BYTES = 256ull << 10;
 
@@ -231,6 +236,7 @@ struct kc_context {
     std::vector<uint32_t> h_overflow;
     uint64_t bloom_words = 0, table_slots_used = 0;
     bool sized = false;
+    bool end_recorded = false;  // ev1 follows the run's last launch, and has been waited for
     uint64_t expected_total_bytes = 0;
 
     // run state
@@ -264,6 +270,21 @@ struct kc_context {
         uint64_t off, bytes;
     };
     std::vector<Readback> readbacks;
+    // control transfers waiting to be launched together (kc::control_ops):
+    // uploads and fills before the next kernel (flush_ctl), readbacks at the
+    // next sync_stream
+    kc::CtlOps ctl{}, down{};
+    int n_ctl = 0, n_down = 0;
+    bool ctl_mbox = false;  // some pending upload reads the mailbox
+
+    // Checks of the last batch put off to the export's synchronisation
+    // (count_and_pack): readbacks of the count in flight
+    struct Unchecked {
+        bool pending = false;
+        uint64_t n_keys = 0, nlow = 0;
+        uint32_t ext_err = 0, cnt_err = 0;
+        bool windowed = false;
+    } chk;
 
     // stage profiling: CUDA event pairs recorded on `stream` around each stage
     bool profiling = false;
@@ -357,19 +378,55 @@ int setup_shape(kc_context* c) {
 // hold up the batch it belongs to.  So: fills run as a kernel, uploads are
 // staged in the mapped mailbox and copied in by a kernel, readbacks are
 // copied out to the mailbox by a kernel and land in their host destination
-// at the next sync_stream().  Sizes and addresses must be 4-byte multiples;
+// at the next sync_stream(); those that meet before a kernel needs them, or
+// before a synchronisation, share a launch.  Sizes and addresses must be 4-byte multiples;
 // anything else, or larger than the mailbox, takes cudaMemcpyAsync.
+int launch_ctl(kc_context* c, kc::CtlOps& ops, int& n) {
+    if (!n) return KC_OK;
+    uint64_t most = 1;
+    for (int i = 0; i < n; ++i) most = std::max<uint64_t>(most, ops.op[i].n);
+    const dim3 grid((uint32_t)std::min<uint64_t>(ceil_div(most, 256), 64), (uint32_t)n);
+    kc::control_ops<<<grid, 256, 0, c->stream>>>(ops);
+    n = 0;
+    CK(cudaGetLastError());
+    return KC_OK;
+}
+
+// Launch the pending uploads and fills; called before a kernel that needs one.
+int flush_ctl(kc_context* c) {
+    if (!c->n_ctl) return KC_OK;
+    const int rc = launch_ctl(c, c->ctl, c->n_ctl);
+    if (rc) return rc;
+    if (c->ctl_mbox) CK(cudaEventRecord(c->ev_mbox, c->stream));
+    c->ctl_mbox = false;
+    return KC_OK;
+}
+
+int queue_ctl(kc_context* c, void* dst, const void* src, uint64_t words, uint32_t word) {
+    if (c->n_ctl == kc::CTL_OPS) {
+        const int rc = flush_ctl(c);
+        if (rc) return rc;
+    }
+    c->ctl.op[c->n_ctl++] = kc::CtlOp{static_cast<uint32_t*>(dst), static_cast<const uint32_t*>(src), words, word};
+    return KC_OK;
+}
+
+// fill_dev and put take effect at the next flush_ctl (the ops of one flush are
+// unordered: their destinations differ).
 int fill_dev(kc_context* c, void* dst, uint64_t bytes, uint32_t word) {
     if (!bytes) return KC_OK;
     if (bytes % 4 || reinterpret_cast<uintptr_t>(dst) % 4) {
         CK(cudaMemsetAsync(dst, (int)(word & 0xFF), bytes, c->stream));
         return KC_OK;
     }
-    const uint64_t n = bytes / 4;
-    kc::fill_words<<<std::min<uint64_t>(ceil_div(n, 256), (uint64_t)c->sm_count * 16), 256, 0, c->stream>>>(
-        static_cast<uint32_t*>(dst), n, word);
-    CK(cudaGetLastError());
-    return KC_OK;
+    if (bytes > (1u << 20)) {  // a large fill spreads over the device
+        const uint64_t n = bytes / 4;
+        kc::fill_words<<<std::min<uint64_t>(ceil_div(n, 256), (uint64_t)c->sm_count * 16), 256, 0, c->stream>>>(
+            static_cast<uint32_t*>(dst), n, word);
+        CK(cudaGetLastError());
+        return KC_OK;
+    }
+    return queue_ctl(c, dst, nullptr, bytes / 4, word);
 }
 
 int put(kc_context* c, void* dst, const void* src, uint64_t bytes) {
@@ -379,20 +436,21 @@ int put(kc_context* c, void* dst, const void* src, uint64_t bytes) {
         return KC_OK;
     }
     if (c->mbox_up_off + bytes > kc_context::MBOX_UP) {
-        // wrap: every earlier upload kernel has to have read its bytes
+        // wrap: every earlier upload has to have read its bytes
+        const int rc = flush_ctl(c);
+        if (rc) return rc;
         CK(cudaEventSynchronize(c->ev_mbox));
         c->mbox_up_off = 0;
     }
     std::memcpy(c->mbox_h + c->mbox_up_off, src, bytes);
-    const uint64_t n = bytes / 4;
-    kc::copy_words<<<std::min<uint64_t>(ceil_div(n, 256), 64), 256, 0, c->stream>>>(
-        reinterpret_cast<const uint32_t*>(c->mbox_d + c->mbox_up_off), static_cast<uint32_t*>(dst), n);
-    CK(cudaGetLastError());
-    CK(cudaEventRecord(c->ev_mbox, c->stream));
+    const int rc = queue_ctl(c, dst, c->mbox_d + c->mbox_up_off, bytes / 4, 0);
+    if (rc) return rc;
+    c->ctl_mbox = true;
     c->mbox_up_off += (bytes + 15) & ~15ull;
     return KC_OK;
 }
 
+// The value the kernels launched before the next sync_stream leave in src.
 int get(kc_context* c, void* dst, const void* src, uint64_t bytes) {
     if (!bytes) return KC_OK;
     if (bytes % 4 || reinterpret_cast<uintptr_t>(src) % 4 || c->mbox_down_off + bytes > kc_context::MBOX_DOWN) {
@@ -400,10 +458,12 @@ int get(kc_context* c, void* dst, const void* src, uint64_t bytes) {
         return KC_OK;
     }
     const uint64_t off = kc_context::MBOX_UP + c->mbox_down_off;
-    const uint64_t n = bytes / 4;
-    kc::copy_words<<<std::min<uint64_t>(ceil_div(n, 256), 64), 256, 0, c->stream>>>(
-        static_cast<const uint32_t*>(src), reinterpret_cast<uint32_t*>(c->mbox_d + off), n);
-    CK(cudaGetLastError());
+    if (c->n_down == kc::CTL_OPS) {
+        const int rc = launch_ctl(c, c->down, c->n_down);
+        if (rc) return rc;
+    }
+    c->down.op[c->n_down++] = kc::CtlOp{reinterpret_cast<uint32_t*>(c->mbox_d + off),
+                                        static_cast<const uint32_t*>(src), bytes / 4, 0};
     c->readbacks.push_back({dst, off, bytes});
     c->mbox_down_off += (bytes + 15) & ~15ull;
     return KC_OK;
@@ -411,6 +471,8 @@ int get(kc_context* c, void* dst, const void* src, uint64_t bytes) {
 
 // Wait for `stream`, then deliver the pending readbacks.
 int sync_stream(kc_context* c) {
+    int rc = flush_ctl(c);
+    if (rc || (rc = launch_ctl(c, c->down, c->n_down))) return rc;
     CK(cudaStreamSynchronize(c->stream));
     for (const auto& r : c->readbacks) std::memcpy(r.dst, c->mbox_h + r.off, r.bytes);
     c->readbacks.clear();
@@ -429,14 +491,20 @@ int sync_stream(kc_context* c) {
 // device total in scalars[slot].
 template <class TI, class TO>
 int device_scan(kc_context* c, const TI* in, uint64_t n, TO* out, uint64_t base, uint64_t* d_total) {
-    const uint64_t nb = std::max<uint64_t>(1, ceil_div(n, kc::SCAN_TILE));
+    CKR(flush_ctl(c));
+    if (n <= kc::SCAN_ONE) {
+        Stage st(c, KC_STAGE_SCAN);
+        kc::scan_one<TI, TO><<<1, kc::SCAN_BLOCK, 0, c->stream>>>(in, n, base, out, d_total);
+        CK(cudaGetLastError());
+        return KC_OK;
+    }
+    const uint64_t nb = ceil_div(n, kc::SCAN_TILE);
     CK(c->scan_sums.ensure(nb * sizeof(uint64_t)));
-    Stage st(c, KC_STAGE_SCAN, n ? 3 : 1);
+    Stage st(c, KC_STAGE_SCAN, 3);
     uint64_t* sums = c->scan_sums.as<uint64_t>();
-    if (n) kc::scan_reduce<TI><<<nb, kc::SCAN_BLOCK, 0, c->stream>>>(in, n, sums);
-    else CKR(fill_dev(c, sums, sizeof(uint64_t), 0));
-    kc::scan_sums<<<1, kc::SCAN_BLOCK, 0, c->stream>>>(sums, n ? nb : 1, base, d_total);
-    if (n) kc::scan_apply<TI, TO><<<nb, kc::SCAN_BLOCK, 0, c->stream>>>(in, n, sums, out);
+    kc::scan_reduce<TI><<<nb, kc::SCAN_BLOCK, 0, c->stream>>>(in, n, sums);
+    kc::scan_sums<<<1, kc::SCAN_BLOCK, 0, c->stream>>>(sums, nb, base, d_total);
+    kc::scan_apply<TI, TO><<<nb, kc::SCAN_BLOCK, 0, c->stream>>>(in, n, sums, out);
     CK(cudaGetLastError());
     return KC_OK;
 }
@@ -559,12 +627,13 @@ int size_structures(kc_context* c, const std::vector<uint64_t>& kb, double scale
 }
 
 template <int NW>
-void launch_count(kc_context* c, uint64_t n_keys, int use_filter) {
+int launch_count(kc_context* c, uint64_t n_keys, int use_filter) {
     constexpr int TILE = kc::count_tile<NW>();
-    join_init(c);
+    CKR(join_init(c));
+    CKR(flush_ctl(c));
     // each CTA covers CNT_SEGS_PER_WARP segments per warp, in blockIdx order
     const uint64_t tiles = ceil_div(n_keys, (uint64_t)TILE * kc::CNT_SEGS_PER_WARP);
-    if (!tiles) return;
+    if (!tiles) return KC_OK;
     kc::CountArgs a{};
     a.routed = c->routed.p;
     a.n_keys = n_keys;
@@ -581,6 +650,8 @@ void launch_count(kc_context* c, uint64_t n_keys, int use_filter) {
     a.filter_in_table = c->nw == 1;
     Stage st(c, use_filter ? KC_STAGE_COUNT_ROUTED : KC_STAGE_REHASH);
     kc::count_routed<NW><<<tiles, kc::CNT_THREADS, 0, c->stream>>>(a);
+    CK(cudaGetLastError());
+    return KC_OK;
 }
 
 // Grow the tables of the given buckets x4 (again x4 for a bucket whose keys
@@ -617,6 +688,7 @@ int grow_buckets(kc_context* c, const std::vector<uint32_t>& buckets) {
         CK(cudaMemcpyAsync(c->grow_jobs.p, jobs.data(), jobs.size() * sizeof(kc::GrowJob), cudaMemcpyHostToDevice,
                            c->stream));
         CKR(fill_dev(c, c->grow_failed.p, jobs.size() * sizeof(uint32_t), 0));
+        CKR(flush_ctl(c));
         std::vector<uint32_t> failed(jobs.size());
         for (size_t j0 = 0; j0 < jobs.size(); j0 += 65535) {  // grid y limit
             const uint32_t nj = (uint32_t)std::min<size_t>(65535, jobs.size() - j0);
@@ -650,12 +722,15 @@ int grow_buckets(kc_context* c, const std::vector<uint32_t>& buckets) {
 
 // Grow the tables of overflowed buckets (x4) and re-insert the keys that
 // met a full table, until none is left.
+// (h_overflow holds the flags of the count that went before.)
 template <int NW>
 int rehash_loop(kc_context* c, uint64_t n_keys) {
     const uint32_t nb = c->n_buckets;
     for (int round = 0;; ++round) {
-        CKR(get(c, c->h_overflow.data(), c->overflow.p, nb * sizeof(uint32_t)));
-        CKR(sync_stream(c));
+        if (round) {
+            CKR(get(c, c->h_overflow.data(), c->overflow.p, nb * sizeof(uint32_t)));
+            CKR(sync_stream(c));
+        }
         std::vector<uint32_t> grow;
         for (uint32_t b = 0; b < nb; ++b)
             if (c->h_overflow[b]) grow.push_back(b);
@@ -665,8 +740,7 @@ int rehash_loop(kc_context* c, uint64_t n_keys) {
         CKR(grow_buckets<NW>(c, grow));
         CKR(put(c, c->meta.p, c->h_meta.data(), nb * sizeof(kc::BucketMeta)));
         c->win_ready = false;  // grown buckets leave the windowed count (their filter and table part)
-        launch_count<NW>(c, n_keys, 0);
-        CK(cudaGetLastError());
+        CKR(launch_count<NW>(c, n_keys, 0));
     }
 }
 
@@ -703,12 +777,13 @@ bool build_windows(kc_context* c, uint32_t nb) {
 // Count the keys [off, off + n) of `routed` (off a multiple of the count
 // segment) with count_routed: the spill area of the windowed count.
 template <int NW>
-void launch_count_range(kc_context* c, uint64_t off, uint64_t n, int use_filter) {
+int launch_count_range(kc_context* c, uint64_t off, uint64_t n, int use_filter) {
     constexpr int TILE = kc::count_tile<NW>();
     constexpr int SEG = kc::count_seg<NW>();
-    join_init(c);
+    CKR(join_init(c));
+    CKR(flush_ctl(c));
     const uint64_t tiles = ceil_div(n, (uint64_t)TILE * kc::CNT_SEGS_PER_WARP);
-    if (!tiles) return;
+    if (!tiles) return KC_OK;
     kc::CountArgs a{};
     a.routed = c->routed.as<uint8_t>() + off * (uint64_t)(8 * NW);
     a.n_keys = n;
@@ -725,6 +800,8 @@ void launch_count_range(kc_context* c, uint64_t off, uint64_t n, int use_filter)
     a.filter_in_table = c->nw == 1;
     Stage st(c, KC_STAGE_COUNT_ROUTED);
     kc::count_routed<NW><<<tiles, kc::CNT_THREADS, 0, c->stream>>>(a);
+    CK(cudaGetLastError());
+    return KC_OK;
 }
 
 // Windowed count of one batch of 64-bit keys in `routed` (kc_window.cuh):
@@ -766,6 +843,7 @@ int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets 
     uint64_t total = 0, spill_start = 0, spill_used = 0;
     for (;;) {
         CKR(fill_dev(c, c->win_count.p, nw * sizeof(uint32_t), 0));
+        CKR(flush_ctl(c));
         {
             Stage st(c, KC_STAGE_SUBROUTE, 2);
             const uint64_t g = ceil_div(cchunks, stride);
@@ -791,6 +869,7 @@ int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets 
         CK(c->tile_low_prefix.ensure(std::max<uint64_t>(arr / kc::WIN_SEG, 1) * sizeof(uint64_t)));
         CKR(put(c, d_scal + 5, &spill_start, sizeof(uint64_t)));
         CKR(fill_dev(c, d_spill_full, sizeof(uint32_t), 0));
+        CKR(flush_ctl(c));
         {
             Stage st(c, KC_STAGE_SUBROUTE, n_keys ? 2 : 1);
             kc::window_bounds<<<small_grid, 256, 0, c->stream>>>(c->win_start.as<uint64_t>(), c->win_padded.as<uint32_t>(),
@@ -845,6 +924,7 @@ int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets 
     a.bucket_overflow = c->overflow.as<uint32_t>();
     a.fresh = c->init_deferred;
     c->init_deferred = false;
+    CKR(flush_ctl(c));
     {
         Stage st(c, KC_STAGE_COUNT_ROUTED, 2);
         for (uint32_t ph = 0; ph < 2; ++ph) {
@@ -855,7 +935,7 @@ int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets 
         }
         CK(cudaGetLastError());
     }
-    if (spill_used) launch_count_range<1>(c, spill_start, spill_used, 1);
+    if (spill_used) CKR(launch_count_range<1>(c, spill_start, spill_used, 1));
     c->window_spill += spill_used;
     CK(cudaGetLastError());
     return KC_OK;
@@ -891,6 +971,7 @@ int launch_extract(kc_context* c, const uint8_t* buf, uint64_t n, int has_halo, 
         a.overflow_start = overflow_start;
         a.overflow_end = overflow_end;
     }
+    CKR(flush_ctl(c));
     Stage st(c, mode == kc::HIST ? KC_STAGE_EXTRACT_HIST : KC_STAGE_EXTRACT_SCATTER);
     if (mode == kc::HIST)
         kc::extract_kernel<NW, kc::HIST>
@@ -903,7 +984,7 @@ int launch_extract(kc_context* c, const uint8_t* buf, uint64_t n, int has_halo, 
 }
 
 template <int NW>
-int count_and_pack(kc_context* c, uint64_t n_keys, uint32_t ext_err);
+int count_and_pack(kc_context* c, uint64_t n_keys);
 
 // Count one batch of FASTQ bytes already in device memory.  route_only:
 // route it exactly (every tile's histogram, no estimated regions) into
@@ -921,6 +1002,11 @@ int process_batch(kc_context* c, const uint8_t* buf, uint64_t n, int has_halo, b
     CK(c->scalars.ensure(64));
     uint64_t* d_scal = c->scalars.as<uint64_t>();
     CKR(fill_dev(c, c->scalars.as<uint32_t>() + 12, 2 * sizeof(uint32_t), 0));  // extraction and count error words
+    CK(c->bucket_count.ensure(nb * sizeof(uint64_t)));
+    CK(c->bucket_cursor.ensure(nb * sizeof(uint64_t)));
+    CK(c->region_end.ensure(nb * sizeof(uint64_t)));
+    CK(c->region_fill.ensure(nb * sizeof(uint64_t)));
+    CKR(fill_dev(c, c->bucket_count.p, nb * sizeof(uint64_t), 0));
     if (tiles) {
         Stage st(c, KC_STAGE_LINES);
         kc::lines_per_tile<<<tiles, kc::EXT_THREADS, 0, c->stream>>>(buf, n, c->tile_nl.as<uint32_t>());
@@ -929,11 +1015,6 @@ int process_batch(kc_context* c, const uint8_t* buf, uint64_t n, int has_halo, b
     int rc = device_scan<uint32_t, uint64_t>(c, c->tile_nl.as<uint32_t>(), tiles, c->tile_line.as<uint64_t>(),
                                              c->line_base, d_scal + 0);
     if (rc) return rc;
-
-    CK(c->bucket_count.ensure(nb * sizeof(uint64_t)));
-    CK(c->bucket_cursor.ensure(nb * sizeof(uint64_t)));
-    CK(c->region_end.ensure(nb * sizeof(uint64_t)));
-    CK(c->region_fill.ensure(nb * sizeof(uint64_t)));
 
     // Bucket regions.  A large batch takes them from a histogram of every
     // EST_STRIDE-th tile: region = estimate x 1.02 + 4 standard deviations +
@@ -956,7 +1037,7 @@ int process_batch(kc_context* c, const uint8_t* buf, uint64_t n, int has_halo, b
     uint64_t n_keys = 0, kb = 0;
     for (int attempt = 0;; ++attempt) {
         const uint32_t stride = est ? kc::EST_STRIDE : 1u;
-        CKR(fill_dev(c, c->bucket_count.p, nb * sizeof(uint64_t), 0));
+        if (attempt) CKR(fill_dev(c, c->bucket_count.p, nb * sizeof(uint64_t), 0));
         if ((rc = launch_extract<NW>(c, buf, n, has_halo, kc::HIST, nb, stride))) return rc;
         c->h_bucket_count.resize(nb);
         uint64_t line_end = 0;
@@ -1007,6 +1088,7 @@ int process_batch(kc_context* c, const uint8_t* buf, uint64_t n, int has_halo, b
             CKR(fill_dev(c, c->region_fill.p, rb * sizeof(uint64_t), 0xFFFFFFFFu));
         }
         if (size_here) {
+            CKR(flush_ctl(c));
             CK(cudaEventRecord(c->ev_side_in, c->stream));
             c->side_in_ready = true;
         }
@@ -1047,22 +1129,48 @@ int process_batch(kc_context* c, const uint8_t* buf, uint64_t n, int has_halo, b
     }
     c->K += kb;
     if (c->after_scatter) CK(cudaEventRecord(c->after_scatter, c->stream));
-    uint32_t ext_err = 0;
-    CKR(get(c, &ext_err, c->scalars.as<uint32_t>() + 12, sizeof(uint32_t)));
     if (route_only) {
+        uint32_t ext_err = 0;
+        CKR(get(c, &ext_err, c->scalars.as<uint32_t>() + 12, sizeof(uint32_t)));
         CKR(sync_stream(c));
         if (ext_err) return fail(KC_ERR_DEVICE, "internal error: routing bucket disagreed with its reservation");
         c->routed_keys = n_keys;
         return KC_OK;
     }
-    return count_and_pack<NW>(c, n_keys, ext_err);
+    return count_and_pack<NW>(c, n_keys);
 }
 
-// Filter, tables and low.bin packing of the n_keys keys in `routed`
-// (EMPTY keys are skipped); ext_err is the extraction's error word, read back
-// with the count's.
+// After the count's readbacks (chk, h_overflow) have arrived: errors, growth
+// of overflowed tables; `grew` tells whether any table has moved.
 template <int NW>
-int count_and_pack(kc_context* c, uint64_t n_keys, uint32_t ext_err) {
+int finish_checks(kc_context* c, bool* grew) {
+    kc_context::Unchecked& k = c->chk;
+    k.pending = false;
+    const uint64_t before = c->rehashes;
+    CKR(rehash_loop<NW>(c, k.n_keys));
+    *grew = c->rehashes != before;
+    if (*grew) {  // the retry may have set the count's error word
+        CKR(get(c, &k.cnt_err, c->scalars.as<uint32_t>() + 13, sizeof(uint32_t)));
+        CKR(sync_stream(c));
+    }
+    if (k.ext_err) return fail(KC_ERR_DEVICE, "internal error: routing bucket disagreed with its reservation");
+    if (k.cnt_err) return fail(KC_ERR_DEVICE, "internal error: a 256-bit table slot was never published");
+    c->win_result = k.windowed && c->win_ready && c->batches == 1;
+    c->low_total += k.nlow;
+    c->last_batch_low = k.nlow;
+    return KC_OK;
+}
+
+// The batch being counted is the run's last.
+bool last_batch(const kc_context* c) { return c->input_bytes >= c->expected_total_bytes; }
+
+// Filter, tables and low.bin packing of the n_keys keys in `routed`
+// (EMPTY keys are skipped); the extraction's error word is read back with the
+// count's.  The last batch of a small input is packed into a buffer for all
+// its keys and its checks wait for the export's synchronisation
+// (finish_checks), so that packing and export follow without one.
+template <int NW>
+int count_and_pack(kc_context* c, uint64_t n_keys) {
     constexpr int SEG = kc::count_seg<NW>();
     uint64_t* d_scal = c->scalars.as<uint64_t>();
     int rc;
@@ -1077,25 +1185,40 @@ int count_and_pack(kc_context* c, uint64_t n_keys, uint32_t ext_err) {
     }
     if (!windowed) {
         CKR(init_now(c));
-        launch_count<NW>(c, n_keys, 1);
+        CKR(launch_count<NW>(c, n_keys, 1));
     }
     const uint64_t nsegs = ceil_div(n_keys, SEG);
-    CK(cudaGetLastError());
-    if ((rc = rehash_loop<NW>(c, n_keys))) return rc;
-    c->win_result = windowed && c->win_ready && c->batches == 1;
     c->win_result_segs = nsegs;
 
-    // first occurrences -> packed low.bin bytes
+    // first occurrences -> packed low.bin bytes (a growth and its retry do
+    // not change them)
     if ((rc = device_scan<uint32_t, uint64_t>(c, c->tile_low.as<uint32_t>(), nsegs,
                                               c->tile_low_prefix.as<uint64_t>(), 0, d_scal + 1)))
         return rc;
-    uint64_t nlow = 0;
-    uint32_t cnt_err = 0;
-    CKR(get(c, &nlow, d_scal + 1, sizeof(uint64_t)));
-    CKR(get(c, &cnt_err, c->scalars.as<uint32_t>() + 13, sizeof(uint32_t)));
+    kc_context::Unchecked& chk = c->chk;
+    chk = kc_context::Unchecked{true, n_keys, 0, 0, 0, windowed};
+    CKR(get(c, c->h_overflow.data(), c->overflow.p, c->n_buckets * sizeof(uint32_t)));
+    CKR(get(c, &chk.nlow, d_scal + 1, sizeof(uint64_t)));
+    CKR(get(c, &chk.ext_err, c->scalars.as<uint32_t>() + 12, sizeof(uint32_t)));
+    CKR(get(c, &chk.cnt_err, c->scalars.as<uint32_t>() + 13, sizeof(uint32_t)));
+    auto pack = [&](uint8_t* dst, uint64_t base) -> int {
+        Stage st(c, KC_STAGE_PACK_LOW);
+        auto kernel = c->packed_bytes % 8 ? kc::pack_low<NW, false> : kc::pack_low<NW, true>;
+        kernel<<<resident_grid(c, kernel, 256, ceil_div(nsegs, 256)), 256, 0, c->stream>>>(
+            c->routed.p, c->tile_low.as<uint32_t>(), c->tile_low_prefix.as<uint64_t>(), nsegs, c->cfg.k, dst, base);
+        CK(cudaGetLastError());
+        return KC_OK;
+    };
+    if (!c->stream_low && last_batch(c) && n_keys * c->packed_bytes <= SMALL_BYTES &&
+        c->table_slots_used * c->slot_bytes <= SMALL_BYTES) {
+        CK(c->low_packed.grow_keep((c->low_total + n_keys) * c->packed_bytes + 64, c->low_total * c->packed_bytes,
+                                   c->stream));
+        return pack(c->low_packed.as<uint8_t>(), c->low_total);
+    }
     CKR(sync_stream(c));
-    if (ext_err) return fail(KC_ERR_DEVICE, "internal error: routing bucket disagreed with its reservation");
-    if (cnt_err) return fail(KC_ERR_DEVICE, "internal error: a 256-bit table slot was never published");
+    const uint64_t nlow = chk.nlow, low_before = c->low_total;
+    bool grew;
+    CKR(finish_checks<NW>(c, &grew));
     uint8_t* low_dst;
     uint64_t low_base;
     if (c->stream_low) {
@@ -1113,25 +1236,15 @@ int count_and_pack(kc_context* c, uint64_t n_keys, uint32_t ext_err) {
         // first occurrences accumulate over the batches; size the buffer for
         // the whole input from the share seen so far (+10%), so that it is
         // reallocated (old and new both live during the copy) about once
-        uint64_t need = (c->low_total + nlow) * c->packed_bytes + 64;
+        uint64_t need = (low_before + nlow) * c->packed_bytes + 64;
         if (need > c->low_packed.cap && c->expected_total_bytes > c->input_bytes && c->input_bytes > 0)
             need = std::max<uint64_t>(need, (uint64_t)((double)need * 1.1 * (double)c->expected_total_bytes /
                                                        (double)c->input_bytes));
-        CK(c->low_packed.grow_keep(need, c->low_total * c->packed_bytes, c->stream));
+        CK(c->low_packed.grow_keep(need, low_before * c->packed_bytes, c->stream));
         low_dst = c->low_packed.as<uint8_t>();
-        low_base = c->low_total;
+        low_base = low_before;
     }
-    {
-        Stage st(c, KC_STAGE_PACK_LOW);
-        auto pack = c->packed_bytes % 8 ? kc::pack_low<NW, false> : kc::pack_low<NW, true>;
-        pack<<<resident_grid(c, pack, 256, ceil_div(nsegs, 256)), 256, 0, c->stream>>>(
-            c->routed.p, c->tile_low.as<uint32_t>(), c->tile_low_prefix.as<uint64_t>(), nsegs, c->cfg.k, low_dst,
-            low_base);
-    }
-    CK(cudaGetLastError());
-    c->low_total += nlow;
-    c->last_batch_low = nlow;
-    return KC_OK;
+    return pack(low_dst, low_base);
 }
 
 // Export every table slot whose count passes min..max: per-chunk counts
@@ -1140,9 +1253,12 @@ int count_and_pack(kc_context* c, uint64_t n_keys, uint32_t ext_err) {
 // (export_write).  Chunks are listed group by group (root id, or set x root
 // id), so each group's records are contiguous; totals[g] receives group g's
 // record count and totals[n_groups] the occupied slots.
+// `grew`: with a small input's checks pending (count_and_pack), they are made
+// here, after the export's synchronisation; if a table had to grow, the
+// export is void and *grew is set.
 template <int NW>
 int run_export(kc_context* c, const std::vector<kc::ExportChunk>& ch, uint64_t n_groups,
-               std::vector<uint64_t>& totals) {
+               std::vector<uint64_t>& totals, bool* grew) {
     const uint64_t nch = ch.size();
     c->n_chunks = nch;
     CKR(join_init(c));
@@ -1152,6 +1268,7 @@ int run_export(kc_context* c, const std::vector<kc::ExportChunk>& ch, uint64_t n
     CK(c->root_count.ensure((n_groups + 1) * sizeof(uint64_t)));
     if (nch) CKR(put(c, c->chunks.p, ch.data(), nch * sizeof(kc::ExportChunk)));
     CKR(fill_dev(c, c->root_count.p, (n_groups + 1) * sizeof(uint64_t), 0));
+    CKR(flush_ctl(c));
     unsigned long long* rcd = c->root_count.as<unsigned long long>();
     const uint64_t grid = std::min<uint64_t>(std::max<uint64_t>(nch, 1), (uint64_t)c->sm_count * 8);
     // the counting pass leaves a bit per passing slot when every chunk is whole
@@ -1176,13 +1293,7 @@ int run_export(kc_context* c, const std::vector<kc::ExportChunk>& ch, uint64_t n
     if ((rc = device_scan<uint32_t, uint64_t>(c, c->chunk_pass.as<uint32_t>(), nch, c->chunk_off.as<uint64_t>(), 0,
                                               nullptr)))
         return rc;
-    totals.assign(n_groups + 1, 0);
-    CKR(get(c, totals.data(), rcd, (n_groups + 1) * sizeof(uint64_t)));
-    CKR(sync_stream(c));
-    uint64_t R = 0;
-    for (uint64_t g = 0; g < n_groups; ++g) R += totals[g];
-    CK(c->roots.ensure(std::max<uint64_t>(R, 1) * c->record_bytes));
-    if (nch && R) {
+    auto write = [&]() -> int {
         Stage st(c, KC_STAGE_EXPORT);
         if (bits)
             kc::export_write_bits<NW><<<resident_grid(c, kc::export_write_bits<NW>, kc::EXP_THREADS, nch),
@@ -1194,7 +1305,31 @@ int run_export(kc_context* c, const std::vector<kc::ExportChunk>& ch, uint64_t n
                 c->table.p, c->chunks.as<kc::ExportChunk>(), nch, c->cfg.min_count, c->cfg.max_count,
                 c->chunk_off.as<uint64_t>(), c->roots.as<uint8_t>());
         CK(cudaGetLastError());
+        return KC_OK;
+    };
+    totals.assign(n_groups + 1, 0);
+    CKR(get(c, totals.data(), rcd, (n_groups + 1) * sizeof(uint64_t)));
+    const bool ahead = c->chk.pending && nch;  // a small input: room for every slot, no wait for their number
+    if (ahead) {
+        CK(c->roots.ensure(c->table_slots_used * c->record_bytes));
+        CKR(write());
+        CKR(flush_ctl(c));
+        CKR(launch_ctl(c, c->down, c->n_down));
+        CK(cudaEventRecord(c->ev1, c->stream));
     }
+    CKR(sync_stream(c));
+    if (c->chk.pending) {
+        CKR(finish_checks<NW>(c, grew));
+        if (*grew) return KC_OK;
+    }
+    uint64_t R = 0;
+    for (uint64_t g = 0; g < n_groups; ++g) R += totals[g];
+    if (ahead) {
+        c->end_recorded = true;
+        return KC_OK;
+    }
+    CK(c->roots.ensure(std::max<uint64_t>(R, 1) * c->record_bytes));
+    if (nch && R) CKR(write());
     return KC_OK;
 }
 
@@ -1202,20 +1337,23 @@ template <int NW>
 int export_tables(kc_context* c) {
     const uint32_t nb = c->n_buckets;
     std::vector<kc::ExportChunk> ch;
-    const uint32_t CH = 16384;
-    for (uint32_t b = 0; b < nb; ++b) {
-        const uint64_t slots = c->h_meta[b].tab_mask + 1;
-        for (uint64_t s = 0; s < slots; s += CH) {
-            kc::ExportChunk e;
-            e.slot_begin = c->h_meta[b].tab_off + s;
-            e.n_slots = (uint32_t)std::min<uint64_t>(CH, slots - s);
-            e.root = b >> (c->bucket_bits - 8);
-            ch.push_back(e);
-        }
-    }
     std::vector<uint64_t> h;
-    int rc;
-    if ((rc = run_export<NW>(c, ch, 256, h))) return rc;
+    const uint32_t CH = 16384;
+    for (bool grew = true; grew;) {  // again when a pending check grew a table
+        grew = false;
+        ch.clear();
+        for (uint32_t b = 0; b < nb; ++b) {
+            const uint64_t slots = c->h_meta[b].tab_mask + 1;
+            for (uint64_t s = 0; s < slots; s += CH) {
+                kc::ExportChunk e;
+                e.slot_begin = c->h_meta[b].tab_off + s;
+                e.n_slots = (uint32_t)std::min<uint64_t>(CH, slots - s);
+                e.root = b >> (c->bucket_bits - 8);
+                ch.push_back(e);
+            }
+        }
+        CKR(run_export<NW>(c, ch, 256, h, &grew));
+    }
     uint64_t tot = 0;
     for (int r = 0; r < 256; ++r) {
         c->root_counts[r] = h[r];
@@ -1237,6 +1375,10 @@ int begin_run(kc_context* c, uint64_t total_bytes) {
     c->K = 0;
     c->readbacks.clear();  // a failed earlier call may have left some behind
     c->mbox_up_off = c->mbox_down_off = 0;
+    c->n_ctl = c->n_down = 0;
+    c->ctl_mbox = false;
+    c->chk = kc_context::Unchecked{};
+    c->end_recorded = false;
     c->rehashes = 0;
     c->overflow_keys = 0;
     c->reroutes = 0;
@@ -1286,8 +1428,12 @@ int finish_run(kc_context* c) {
         Stage st(c, KC_STAGE_SORT, 4 * ((2 * c->cfg.k + 7) / 8));
         rc = kc_sort_roots(c->roots.p, c->root_total, c->record_bytes, c->cfg.k, w, c->stream);
         if (rc) return fail(rc, "root record sort failed: %s", kc_sort_error());
+        c->end_recorded = false;
     }
-    CKR(sync_stream(c));
+    if (!c->end_recorded) {
+        CK(cudaEventRecord(c->ev1, c->stream));
+        CKR(sync_stream(c));
+    }
     c->have_result = true;
     return KC_OK;
 }
@@ -1455,7 +1601,7 @@ int count_keys(kc_context* c, const void* d_keys, uint64_t n_keys, const uint64_
     CK(cudaMemcpyAsync(c->routed.p, d_keys, n_keys * (uint64_t)(8 * NW), cudaMemcpyDefault, c->stream));
     c->K += n_keys;
     c->batches++;
-    return count_and_pack<NW>(c, n_keys, 0);
+    return count_and_pack<NW>(c, n_keys);
 }
 
 }  // namespace
@@ -1653,8 +1799,6 @@ int kc_count_device(kc_context* c, const uint8_t* d_fastq, uint64_t n, kc_stats*
         if ((rc = run_batch(c, d_fastq + off, len, off > 0))) return rc;
     }
     if ((rc = finish_run(c))) return rc;
-    CK(cudaEventRecord(c->ev1, c->stream));
-    CK(cudaEventSynchronize(c->ev1));
     collect_stage_times(c);
     float ms = 0;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
@@ -1842,8 +1986,6 @@ int kc_count_keys_device(kc_context* c, const void* d_keys, uint64_t n_keys, con
         if (rc) return rc;
     }
     if ((rc = finish_run(c))) return rc;
-    CK(cudaEventRecord(c->ev1, c->stream));
-    CK(cudaEventSynchronize(c->ev1));
     collect_stage_times(c);
     float ms = 0;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
@@ -1861,8 +2003,6 @@ int kc_count_host(kc_context* c, const uint8_t* fastq, uint64_t n, kc_stats* sta
     CK(cudaEventRecord(c->ev0, c->stream));
     if ((rc = host_pipeline(c, fastq, n))) return rc;
     if ((rc = finish_run(c))) return rc;
-    CK(cudaEventRecord(c->ev1, c->stream));
-    CK(cudaEventSynchronize(c->ev1));
     collect_stage_times(c);
     float ms = 0;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
@@ -2078,6 +2218,7 @@ int kc_histogram(kc_context* c, uint32_t min_freq, uint32_t max_freq, uint64_t* 
     CK(gh.ensure(hist_bytes));
     unsigned long long* d = gh.as<unsigned long long>();
     CKR(fill_dev(c, d, hist_bytes, 0));
+    CKR(flush_ctl(c));
     CKR(c->nw == 1 ? histogram_kernels<1>(c, min_freq, max_freq, d, bins)
                    : (c->nw == 2 ? histogram_kernels<2>(c, min_freq, max_freq, d, bins)
                                  : histogram_kernels<4>(c, min_freq, max_freq, d, bins)));
@@ -2208,6 +2349,7 @@ int prefix_counts_impl(kc_context* c, const uint8_t* host, uint64_t n, uint64_t*
     if (tiles) {
         kc::lines_per_tile<<<tiles, kc::EXT_THREADS, 0, c->stream>>>(buf, n, c->tile_nl.as<uint32_t>());
         CK(cudaGetLastError());
+        CKR(flush_ctl(c));
         int rc = device_scan<uint32_t, uint64_t>(c, c->tile_nl.as<uint32_t>(), tiles, c->tile_line.as<uint64_t>(), 0,
                                                  c->scalars.as<uint64_t>());
         if (rc) return rc;
@@ -2225,6 +2367,8 @@ int kc_internal_prefix_counts(kc_context* c, const uint8_t* host, uint64_t n, ui
     CK(cudaSetDevice(c->device));
     c->readbacks.clear();
     c->mbox_up_off = c->mbox_down_off = 0;
+    c->n_ctl = c->n_down = 0;
+    c->ctl_mbox = false;
     return c->nw == 1 ? prefix_counts_impl<1>(c, host, n, counts)
                       : (c->nw == 2 ? prefix_counts_impl<2>(c, host, n, counts) : prefix_counts_impl<4>(c, host, n, counts));
 }
@@ -2655,7 +2799,8 @@ route_again:
             ch.push_back(kc::ExportChunk{c->h_meta[b].tab_off + q, (uint32_t)std::min<uint64_t>(CH, slots - q), (uint32_t)b});
     }
     std::vector<uint64_t> rc_h;
-    if ((rc = run_export<NW>(c, ch, nbk, rc_h))) return rc;
+    bool grew = false;
+    if ((rc = run_export<NW>(c, ch, nbk, rc_h, &grew))) return rc;
     std::vector<uint64_t> rstart(nbk);
     uint64_t R = 0;
     for (uint64_t b = 0; b < nbk; ++b) {

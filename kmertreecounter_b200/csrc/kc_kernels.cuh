@@ -331,9 +331,23 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
 // copy engines are kept for the bulk FASTQ and output copies, behind which a
 // few-byte copy would otherwise wait.
 
-static __global__ void copy_words(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint64_t n) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        dst[i] = src[i];
+// Up to CTL_OPS of them, with nothing in between, are one launch (a launch
+// per few bytes was a third of the launches of a small count): op
+// blockIdx.y copies n words from src, or fills with `word` without one.
+constexpr int CTL_OPS = 8;
+struct CtlOp {
+    uint32_t* dst;
+    const uint32_t* src;
+    uint64_t n;
+    uint32_t word;
+};
+struct CtlOps {
+    CtlOp op[CTL_OPS];
+};
+static __global__ void control_ops(const __grid_constant__ CtlOps o) {
+    const CtlOp p = o.op[blockIdx.y];
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += (uint64_t)gridDim.x * blockDim.x)
+        p.dst[i] = p.src ? p.src[i] : p.word;
 }
 
 static __global__ void fill_words(uint32_t* __restrict__ dst, uint64_t n, uint32_t v) {

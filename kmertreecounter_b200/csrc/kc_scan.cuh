@@ -1,6 +1,8 @@
 // Device-wide exclusive scan used by the batch pipeline (line index per
 // tile, per-tile first-occurrence offsets).  Three launches: per-block
-// totals, one block scanning those totals, per-block rescan with its offset.
+// totals, one block scanning those totals, per-block rescan with its offset;
+// or one launch of one block up to SCAN_ONE values, where three launches take
+// longer than the block's few rounds of SCAN_TILE.
 #pragma once
 
 #include <cstdint>
@@ -89,6 +91,34 @@ __global__ void __launch_bounds__(SCAN_BLOCK) scan_apply(const TI* __restrict__ 
         if (b0 + i < n) out[b0 + i] = (TO)run;
         run += v[i];
     }
+}
+
+constexpr uint64_t SCAN_ONE = 4 * SCAN_TILE;
+
+// The whole scan in one block; n may be 0.
+template <class TI, class TO>
+__global__ void __launch_bounds__(SCAN_BLOCK) scan_one(const TI* __restrict__ in, uint64_t n, uint64_t base,
+                                                       TO* __restrict__ out, uint64_t* __restrict__ total_out) {
+    __shared__ uint64_t sw[32];
+    uint64_t carry = base;
+    for (uint64_t t = 0; t < n; t += SCAN_TILE) {
+        const uint64_t b0 = t + (uint64_t)threadIdx.x * SCAN_ITEMS;
+        uint64_t v[SCAN_ITEMS];
+        uint64_t s = 0, tot;
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS; ++i) {
+            v[i] = (b0 + i < n) ? (uint64_t)in[b0 + i] : 0;
+            s += v[i];
+        }
+        uint64_t run = carry + block_exclusive_scan_u64(s, sw, &tot);
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS; ++i) {
+            if (b0 + i < n) out[b0 + i] = (TO)run;
+            run += v[i];
+        }
+        carry += tot;
+    }
+    if (threadIdx.x == 0 && total_out) *total_out = carry;
 }
 
 }  // namespace kc
