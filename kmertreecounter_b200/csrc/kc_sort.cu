@@ -12,6 +12,16 @@
 // a tile of 256 threads x ITEMS records is processed in ITEMS rounds of 256
 // consecutive records; inside a round, __match_any_sync ranks equal digits
 // within a warp and per-warp digit counts in shared memory order the warps.
+//
+// n records are told apart by little more than log2(n) leading key bits, so
+// the passes go over the leading digits only (log2(n) + 8 bits, whole digits:
+// 4 of 8 passes for 12 M keys of k = 31, 4 of 16 for k = 63), and the few runs
+// of records that agree in all of those are sorted by the rest of the key
+// where they lie: short runs by a thread, runs up to WARP_RUN by a warp and up
+// to LONG_RUN by a block in shared memory.  Keys with longer runs (many
+// distinct keys behind one long common prefix) take the passes over all digits
+// after all.  11.7 M records of k = 31: 2.20 ms over all digits, 1.35 over four
+// and the runs (high-coverage repeats with errors make ~100,000 of them).
 
 #include <algorithm>
 #include <cstdint>
@@ -120,6 +130,143 @@ __global__ void __launch_bounds__(SORT_THREADS) downsweep(const Rec<W>* __restri
     }
 }
 
+constexpr uint32_t SHORT_RUN = 16;     // records a thread sorts in place
+constexpr uint32_t WARP_RUN = 128;     // records a warp sorts in shared memory
+constexpr uint32_t LONG_RUN = 1024;    // records a block sorts in shared memory
+constexpr uint64_t PREFIX_MIN = 1ull << 16;  // smaller sorts are a few launches either way
+
+template <int NW>
+__device__ __forceinline__ bool key_less(const uint64_t* a, const uint64_t* b) {
+#pragma unroll
+    for (int w = 0; w < NW; ++w)
+        if (a[w] != b[w]) return a[w] < b[w];
+    return false;
+}
+
+// Runs of records that agree in the leading `bits` key bits (at most 64),
+// found by their first record; runs longer than SHORT_RUN go to the list,
+// which has room for them all (n / 8 entries).
+struct RunList {
+    unsigned long long* warp;   // runs longer than SHORT_RUN, by first record
+    unsigned long long* block;  // of these, runs longer than WARP_RUN
+    unsigned long long* count;  // [0], [1]: entries of the lists; [2]: set when a run is longer than LONG_RUN
+};
+
+template <int NW, int W>
+__global__ void __launch_bounds__(SORT_THREADS) sort_runs(Rec<W>* __restrict__ r, uint64_t n, uint32_t bits, RunList list) {
+    const uint32_t drop = 64 - bits;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i + 1 < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t top = r[i].w[0] >> drop;
+        if (r[i + 1].w[0] >> drop != top || (i && r[i - 1].w[0] >> drop == top)) continue;
+        uint32_t len = 2;
+        while (len <= SHORT_RUN && i + len < n && r[i + len].w[0] >> drop == top) ++len;
+        if (len > SHORT_RUN) {
+            list.warp[atomicAdd(list.count, 1ull)] = i;
+            continue;
+        }
+        for (uint32_t a = 1; a < len; ++a) {  // insertion sort
+            const Rec<W> x = r[i + a];
+            uint32_t b = a;
+            for (; b > 0; --b) {
+                const Rec<W> y = r[i + b - 1];
+                if (!key_less<NW>(x.w, y.w)) break;
+                r[i + b] = y;
+            }
+            if (b != a) r[i + b] = x;
+        }
+    }
+}
+
+// Bitonic sort of s[0..size) (a power of two) by the threads t, t + step, ...;
+// `sync` orders the steps.
+template <int NW, int W, class Sync>
+__device__ __forceinline__ void bitonic(Rec<W>* s, uint32_t size, uint32_t first, uint32_t step, Sync sync) {
+    for (uint32_t k = 2; k <= size; k *= 2)
+        for (uint32_t j = k / 2; j > 0; j /= 2) {
+            for (uint32_t t = first; t < size; t += step) {
+                const uint32_t o = t ^ j;
+                if (o > t && key_less<NW>(s[(t & k) ? t : o].w, s[(t & k) ? o : t].w)) {
+                    const Rec<W> x = s[t];
+                    s[t] = s[o];
+                    s[o] = x;
+                }
+            }
+            sync();
+        }
+}
+
+// A warp per listed run: its length, then a bitonic sort; longer runs to the
+// block list.
+template <int NW, int W>
+__global__ void __launch_bounds__(128) sort_warp_runs(Rec<W>* __restrict__ r, uint64_t n, uint32_t bits, RunList list) {
+    __shared__ Rec<W> smem[4][WARP_RUN];
+    const uint32_t drop = 64 - bits, lane = threadIdx.x & 31;
+    Rec<W>* s = smem[threadIdx.x >> 5];
+    const uint64_t runs = list.count[0];
+    for (uint64_t q = (uint64_t)blockIdx.x * 4 + (threadIdx.x >> 5); q < runs; q += (uint64_t)gridDim.x * 4) {
+        const uint64_t i = list.warp[q];
+        const uint64_t top = r[i].w[0] >> drop;
+        uint32_t len = 0;
+        for (uint32_t j = 0; j <= WARP_RUN; j += 32) {
+            const bool in = i + j + lane < n && r[i + j + lane].w[0] >> drop == top;
+            const uint32_t m = __ballot_sync(0xffffffffu, in);
+            len += m == 0xffffffffu ? 32 : __ffs(~m) - 1;
+            if (m != 0xffffffffu) break;
+        }
+        if (len > WARP_RUN) {
+            if (lane == 0) list.block[atomicAdd(list.count + 1, 1ull)] = i;
+            continue;
+        }
+        uint32_t size = 32;
+        while (size < len) size *= 2;
+        for (uint32_t j = lane; j < size; j += 32) {
+            if (j < len) s[j] = r[i + j];
+            else
+                for (int w = 0; w < W; ++w) s[j].w[w] = ~0ull;  // after every key
+        }
+        __syncwarp();
+        bitonic<NW, W>(s, size, lane, 32, [] { __syncwarp(); });
+        for (uint32_t j = lane; j < len; j += 32) r[i + j] = s[j];
+        __syncwarp();
+    }
+}
+
+// A block per run of the block list.
+template <int NW, int W>
+__global__ void __launch_bounds__(SORT_THREADS) sort_long_runs(Rec<W>* __restrict__ r, uint64_t n, uint32_t bits,
+                                                               RunList list) {
+    __shared__ Rec<W> s[LONG_RUN];
+    __shared__ uint32_t s_len;
+    const uint32_t drop = 64 - bits;
+    const uint64_t runs = list.count[1];
+    for (uint64_t q = blockIdx.x; q < runs; q += gridDim.x) {
+        const uint64_t i = list.block[q];
+        const uint64_t top = r[i].w[0] >> drop;
+        if (threadIdx.x == 0) s_len = LONG_RUN + 1;
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j <= LONG_RUN; j += SORT_THREADS)
+            if (i + j >= n || r[i + j].w[0] >> drop != top) atomicMin(&s_len, j);
+        __syncthreads();
+        const uint32_t len = s_len;
+        __syncthreads();
+        if (len > LONG_RUN) {  // block-uniform
+            if (threadIdx.x == 0) list.count[2] = 1;
+            continue;
+        }
+        uint32_t size = 32;
+        while (size < len) size *= 2;
+        for (uint32_t j = threadIdx.x; j < size; j += SORT_THREADS) {
+            if (j < len) s[j] = r[i + j];
+            else
+                for (int w = 0; w < W; ++w) s[j].w[w] = ~0ull;  // after every key
+        }
+        __syncthreads();
+        bitonic<NW, W>(s, size, threadIdx.x, SORT_THREADS, [] { __syncthreads(); });
+        for (uint32_t j = threadIdx.x; j < len; j += SORT_THREADS) r[i + j] = s[j];
+        __syncthreads();
+    }
+}
+
 template <int NW, int W>
 int sort_impl(void* records, uint64_t n, uint32_t k, const KcSortScratch& w, cudaStream_t st) {
     using R = Rec<W>;
@@ -129,23 +276,50 @@ int sort_impl(void* records, uint64_t n, uint32_t k, const KcSortScratch& w, cud
     const uint64_t n_tiles = (n + SORT_TILE - 1) / SORT_TILE;
     const uint64_t hn = (uint64_t)RADIX * n_tiles;
     R* a = static_cast<R*>(records);
-    R* src = a;
-    R* dst = static_cast<R*>(w.tmp);
+    R* tmp = static_cast<R*>(w.tmp);
     uint32_t* hist = static_cast<uint32_t*>(w.hist);
     uint64_t* offs = static_cast<uint64_t*>(w.offs);
     uint64_t* sums = static_cast<uint64_t*>(w.sums);
-    for (uint32_t p = 0; p < passes; ++p) {
-        const uint32_t bit = lowbit + 8 * p;
-        upsweep<NW, W><<<n_tiles, SORT_THREADS, 0, st>>>(src, n, bit, hist, n_tiles);
-        const uint64_t nb = (hn + kc::SCAN_TILE - 1) / kc::SCAN_TILE;
-        kc::scan_reduce<uint32_t><<<nb, kc::SCAN_BLOCK, 0, st>>>(hist, hn, sums);
-        kc::scan_sums<<<1, kc::SCAN_BLOCK, 0, st>>>(sums, nb, 0, nullptr);
-        kc::scan_apply<uint32_t, uint64_t><<<nb, kc::SCAN_BLOCK, 0, st>>>(hist, hn, sums, offs);
-        downsweep<NW, W><<<n_tiles, SORT_THREADS, 0, st>>>(src, dst, n, bit, offs, n_tiles);
-        std::swap(src, dst);
+    // `count` passes over the digits from bit `bit` on; the result is in `a`
+    auto run = [&](uint32_t bit, uint32_t count) {
+        R *src = a, *dst = tmp;
+        for (uint32_t p = 0; p < count; ++p, bit += 8) {
+            upsweep<NW, W><<<n_tiles, SORT_THREADS, 0, st>>>(src, n, bit, hist, n_tiles);
+            const uint64_t nb = (hn + kc::SCAN_TILE - 1) / kc::SCAN_TILE;
+            kc::scan_reduce<uint32_t><<<nb, kc::SCAN_BLOCK, 0, st>>>(hist, hn, sums);
+            kc::scan_sums<<<1, kc::SCAN_BLOCK, 0, st>>>(sums, nb, 0, nullptr);
+            kc::scan_apply<uint32_t, uint64_t><<<nb, kc::SCAN_BLOCK, 0, st>>>(hist, hn, sums, offs);
+            downsweep<NW, W><<<n_tiles, SORT_THREADS, 0, st>>>(src, dst, n, bit, offs, n_tiles);
+            std::swap(src, dst);
+        }
+        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess && src != a) e = cudaMemcpyAsync(a, src, n * sizeof(R), cudaMemcpyDeviceToDevice, st);
+        return e;
+    };
+    uint32_t need = 8;
+    while (need < 64 && (n >> (need - 8)) != 0) ++need;  // log2(n) + 8 bits
+    const uint32_t lead = (need + 7) / 8;
+    cudaError_t e;
+    if (n >= PREFIX_MIN && lead <= 8 && lead < passes) {
+        // the lists take the place of the offsets (256 n_tiles words: at most
+        // n / 17 runs after the counters) and of the digit counts (128 n_tiles
+        // words: n / 129)
+        unsigned long long* base = reinterpret_cast<unsigned long long*>(offs);
+        const RunList list{base + 8, reinterpret_cast<unsigned long long*>(hist), base};
+        e = run(64 * NW - 8 * lead, lead);
+        if (e == cudaSuccess) e = cudaMemsetAsync(list.count, 0, 8 * sizeof(*base), st);
+        sort_runs<NW, W><<<(uint32_t)std::min<uint64_t>((n + SORT_THREADS - 1) / SORT_THREADS, 148 * 8), SORT_THREADS, 0,
+                           st>>>(a, n, 8 * lead, list);
+        sort_warp_runs<NW, W><<<148 * 8, 128, 0, st>>>(a, n, 8 * lead, list);
+        sort_long_runs<NW, W><<<148 * 2, SORT_THREADS, 0, st>>>(a, n, 8 * lead, list);
+        unsigned long long head[3] = {0, 0, 0};
+        if (e == cudaSuccess) e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaMemcpyAsync(head, list.count, sizeof head, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e == cudaSuccess && head[2]) e = run(lowbit, passes);
+    } else {
+        e = run(lowbit, passes);
     }
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess && src != a) e = cudaMemcpyAsync(a, src, n * sizeof(R), cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess) {
         g_sort_err = cudaGetErrorString(e);
         return KC_ERR_DEVICE;
