@@ -32,7 +32,14 @@ namespace {
 constexpr int GM = 64, GN = 64, GK = 32;  // CTA tile
 constexpr int G_THREADS = 128;            // 4 warps, 2x2 of 32x32
 
-enum Epi { EPI_STORE = 0, EPI_BIAS = 1, EPI_BIAS_RELU = 2 };
+enum Epi { EPI_STORE = 0, EPI_BIAS = 1, EPI_BIAS_RELU = 2, EPI_ADAM = 3 };
+
+// Adam state of a parameter array and the step's constants.
+struct AdamArgs {
+    float *w, *m, *v;
+    __nv_bfloat16* wb;  // BF16 copy (nullptr: none)
+    float lr, b1, b2, eps, c1, c2;
+};
 
 // C[m, n] = sum_k A[m, k] * B[k, n] (+ epilogue); element (i, j) of A at
 // A[i*sa0 + j*sa1], of B at B[i*sb0 + j*sb1]; C row-major with ldc; optional
@@ -46,7 +53,22 @@ struct GemmArgs {
     int M, N, K;
     long sa0, sa1, sb0, sb1, ldc;
     int epi;
+    AdamArgs adam;  // EPI_ADAM: C is the gradient of adam.w, which takes the step; C itself is not stored
 };
+
+// One parameter's step.  The roundings are spelled out: left to the compiler
+// they depend on the kernel around it, and a last bit of a moment decides the
+// direction of steps whose gradient is near zero.
+__device__ __forceinline__ void adam_step(const AdamArgs& a, long i, float gi) {
+    const float mi = __fmaf_rn(__fsub_rn(1.f, a.b1), gi, __fmul_rn(a.b1, a.m[i]));
+    const float vi = __fmaf_rn(__fmul_rn(__fsub_rn(1.f, a.b2), gi), gi, __fmul_rn(a.b2, a.v[i]));
+    a.m[i] = mi;
+    a.v[i] = vi;
+    const float step = __fdiv_rn(__fmul_rn(a.lr, __fdiv_rn(mi, a.c1)), __fadd_rn(__fsqrt_rn(__fdiv_rn(vi, a.c2)), a.eps));
+    const float w = __fsub_rn(a.w[i], step);
+    a.w[i] = w;
+    if (a.wb) a.wb[i] = __float2bfloat16(w);
+}
 
 __device__ __forceinline__ uint32_t pack_bf16(__nv_bfloat16 lo, __nv_bfloat16 hi) {
     return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
@@ -68,13 +90,15 @@ __global__ void __launch_bounds__(G_THREADS) gemm_bf16(GemmArgs g) {
             for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.f;
     const __nv_bfloat16 zero = __float2bfloat16(0.f);
     for (int k0 = 0; k0 < g.K; k0 += GK) {
+        // neighbouring threads load neighbouring elements, whichever index
+        // they differ in
         for (int e = tid; e < GM * GK; e += G_THREADS) {
-            const int m = e / GK, k = e % GK;
+            const int m = g.sa0 == 1 ? e % GM : e / GK, k = g.sa0 == 1 ? e / GM : e % GK;
             const long gm = m0 + m, gk = k0 + k;
             As[m][k] = (gm < g.M && gk < g.K) ? g.A[gm * g.sa0 + gk * g.sa1] : zero;
         }
         for (int e = tid; e < GN * GK; e += G_THREADS) {
-            const int n = e / GK, k = e % GK;
+            const int n = g.sb1 == 1 ? e % GN : e / GK, k = g.sb1 == 1 ? e / GN : e % GK;
             const long gn = n0 + n, gk = k0 + k;
             Bs[n][k] = (gn < g.N && gk < g.K) ? g.B[gk * g.sb0 + gn * g.sb1] : zero;
         }
@@ -120,6 +144,10 @@ __global__ void __launch_bounds__(G_THREADS) gemm_bf16(GemmArgs g) {
                 const int n = n0 + wn + j * 8 + tig * 2 + (r & 1);
                 if (m >= g.M || n >= g.N) continue;
                 float v = acc[i][j][r];
+                if (g.epi == EPI_ADAM) {
+                    adam_step(g.adam, (long)m * g.ldc + n, v);
+                    continue;
+                }
                 if (g.epi == EPI_BIAS || g.epi == EPI_BIAS_RELU) v += g.bias[n];
                 if (g.epi == EPI_BIAS_RELU) v = fmaxf(v, 0.f);
                 g.C[(long)m * g.ldc + n] = v;
@@ -133,17 +161,21 @@ __global__ void __launch_bounds__(G_THREADS) gemm_bf16(GemmArgs g) {
 // K = 512..8192: one 64 x 64 tile per CTA left 8 CTAs loading element by
 // element, 129..256 dependent steps each (0.2-0.4 ms a product).  Here a CTA
 // takes 16 columns and 64 rows; its warps are 16 x 8 tiles and the operands
-// arrive in 128-deep chunks, four in flight (cp.async, 16 bytes a copy).  The
+// arrive in 128-deep chunks, several in flight (cp.async, 16 bytes a copy).  The
 // k16 steps of a tile keep their order, so results are the same bits as the
 // 64 x 64 kernel's; splitting K would fill more SMs but round differently.
 // Bound by the chain of dependent MMAs (K / 16) of a tile.  A training step of
-// 32 rows with its copies: 1.66 -> 0.43 ms.
-constexpr int C_M = 64, C_N = 16, C_K = 128, C_STAGES = 4;
+// 32 rows with its copies: 1.66 -> 0.32 ms, and 0.27 with the fused steps
+// and the copies beside the backward pass.
+constexpr int C_M = 64, C_N = 16, C_K = 128;
 constexpr int C_PITCH = C_K + 8;    // [row][k] chunks: rows of 272 bytes
 constexpr int C_BPITCH = C_N + 8;   // [k][column] chunks of B: rows of 48 bytes
 constexpr int C_A = C_M * C_PITCH;  // elements
 constexpr int C_B = C_K * C_BPITCH > C_N * C_PITCH ? C_K * C_BPITCH : C_N * C_PITCH;
-constexpr size_t C_SMEM = (size_t)C_STAGES * (C_A + C_B) * sizeof(__nv_bfloat16);
+// Chunks in flight: 8 where the contraction is long (32 CTAs, one per SM, each
+// waiting for L2), 4 where there are many CTAs (two per SM).
+constexpr size_t chain_smem(int stages) { return (size_t)stages * (C_A + C_B) * sizeof(__nv_bfloat16); }
+constexpr int C_LONG = 2048;  // K from which 8 chunks pay
 
 __device__ __forceinline__ void copy16(void* smem, const void* gmem, bool valid) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
@@ -154,7 +186,7 @@ __device__ __forceinline__ void copy16(void* smem, const void* gmem, bool valid)
 // A: row-major, ldA; B: BT ? columns contiguous in k (element (k, n) at
 // B[n * ldb + k]) : rows contiguous in n (B[k * ldb + n]).  ldA, ldb, K (and
 // N without BT) are multiples of 8 and the arrays 16-byte aligned.
-template <bool BT>
+template <bool BT, int C_STAGES>
 __global__ void __launch_bounds__(256) gemm_chain(GemmArgs g, long lda, long ldb) {
     extern __shared__ __align__(16) uint8_t c_smem[];
     __nv_bfloat16* sa = reinterpret_cast<__nv_bfloat16*>(c_smem);
@@ -281,18 +313,13 @@ __global__ void col_sum(const float* d, float* g, int rows, int cols) {
     g[c] = s;
 }
 
-// Adam on FP32 master weights, then the BF16 copy.
-__global__ void adam(float* w, __nv_bfloat16* wb, const float* g, float* m, float* v, long n, float lr, float b1,
-                     float b2, float eps, float c1, float c2) {
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-        if (wb) wb[i] = __float2bfloat16(w[i]);
-    }
+// The bias's gradient and its Adam step.
+__global__ void col_sum_adam(const float* d, int rows, int cols, AdamArgs a) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= cols) return;
+    float s = 0.f;
+    for (int r = 0; r < rows; ++r) s += d[(long)r * cols + c];
+    adam_step(a, c, s);
 }
 
 thread_local std::string g_mlp_err;
@@ -305,7 +332,14 @@ struct kc_mlp {
     float *W[3] = {}, *b[3] = {}, *gW[3] = {}, *gb[3] = {}, *mW[3] = {}, *vW[3] = {}, *mb[3] = {}, *vb[3] = {};
     __nv_bfloat16* Wb[3] = {};
     long nW[3] = {}, nb[3] = {};
-    float *x = nullptr, *h1 = nullptr, *h2 = nullptr, *y = nullptr, *t = nullptr;
+    // a batch's inputs and targets arrive on `cs` in one of two buffers, while
+    // the step before is still in its backward pass on `st`
+    cudaStream_t cs = nullptr;
+    cudaEvent_t ev_in[2] = {}, ev_used[2] = {}, ev_loss = nullptr;
+    float *xs[2] = {}, *ts[2] = {};
+    int slot = 0;
+    float* h_loss = nullptr;  // page-locked
+    float *h1 = nullptr, *h2 = nullptr, *y = nullptr;
     __nv_bfloat16 *xb = nullptr, *h1b = nullptr, *h2b = nullptr;
     float *dy = nullptr, *dh2 = nullptr, *dh1 = nullptr;
     __nv_bfloat16 *dyb = nullptr, *dh2b = nullptr, *dh1b = nullptr;
@@ -330,18 +364,25 @@ cudaError_t dalloc(T** p, long n) {
     return cudaMalloc(reinterpret_cast<void**>(p), std::max<long>(n, 1) * sizeof(T));
 }
 
+template <bool BT>
+void launch_chain(const GemmArgs& g, long lda, long ldb, cudaStream_t st) {
+    const dim3 grid((g.N + C_N - 1) / C_N, (g.M + C_M - 1) / C_M);
+    const int warps = 2 * ((std::min(g.M, C_M) + 15) / 16);
+    if (g.K >= C_LONG) gemm_chain<BT, 8><<<grid, warps * 32, chain_smem(8), st>>>(g, lda, ldb);
+    else gemm_chain<BT, 4><<<grid, warps * 32, chain_smem(4), st>>>(g, lda, ldb);
+}
+
 void gemm(cudaStream_t st, const __nv_bfloat16* A, long sa0, long sa1, const __nv_bfloat16* B, long sb0, long sb1,
-          float* C, __nv_bfloat16* Cb, long ldc, const float* bias, int M, int N, int K, int epi) {
-    GemmArgs g{A, B, C, Cb, bias, M, N, K, sa0, sa1, sb0, sb1, ldc, epi};
+          float* C, __nv_bfloat16* Cb, long ldc, const float* bias, int M, int N, int K, int epi,
+          const AdamArgs& adam = {}) {
+    GemmArgs g{A, B, C, Cb, bias, M, N, K, sa0, sa1, sb0, sb1, ldc, epi, adam};
     // rows of A contiguous in k, 16-byte copies possible, and a contraction
     // long enough for the chunks (the weight gradients contract a batch)
     const bool bt = sb0 == 1;
-    if (sa1 == 1 && sa0 % 8 == 0 && K % 8 == 0 && K >= C_K &&
+    if (epi != EPI_ADAM && sa1 == 1 && sa0 % 8 == 0 && K % 8 == 0 && K >= C_K &&
         (bt ? sb1 % 8 == 0 : sb1 == 1 && sb0 % 8 == 0 && N % 8 == 0)) {
-        const dim3 grid((N + C_N - 1) / C_N, (M + C_M - 1) / C_M);
-        const int warps = 2 * ((std::min(M, C_M) + 15) / 16);
-        if (bt) gemm_chain<true><<<grid, warps * 32, C_SMEM, st>>>(g, sa0, sb1);
-        else gemm_chain<false><<<grid, warps * 32, C_SMEM, st>>>(g, sa0, sb0);
+        if (bt) launch_chain<true>(g, sa0, sb1, st);
+        else launch_chain<false>(g, sa0, sb0, st);
         return;
     }
     dim3 grid((N + GN - 1) / GN, (M + GM - 1) / GM);
@@ -357,28 +398,44 @@ int forward(kc_mlp* m, int B) {
     return KC_OK;
 }
 
-int backward(kc_mlp* m, int B, float* h_loss) {
+// Backward pass; the gradients to gW and gb, or, with `adam` (per layer:
+// weights, bias), the parameters' step instead.  A layer's weights take their
+// step after the product that reads them.  *h_loss is there when the loss is:
+// the rest of the pass may still run.
+int backward(kc_mlp* m, int B, float* h_loss, const AdamArgs (*adam)[2]) {
     const int I = m->in, H = m->hid, O = m->out;
     const long nout = (long)B * O;
     MK(cudaMemsetAsync(m->loss, 0, sizeof(float), m->st));
-    mse_grad<<<256, 256, 0, m->st>>>(m->y, m->t, m->dy, m->dyb, nout, 1.f / (float)nout, m->under, m->loss);
-    // layer 3: gW3 = h2^T dy, gb3 = colsum(dy), dh2 = dy W3^T
-    gemm(m->st, m->h2b, 1, H, m->dyb, O, 1, m->gW[2], nullptr, O, nullptr, H, O, B, EPI_STORE);
-    col_sum<<<(O + 255) / 256, 256, 0, m->st>>>(m->dy, m->gb[2], B, O);
+    mse_grad<<<256, 256, 0, m->st>>>(m->y, m->ts[m->slot], m->dy, m->dyb, nout, 1.f / (float)nout, m->under, m->loss);
+    MK(cudaEventRecord(m->ev_used[m->slot], m->st));
+    if (h_loss) {
+        MK(cudaMemcpyAsync(m->h_loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->st));
+        MK(cudaEventRecord(m->ev_loss, m->st));
+    }
+    // layer l: its input xin (B x n_in), the gradient d of its output
+    auto gradients = [&](int l, const __nv_bfloat16* xin, const __nv_bfloat16* db, const float* d, int n_in, int n_out) {
+        if (adam) {
+            gemm(m->st, xin, 1, n_in, db, n_out, 1, nullptr, nullptr, n_out, nullptr, n_in, n_out, B, EPI_ADAM, adam[l][0]);
+            col_sum_adam<<<(n_out + 255) / 256, 256, 0, m->st>>>(d, B, n_out, adam[l][1]);
+        } else {
+            gemm(m->st, xin, 1, n_in, db, n_out, 1, m->gW[l], nullptr, n_out, nullptr, n_in, n_out, B, EPI_STORE);
+            col_sum<<<(n_out + 255) / 256, 256, 0, m->st>>>(d, m->gb[l], B, n_out);
+        }
+    };
+    // dh2 = dy W3^T, then layer 3: gW3 = h2^T dy, gb3 = colsum(dy)
     gemm(m->st, m->dyb, O, 1, m->Wb[2], 1, O, m->dh2, nullptr, H, nullptr, B, H, O, EPI_STORE);
+    gradients(2, m->h2b, m->dyb, m->dy, H, O);
     relu_back<<<256, 256, 0, m->st>>>(m->dh2, m->h2, m->dh2b, (long)B * H);
     // layer 2
-    gemm(m->st, m->h1b, 1, H, m->dh2b, H, 1, m->gW[1], nullptr, H, nullptr, H, H, B, EPI_STORE);
-    col_sum<<<(H + 255) / 256, 256, 0, m->st>>>(m->dh2, m->gb[1], B, H);
     gemm(m->st, m->dh2b, H, 1, m->Wb[1], 1, H, m->dh1, nullptr, H, nullptr, B, H, H, EPI_STORE);
+    gradients(1, m->h1b, m->dh2b, m->dh2, H, H);
     relu_back<<<256, 256, 0, m->st>>>(m->dh1, m->h1, m->dh1b, (long)B * H);
     // layer 1
-    gemm(m->st, m->xb, 1, I, m->dh1b, H, 1, m->gW[0], nullptr, H, nullptr, I, H, B, EPI_STORE);
-    col_sum<<<(H + 255) / 256, 256, 0, m->st>>>(m->dh1, m->gb[0], B, H);
+    gradients(0, m->xb, m->dh1b, m->dh1, I, H);
     MK(cudaGetLastError());
     if (h_loss) {
-        MK(cudaMemcpyAsync(h_loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->st));
-        MK(cudaStreamSynchronize(m->st));
+        MK(cudaEventSynchronize(m->ev_loss));
+        *h_loss = *m->h_loss;
     }
     return KC_OK;
 }
@@ -388,10 +445,15 @@ int load_batch(kc_mlp* m, const float* x, const float* t, int B) {
         g_mlp_err = "batch size out of range";
         return KC_ERR_INVALID;
     }
-    MK(cudaMemcpyAsync(m->x, x, (size_t)B * m->in * sizeof(float), cudaMemcpyHostToDevice, m->st));
-    to_bf16<<<256, 256, 0, m->st>>>(m->x, m->xb, (long)B * m->in);
-    if (t) MK(cudaMemcpyAsync(m->t, t, (size_t)B * m->out * sizeof(float), cudaMemcpyHostToDevice, m->st));
+    const int s = m->slot ^= 1;
+    MK(cudaStreamWaitEvent(m->cs, m->ev_used[s], 0));
+    MK(cudaMemcpyAsync(m->xs[s], x, (size_t)B * m->in * sizeof(float), cudaMemcpyHostToDevice, m->cs));
+    if (t) MK(cudaMemcpyAsync(m->ts[s], t, (size_t)B * m->out * sizeof(float), cudaMemcpyHostToDevice, m->cs));
+    MK(cudaEventRecord(m->ev_in[s], m->cs));
+    MK(cudaStreamWaitEvent(m->st, m->ev_in[s], 0));
+    to_bf16<<<256, 256, 0, m->st>>>(m->xs[s], m->xb, (long)B * m->in);
     MK(cudaGetLastError());
+    MK(cudaEventRecord(m->ev_used[s], m->st));  // and again once the targets are read
     return KC_OK;
 }
 
@@ -403,15 +465,20 @@ const char* kc_mlp_last_error(void) { return g_mlp_err.c_str(); }
 
 void kc_mlp_destroy(kc_mlp* m) {
     if (!m) return;
+    if (m->cs) cudaStreamSynchronize(m->cs);
     if (m->st) cudaStreamSynchronize(m->st);
     for (int l = 0; l < 3; ++l)
         for (void* p : {(void*)m->W[l], (void*)m->Wb[l], (void*)m->gW[l], (void*)m->mW[l], (void*)m->vW[l],
                         (void*)m->b[l], (void*)m->gb[l], (void*)m->mb[l], (void*)m->vb[l]})
             if (p) cudaFree(p);
-    for (void* p : {(void*)m->x, (void*)m->xb, (void*)m->h1, (void*)m->h1b, (void*)m->h2, (void*)m->h2b, (void*)m->y,
-                    (void*)m->t, (void*)m->dy, (void*)m->dyb, (void*)m->dh2, (void*)m->dh2b, (void*)m->dh1,
+    for (void* p : {(void*)m->xs[0], (void*)m->xs[1], (void*)m->ts[0], (void*)m->ts[1], (void*)m->xb, (void*)m->h1, (void*)m->h1b, (void*)m->h2, (void*)m->h2b, (void*)m->y,
+                    (void*)m->dy, (void*)m->dyb, (void*)m->dh2, (void*)m->dh2b, (void*)m->dh1,
                     (void*)m->dh1b, (void*)m->loss})
         if (p) cudaFree(p);
+    if (m->h_loss) cudaFreeHost(m->h_loss);
+    for (cudaEvent_t e : {m->ev_in[0], m->ev_in[1], m->ev_used[0], m->ev_used[1], m->ev_loss})
+        if (e) cudaEventDestroy(e);
+    if (m->cs) cudaStreamDestroy(m->cs);
     if (m->st) cudaStreamDestroy(m->st);
     delete m;
 }
@@ -450,8 +517,15 @@ int kc_mlp_create(int in, int hid, int out, int max_batch, uint64_t seed, kc_mlp
         g_mlp_err = "stream creation failed";
         return KC_ERR_DEVICE;
     }
-    bool ok = cudaFuncSetAttribute(gemm_chain<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C_SMEM) == cudaSuccess &&
-              cudaFuncSetAttribute(gemm_chain<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C_SMEM) == cudaSuccess;
+    const cudaFuncAttribute smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    bool ok = cudaFuncSetAttribute(gemm_chain<true, 4>, smem, (int)chain_smem(4)) == cudaSuccess &&
+              cudaFuncSetAttribute(gemm_chain<true, 8>, smem, (int)chain_smem(8)) == cudaSuccess &&
+              cudaFuncSetAttribute(gemm_chain<false, 4>, smem, (int)chain_smem(4)) == cudaSuccess &&
+              cudaFuncSetAttribute(gemm_chain<false, 8>, smem, (int)chain_smem(8)) == cudaSuccess &&
+              cudaStreamCreateWithPriority(&m->cs, cudaStreamNonBlocking, prio_high) == cudaSuccess &&
+              cudaHostAlloc(reinterpret_cast<void**>(&m->h_loss), sizeof(float), cudaHostAllocDefault) == cudaSuccess;
+    for (cudaEvent_t* e : {&m->ev_in[0], &m->ev_in[1], &m->ev_used[0], &m->ev_used[1], &m->ev_loss})
+        ok &= cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
     for (int l = 0; l < 3; ++l) {
         m->nW[l] = (long)dims[l] * dims[l + 1];
         m->nb[l] = dims[l + 1];
@@ -462,10 +536,12 @@ int kc_mlp_create(int in, int hid, int out, int max_batch, uint64_t seed, kc_mlp
               dalloc(&m->vb[l], m->nb[l]) == cudaSuccess;
     }
     const long B = max_batch;
-    ok &= dalloc(&m->x, B * in) == cudaSuccess && dalloc(&m->xb, B * in) == cudaSuccess &&
+    ok &= dalloc(&m->xs[0], B * in) == cudaSuccess && dalloc(&m->xs[1], B * in) == cudaSuccess &&
+          dalloc(&m->ts[0], B * out) == cudaSuccess && dalloc(&m->ts[1], B * out) == cudaSuccess &&
+          dalloc(&m->xb, B * in) == cudaSuccess &&
           dalloc(&m->h1, B * hid) == cudaSuccess && dalloc(&m->h1b, B * hid) == cudaSuccess &&
           dalloc(&m->h2, B * hid) == cudaSuccess && dalloc(&m->h2b, B * hid) == cudaSuccess &&
-          dalloc(&m->y, B * out) == cudaSuccess && dalloc(&m->t, B * out) == cudaSuccess &&
+          dalloc(&m->y, B * out) == cudaSuccess &&
           dalloc(&m->dy, B * out) == cudaSuccess && dalloc(&m->dyb, B * out) == cudaSuccess &&
           dalloc(&m->dh2, B * hid) == cudaSuccess && dalloc(&m->dh2b, B * hid) == cudaSuccess &&
           dalloc(&m->dh1, B * hid) == cudaSuccess && dalloc(&m->dh1b, B * hid) == cudaSuccess &&
@@ -528,7 +604,7 @@ int kc_mlp_forward(kc_mlp* m, const float* x, int B, float* y) {
 int kc_mlp_gradients(kc_mlp* m, const float* x, const float* t, int B, int l, float* gw, float* gbias, float* loss) {
     if (!m || !x || !t || l < 0 || l > 2) return KC_ERR_INVALID;
     int rc = load_batch(m, x, t, B);
-    if (rc || (rc = forward(m, B)) || (rc = backward(m, B, loss))) return rc;
+    if (rc || (rc = forward(m, B)) || (rc = backward(m, B, loss, nullptr))) return rc;
     if (gw) MK(cudaMemcpyAsync(gw, m->gW[l], m->nW[l] * sizeof(float), cudaMemcpyDeviceToHost, m->st));
     if (gbias) MK(cudaMemcpyAsync(gbias, m->gb[l], m->nb[l] * sizeof(float), cudaMemcpyDeviceToHost, m->st));
     MK(cudaStreamSynchronize(m->st));
@@ -538,17 +614,16 @@ int kc_mlp_gradients(kc_mlp* m, const float* x, const float* t, int B, int l, fl
 int kc_mlp_train_step(kc_mlp* m, const float* x, const float* t, int B, float lr, float* loss) {
     if (!m || !x || !t) return KC_ERR_INVALID;
     int rc = load_batch(m, x, t, B);
-    if (rc || (rc = forward(m, B)) || (rc = backward(m, B, loss))) return rc;
+    if (rc || (rc = forward(m, B))) return rc;
     m->step++;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
+    AdamArgs adam[3][2];
     for (int l = 0; l < 3; ++l) {
-        adam<<<512, 256, 0, m->st>>>(m->W[l], m->Wb[l], m->gW[l], m->mW[l], m->vW[l], m->nW[l], lr, b1, b2, eps, c1,
-                                     c2);
-        adam<<<64, 256, 0, m->st>>>(m->b[l], nullptr, m->gb[l], m->mb[l], m->vb[l], m->nb[l], lr, b1, b2, eps, c1, c2);
+        adam[l][0] = AdamArgs{m->W[l], m->mW[l], m->vW[l], m->Wb[l], lr, b1, b2, eps, c1, c2};
+        adam[l][1] = AdamArgs{m->b[l], m->mb[l], m->vb[l], nullptr, lr, b1, b2, eps, c1, c2};
     }
-    MK(cudaGetLastError());
-    return KC_OK;
+    return backward(m, B, loss, adam);
 }
 
 }  // extern "C"
