@@ -595,7 +595,8 @@ int size_structures(kc_context* c, const std::vector<uint64_t>& kb, double scale
         uint64_t batch_keys = 0;
         for (uint32_t b = 0; b < nb; ++b) batch_keys += kb[b];
         c->init_deferred = c->nw == 1 && windows_pay(c, batch_keys);
-        const bool beside = init_bytes < 4 * batch_bytes;
+        // (a small one is not worth the events)
+        const bool beside = init_bytes < 4 * batch_bytes && init_bytes > SMALL_BYTES;
         cudaStream_t is = c->stream;
         if (beside && !c->init_deferred) {
             // after the work queued before this batch's extraction (recorded

@@ -1085,6 +1085,17 @@ static __device__ __noinline__ bool table_add_slow(Slot2* __restrict__ tab, uint
     return false;
 }
 
+__device__ __forceinline__ bool same_key(uint64_t a, uint64_t b) { return a == b; }
+__device__ __forceinline__ bool same_key(const Key2& a, const Key2& b) { return a.w0 == b.w0 && a.w1 == b.w1; }
+__device__ __forceinline__ bool same_key(const Key4& a, const Key4& b) {
+    return a.w0 == b.w0 && a.w1 == b.w1 && a.w2 == b.w2 && a.w3 == b.w3;
+}
+__device__ __forceinline__ Key4 cell_key4(const Slot4* s) {
+    const ulonglong2 a = __ldcg(reinterpret_cast<const ulonglong2*>(s));
+    const ulonglong2 b = __ldcg(reinterpret_cast<const ulonglong2*>(s) + 1);
+    return Key4{a.x, a.y, b.x, b.y};
+}
+
 // Insert `add` occurrences of a 256-bit key, probing from (h >> 17) & mask.
 // Returns 1 when added, 0 when the probe limit was hit (the bucket
 // overflows; or `overflowed` says that it has), -1 when a slot stayed
@@ -1097,7 +1108,17 @@ static __device__ __noinline__ int table_add4(Slot4* __restrict__ tab, uint64_t 
         if (p && p % PROBE_CHECK == 0 && overflowed && __ldcg(overflowed)) return 0;
         Slot4* s = tab + ((i + p) & mask);
         volatile uint32_t* state = &s->state;
+        // state and key in one round trip.  A key that agrees in all words of
+        // a READY slot is that slot's, whenever they were read (its words are
+        // written once); one that does not may have been read too early and is
+        // read again behind a fence.  A fence per probe and a second round trip
+        // made the count of 136 M keys 7.56 ms; 6.62 now.
         uint32_t st = *state;
+        Key4 have = cell_key4(s);
+        if (st == SLOT_READY && same_key(have, key)) {
+            atomicAdd(&s->count, add);
+            return 1;
+        }
         if (st == SLOT_EMPTY) {
             st = atomicCAS(&s->state, SLOT_EMPTY, SLOT_WRITING);
             if (st == SLOT_EMPTY) {  // claimed: key and first count, then publish
@@ -1116,8 +1137,8 @@ static __device__ __noinline__ int table_add4(Slot4* __restrict__ tab, uint64_t 
             st = *state;
         }
         __threadfence();  // pairs with the owner's fence: its key words are visible
-        const Key4 have{__ldcg(&s->w0), __ldcg(&s->w1), __ldcg(&s->w2), __ldcg(&s->w3)};
-        if (have.w0 == key.w0 && have.w1 == key.w1 && have.w2 == key.w2 && have.w3 == key.w3) {
+        have = cell_key4(s);
+        if (same_key(have, key)) {
             atomicAdd(&s->count, add);
             return 1;
         }
@@ -2191,11 +2212,6 @@ __device__ __forceinline__ Cell<NW> read_cell_all(const typename SlotOf<NW>::T* 
         c.used = t.y == SLOT_READY;  // after the count every used slot is ready
     }
     return c;
-}
-__device__ __forceinline__ bool same_key(uint64_t a, uint64_t b) { return a == b; }
-__device__ __forceinline__ bool same_key(const Key2& a, const Key2& b) { return a.w0 == b.w0 && a.w1 == b.w1; }
-__device__ __forceinline__ bool same_key(const Key4& a, const Key4& b) {
-    return a.w0 == b.w0 && a.w1 == b.w1 && a.w2 == b.w2 && a.w3 == b.w3;
 }
 
 // `add` keys of exact count `merged` (add may be -1: bins and totals are
