@@ -140,6 +140,7 @@ struct kc_context {
     cudaStream_t side = nullptr;
     cudaEvent_t ev_side_in = nullptr, ev_init = nullptr;
     bool init_pending = false;
+    bool cells2 = false;         // 128-bit keys: this run's filter words are fields of the table cells
     bool init_deferred = false;  // tables not initialised: the windowed count of the first batch writes every cell
     uint32_t nw = 1, bucket_bits = 8, n_buckets = 256, bucket_shift = 56;
     int sm_count = 148;
@@ -513,7 +514,7 @@ int device_scan(kc_context* c, const TI* in, uint64_t n, TO* out, uint64_t base,
 // 2 keys per cell, e.g. a whole input in one pass, not for the host path's
 // batches against the whole input's tables.
 bool windows_pay(const kc_context* c, uint64_t n_keys) {
-    return c->window_count && n_keys >= 2 * c->table_slots_used;
+    return c->window_count && (c->nw == 1 || c->cells2) && n_keys >= 2 * c->table_slots_used;
 }
 
 // Initialisation put off in the hope of a windowed count, when the batch is
@@ -522,9 +523,49 @@ int init_now(kc_context* c) {
     if (!c->init_deferred) return KC_OK;
     c->init_deferred = false;
     Stage st(c, KC_STAGE_INIT);
-    kc::init_slots<1><<<c->sm_count * 8, 256, 0, c->stream>>>(c->table.p, c->table_slots_used);
+    const int g = c->sm_count * 8;
+    if (c->nw == 1) kc::init_slots<1><<<g, 256, 0, c->stream>>>(c->table.p, c->table_slots_used);
+    else kc::init_slots<2><<<g, 256, 0, c->stream>>>(c->table.p, c->table_slots_used);
     CK(cudaGetLastError());
     return KC_OK;
+}
+
+// Whether the device has room for 128-bit keys counted in windows: `slots`
+// cells with their growth share, the keys and their sub-routed copy, and all
+// of the input's keys packed (the buffers that the context holds already
+// counted as free).  Where it has not, the filter gets its own array (1.5
+// bytes a key, not 8) and the keys no copy, so that an input is refused for
+// memory no sooner.
+bool windows2_fit(const kc_context* c, uint64_t slots, uint64_t keys, double scale) {
+    const double kb = (double)keys * sizeof(kc::Key2);
+    const double need[4] = {(double)slots * c->slot_bytes * 1.25, kb, kb * 17 / 16, (double)keys * scale * c->packed_bytes};
+    const size_t cap[4] = {c->table.cap, c->routed.cap, c->routed2.cap, c->low_packed.cap};
+    double want = 0, held = 0;
+    bool held_all = true;
+    for (int i = 0; i < 4; ++i) {
+        held_all = held_all && need[i] <= (double)cap[i];
+        want += need[i] * 9 / 8;  // as DevBuf::ensure allocates
+        held += (double)cap[i];
+    }
+    if (held_all) return true;
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return want <= (double)free_bytes + held - (double)total / 16;
+}
+
+// The global count of 128-bit keys comes in two forms.
+template <int NW>
+void count_routed(const kc_context* c, const kc::CountArgs& a, uint64_t tiles) {
+    if constexpr (NW == 2) {
+        if (c->cells2) {
+            kc::count_routed<2, true><<<tiles, kc::CNT_THREADS, 0, c->stream>>>(a);
+            return;
+        }
+    }
+    kc::count_routed<NW><<<tiles, kc::CNT_THREADS, 0, c->stream>>>(a);
 }
 
 // Allocate filter and tables from per-bucket k-mer totals of the first batch
@@ -532,45 +573,61 @@ int init_now(kc_context* c) {
 int size_structures(kc_context* c, const std::vector<uint64_t>& kb, double scale, uint64_t batch_bytes) {
     const kc_config& g = c->cfg;
     const uint32_t nb = c->n_buckets;
-    c->h_meta.assign(nb, kc::BucketMeta{});
     uint64_t bw = 0, ts = 0;
     const bool learned = g.sizing == KC_SIZING_LEARNED && c->pred_table.size() == KC_MODEL_BUCKETS;
     const uint32_t per = KC_MODEL_BUCKETS / nb;  // model buckets per engine bucket (16 or 1)
-    for (uint32_t b = 0; b < nb; ++b) {
-        const double kest = (double)kb[b] * scale;
-        uint64_t words, slots;
-        if (learned) {
-            // filter: 12 bits per predicted distinct key; table: predicted
-            // table keys with 15% headroom at the target load
-            double d = 0, t = 0;
-            for (uint32_t q = 0; q < per; ++q) {
-                d += c->pred_distinct[b * per + q];
-                t += c->pred_table[b * per + q];
+    auto place = [&](bool in_cells) {
+        c->h_meta.assign(nb, kc::BucketMeta{});
+        bw = ts = 0;
+        for (uint32_t b = 0; b < nb; ++b) {
+            const double kest = (double)kb[b] * scale;
+            uint64_t words, slots;
+            if (learned) {
+                // filter: 12 bits per predicted distinct key; table: predicted
+                // table keys with 15% headroom at the target load
+                double d = 0, t = 0;
+                for (uint32_t q = 0; q < per; ++q) {
+                    d += c->pred_distinct[b * per + q];
+                    t += c->pred_table[b * per + q];
+                }
+                words = pow2_at_least(std::max<uint64_t>((uint64_t)(d * 12.0 / 64.0), 256));
+                slots = pow2_at_least(std::max<uint64_t>((uint64_t)(t * 1.15 / g.table_load), 256));
+            } else {
+                words = pow2_at_least(std::max<uint64_t>((uint64_t)(kest * g.bloom_bits / 64.0), 256));
+                slots = pow2_at_least(std::max<uint64_t>((uint64_t)(kest * g.repeat_ratio / g.table_load), 256));
             }
-            words = pow2_at_least(std::max<uint64_t>((uint64_t)(d * 12.0 / 64.0), 256));
-            slots = pow2_at_least(std::max<uint64_t>((uint64_t)(t * 1.15 / g.table_load), 256));
-        } else {
-            words = pow2_at_least(std::max<uint64_t>((uint64_t)(kest * g.bloom_bits / 64.0), 256));
-            slots = pow2_at_least(std::max<uint64_t>((uint64_t)(kest * g.repeat_ratio / g.table_load), 256));
+            if (in_cells) {
+                // the filter is the 32-bit pad field of the table cells, at the
+                // index of the first table probe, so one read serves both; cells =
+                // the larger of the table's slots and the filter's 32-bit words.
+                // After a table grows, the old cells stay the filter.
+                slots = std::max<uint64_t>(slots, 2 * words);
+                c->h_meta[b].bloom_off = ts;
+                c->h_meta[b].bloom_mask = slots - 1;
+            } else {
+                c->h_meta[b].bloom_off = bw;
+                c->h_meta[b].bloom_mask = words - 1;
+                bw += words;
+            }
+            c->h_meta[b].tab_off = ts;
+            c->h_meta[b].tab_mask = slots - 1;
+            ts += slots;
         }
-        if (c->nw == 1) {
-            // 64-bit keys: the filter is the 32-bit pad field of the table
-            // cells, at the index of the first table probe, so one read serves
-            // both; cells = the larger of the table's slots and the filter's
-            // 32-bit words.  After a table grows, the old cells stay the filter.
-            slots = std::max<uint64_t>(slots, 2 * words);
-            c->h_meta[b].bloom_off = ts;
-            c->h_meta[b].bloom_mask = slots - 1;
-        } else {
-            c->h_meta[b].bloom_off = bw;
-            c->h_meta[b].bloom_mask = words - 1;
-            bw += words;
-        }
-        c->h_meta[b].tab_off = ts;
-        c->h_meta[b].tab_mask = slots - 1;
-        ts += slots;
+    };
+    // 64-bit keys always; 128-bit keys (k <= 63: count_window's claims need a
+    // second word that is never EMPTY) when the batch will be counted in
+    // windows: outside them an array of its own is faster (first occurrences
+    // then dirty a bit of it, not a cell: 12.0 against 13.2 ms at k = 63)
+    place(c->nw == 1);
+    uint64_t batch_keys = 0;
+    for (uint32_t b = 0; b < nb; ++b) batch_keys += kb[b];
+    c->cells2 = false;
+    if (c->nw == 2 && g.k <= 63 && c->window_count) {
+        place(true);
+        c->cells2 = batch_keys >= 2 * ts && windows2_fit(c, ts, batch_keys, scale);
+        if (!c->cells2) place(false);
     }
-    c->bloom_words = c->nw == 1 ? ts / 2 : bw;  // in 64-bit words (cells hold 32 filter bits each)
+    c->bloom_words = c->nw == 1 || c->cells2 ? ts / 2 : bw;  // in 64-bit words (cells hold 32 filter bits each)
     c->table_slots_used = ts;
     c->win_ready = false;
     CK(c->bloom.ensure(bw * sizeof(uint64_t)));
@@ -588,13 +645,11 @@ int size_structures(kc_context* c, const std::vector<uint64_t>& kb, double scale
         // of 128-bit tables behind a 2 GiB batch slowed that batch's
         // extraction and still held up the count.
         //
-        // 64-bit keys that will be counted in windows (their number estimated
-        // from the histogram) need none: the windowed count starts its cells
+        // Keys that will be counted in windows (their number estimated from
+        // the histogram) need none: the windowed count starts its cells
         // EMPTY and writes them all.
         const uint64_t init_bytes = bw * sizeof(uint64_t) + ts * c->slot_bytes;
-        uint64_t batch_keys = 0;
-        for (uint32_t b = 0; b < nb; ++b) batch_keys += kb[b];
-        c->init_deferred = c->nw == 1 && windows_pay(c, batch_keys);
+        c->init_deferred = windows_pay(c, batch_keys);
         // (a small one is not worth the events)
         const bool beside = init_bytes < 4 * batch_bytes && init_bytes > SMALL_BYTES;
         cudaStream_t is = c->stream;
@@ -650,7 +705,7 @@ int launch_count(kc_context* c, uint64_t n_keys, int use_filter) {
     a.use_filter = use_filter;
     a.filter_in_table = c->nw == 1;
     Stage st(c, use_filter ? KC_STAGE_COUNT_ROUTED : KC_STAGE_REHASH);
-    kc::count_routed<NW><<<tiles, kc::CNT_THREADS, 0, c->stream>>>(a);
+    count_routed<NW>(c, a, tiles);
     CK(cudaGetLastError());
     return KC_OK;
 }
@@ -756,8 +811,9 @@ bool build_windows(kc_context* c, uint32_t nb) {
         const kc::BucketMeta& m = c->h_meta[b];
         if (m.bloom_off != m.tab_off || m.bloom_mask != m.tab_mask) return false;
         const uint64_t cells = m.tab_mask + 1;
-        const uint32_t n = cells <= (uint64_t)kc::WIN_Z ? 1u : (uint32_t)(cells >> kc::WIN_ZSHIFT);
-        c->h_bucket_win[b] = kc::BucketWin{(uint32_t)c->h_win_info.size(), n == 1 ? kc::WIN_SINGLE : kc::WIN_ZSHIFT};
+        const uint32_t zshift = c->nw == 1 ? kc::Win<1>::ZSHIFT : kc::Win<2>::ZSHIFT;
+        const uint32_t n = cells <= (1ull << zshift) ? 1u : (uint32_t)(cells >> zshift);
+        c->h_bucket_win[b] = kc::BucketWin{(uint32_t)c->h_win_info.size(), n == 1 ? kc::WIN_SINGLE : zshift};
         for (uint32_t q = 0; q < n; ++q) c->h_win_info.push_back(kc::WinInfo{b, q});
     }
     c->n_wins = c->h_win_info.size();
@@ -800,7 +856,7 @@ int launch_count_range(kc_context* c, uint64_t off, uint64_t n, int use_filter) 
     a.use_filter = use_filter;
     a.filter_in_table = c->nw == 1;
     Stage st(c, KC_STAGE_COUNT_ROUTED);
-    kc::count_routed<NW><<<tiles, kc::CNT_THREADS, 0, c->stream>>>(a);
+    count_routed<NW>(c, a, tiles);
     CK(cudaGetLastError());
     return KC_OK;
 }
@@ -814,10 +870,14 @@ int launch_count_range(kc_context* c, uint64_t off, uint64_t n, int use_filter) 
 // overflowed keys as count_routed leaves them, and n_keys becomes its length.
 // A multi-set batch (sets.n sets, nb = 256 buckets each) takes exact ranges:
 // a spill area would mix the sets' keys.  src: the keys, where they are not
-// in `routed` (read only).
+// in `routed` (read only).  NO_WINDOWS, with nothing counted, when the second
+// key buffer does not fit the device.
+constexpr int NO_WINDOWS = 2;
+template <int NW>
 int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets = {nullptr, 0},
-                 const uint64_t* src = nullptr) {
-    if (!src) src = c->routed.as<uint64_t>();
+                 const void* src = nullptr) {
+    using K = typename kc::KeyOf<NW>::T;
+    if (!src) src = c->routed.p;
     const uint64_t nw = c->n_wins;
     if (!c->win_ready) {
         CK(c->bucket_win.ensure(nb * sizeof(kc::BucketWin)));
@@ -852,8 +912,8 @@ int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets 
             Stage st(c, KC_STAGE_SUBROUTE, 2);
             const uint64_t g = ceil_div(cchunks, stride);
             if (g)
-                kc::subroute_count<<<g, kc::SUB_THREADS, 0, c->stream>>>(
-                    src, n_keys, meta, bwin, c->bucket_shift, stride, sets, c->win_count.as<uint32_t>());
+                kc::subroute_count<NW><<<g, kc::SUB_THREADS, 0, c->stream>>>(
+                    static_cast<const K*>(src), n_keys, meta, bwin, c->bucket_shift, stride, sets, c->win_count.as<uint32_t>());
             kc::window_caps<<<small_grid, 256, 0, c->stream>>>(c->win_count.as<uint32_t>(), nw, stride,
                                                                 c->win_padded.as<uint32_t>());
             CK(cudaGetLastError());
@@ -867,7 +927,12 @@ int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets 
         spill_start = total;
         const uint64_t spill_cap = stride > 1 ? std::max<uint64_t>(1ull << 16, (total / 16 + 63) & ~63ull) : 0;
         const uint64_t arr = total + spill_cap;
-        CK(c->routed2.ensure(std::max<uint64_t>(arr, 1) * sizeof(uint64_t)));
+        const cudaError_t room = c->routed2.ensure(std::max<uint64_t>(arr, 1) * sizeof(K));
+        if (room == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            return NO_WINDOWS;
+        }
+        CK(room);
         CK(c->tile_low.ensure(std::max<uint64_t>(arr / kc::WIN_SEG, 1) * sizeof(uint32_t)));
         CK(c->tile_fail.ensure(std::max<uint64_t>(arr / kc::WIN_SEG, 1) * sizeof(uint32_t)));
         CK(c->tile_low_prefix.ensure(std::max<uint64_t>(arr / kc::WIN_SEG, 1) * sizeof(uint64_t)));
@@ -889,11 +954,12 @@ int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets 
             sa.spill_cursor = reinterpret_cast<unsigned long long*>(d_scal + 5);
             sa.spill_end = arr;
             sa.spill_full = d_spill_full;
-            sa.out = c->routed2.as<uint64_t>();
+            sa.out = c->routed2.p;
             sa.sets = sets;
             if (n_keys)
-                (sets.n ? kc::subroute_scatter<true> : kc::subroute_scatter<false>)<<<
-                    ceil_div(n_keys, kc::SCAT_CHUNK), kc::SCAT_THREADS, kc::scatter_smem_bytes(), c->stream>>>(sa);
+                (sets.n ? kc::subroute_scatter<NW, true> : kc::subroute_scatter<NW, false>)<<<
+                    ceil_div(n_keys, kc::scat_chunk<NW>()), kc::SCAT_THREADS, kc::scatter_smem_bytes<NW>(),
+                    c->stream>>>(sa);
             CK(cudaGetLastError());
         }
         uint32_t full = 0;
@@ -914,7 +980,7 @@ int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets 
     c->win_result_spill_seg = spill_start / kc::WIN_SEG;
     CKR(join_init(c));
     kc::WindowArgs a{};
-    a.keys = c->routed.as<uint64_t>();
+    a.keys = c->routed.p;
     a.win_start = c->win_start.as<uint64_t>();
     a.win_fill = c->win_cursor.as<unsigned long long>();
     a.win_cap = c->win_padded.as<uint32_t>();
@@ -922,7 +988,7 @@ int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets 
     a.order = c->win_order.as<uint32_t>();
     a.bw = bwin;
     a.meta = meta;
-    a.table = c->table.as<kc::Slot1>();
+    a.table = c->table.p;
     a.seg_low = c->tile_low.as<uint32_t>();
     a.seg_fail = c->tile_fail.as<uint32_t>();
     a.bucket_overflow = c->overflow.as<uint32_t>();
@@ -935,11 +1001,12 @@ int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets 
             a.phase = ph;
             a.order_base = ph ? (uint32_t)c->n_wins_phase0 : 0u;
             const uint64_t grid = ph ? nw - c->n_wins_phase0 : c->n_wins_phase0;
-            if (grid) kc::count_window<<<grid, kc::WIN_THREADS, kc::window_smem_bytes(), c->stream>>>(a);
+            if (grid)
+                kc::count_window<NW><<<grid, kc::Win<NW>::THREADS, kc::window_smem_bytes<NW>(), c->stream>>>(a);
         }
         CK(cudaGetLastError());
     }
-    if (spill_used) CKR(launch_count_range<1>(c, spill_start, spill_used, 1));
+    if (spill_used) CKR(launch_count_range<NW>(c, spill_start, spill_used, 1));
     c->window_spill += spill_used;
     CK(cudaGetLastError());
     return KC_OK;
@@ -1165,14 +1232,14 @@ int finish_checks(kc_context* c, bool* grew) {
     return KC_OK;
 }
 
-// Whether the context's device can read p in place as 8-byte words.
+// Whether the context's device can read p in place, key by key.
 bool on_device(const kc_context* c, const void* p) {
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return at.type == cudaMemoryTypeDevice && at.device == c->device && reinterpret_cast<uintptr_t>(p) % 8 == 0;
+    return at.type == cudaMemoryTypeDevice && at.device == c->device && reinterpret_cast<uintptr_t>(p) % (8 * c->nw) == 0;
 }
 
 // Copy the caller's keys into `routed` (cap bytes).
@@ -1202,15 +1269,16 @@ int count_and_pack(kc_context* c, uint64_t n_keys, const void* src) {
     uint64_t* d_scal = c->scalars.as<uint64_t>();
     int rc;
     bool windowed = false;
-    if constexpr (NW == 1) {
-        // 64-bit keys count in shared-memory windows while every bucket's
-        // filter sits in its table's cells (no table has grown yet)
+    if constexpr (NW <= 2) {
+        // 64- and 128-bit keys count in shared-memory windows while every
+        // bucket's filter sits in its table's cells (no table has grown yet)
         if (windows_pay(c, n_keys) && (c->win_ready || build_windows(c, c->n_buckets))) {
-            const uint64_t* keys = nullptr;
-            if (src && on_device(c, src)) keys = static_cast<const uint64_t*>(src);
-            else if (src) CKR(take_keys(c, src, n_keys * sizeof(uint64_t), ceil_div(n_keys, CT) * CT * sizeof(uint64_t)));
-            if ((rc = window_count(c, n_keys, c->n_buckets, {nullptr, 0}, keys))) return rc;
-            windowed = true;
+            const void* keys = nullptr;
+            if (src && on_device(c, src)) keys = src;
+            else if (src) CKR(take_keys(c, src, n_keys * (uint64_t)(8 * NW), ceil_div(n_keys, CT) * CT * (uint64_t)(8 * NW)));
+            rc = window_count<NW>(c, n_keys, c->n_buckets, {nullptr, 0}, keys);
+            if (rc && rc != NO_WINDOWS) return rc;
+            windowed = rc == 0;
         }
     }
     if (!windowed) {
@@ -1427,6 +1495,7 @@ int begin_run(kc_context* c, uint64_t total_bytes) {
     c->batch_result = false;
     c->win_result = false;
     c->init_deferred = false;
+    c->cells2 = false;
     c->expected_total_bytes = total_bytes;
     c->ev_used = 0;
     c->spans.clear();
@@ -1493,7 +1562,8 @@ void fill_stats(kc_context* c, kc_stats* s, double dev_ms, double wall_ms) {
         live += m.tab_mask + 1;
         s->max_bucket_table_slots = std::max<uint64_t>(s->max_bucket_table_slots, m.tab_mask + 1);
         s->max_bucket_filter_words =
-            std::max<uint64_t>(s->max_bucket_filter_words, c->nw == 1 ? (m.bloom_mask + 1) / 2 : m.bloom_mask + 1);
+            std::max<uint64_t>(s->max_bucket_filter_words,
+                               c->nw == 1 || c->cells2 ? (m.bloom_mask + 1) / 2 : m.bloom_mask + 1);
     }
     s->table_slots = live;
     s->filter_words = c->bloom_words;
@@ -1729,13 +1799,17 @@ int kc_create(const kc_config* cfg, kc_context** out) {
                          (int)kc::extract_smem_bytes<4, kc::HIST>(4096));
     cudaFuncSetAttribute(kc::extract_kernel<4, kc::SCATTER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kc::extract_smem_bytes<4, kc::SCATTER>(4096));
-    cudaFuncSetAttribute(kc::count_window, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::window_smem_bytes());
-    cudaFuncSetAttribute(kc::hist_window, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::window_smem_bytes());
+    cudaFuncSetAttribute(kc::count_window<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::window_smem_bytes<1>());
+    cudaFuncSetAttribute(kc::count_window<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::window_smem_bytes<2>());
+    cudaFuncSetAttribute(kc::hist_window<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::hist_window_smem<1>());
+    cudaFuncSetAttribute(kc::hist_window<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::hist_window_smem<2>());
     cudaFuncSetAttribute(kc::loads_table_pass<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::loads_table_smem());
     cudaFuncSetAttribute(kc::loads_table_pass<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::loads_table_smem());
     cudaFuncSetAttribute(kc::loads_table_pass<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::loads_table_smem());
-    for (auto k : {kc::subroute_scatter<false>, kc::subroute_scatter<true>})
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::scatter_smem_bytes());
+    for (auto k : {kc::subroute_scatter<1, false>, kc::subroute_scatter<1, true>})
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kc::scatter_smem_bytes<1>());
+    cudaFuncSetAttribute(kc::subroute_scatter<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)kc::scatter_smem_bytes<2>());
     if ((e = cudaGetLastError()) != cudaSuccess) {
         delete c;
         return fail(KC_ERR_DEVICE, "kernel attribute setup failed: %s", cudaGetErrorString(e));
@@ -2162,7 +2236,7 @@ int histogram_kernels(kc_context* c, uint32_t min_freq, uint32_t max_freq, unsig
     const auto* meta = c->meta.as<kc::BucketMeta>();
     const uint64_t* prefix = nullptr;
     uint64_t nsegs = 0, first_seg = 0;
-    if constexpr (NW == 1) {
+    if constexpr (NW <= 2) {
         if (c->win_result) {
             kc::HistWindowArgs a{};
             a.low = c->low_packed.as<uint8_t>();
@@ -2175,14 +2249,14 @@ int histogram_kernels(kc_context* c, uint32_t min_freq, uint32_t max_freq, unsig
             a.wins = c->win_info.as<kc::WinInfo>();
             a.bw = c->bucket_win.as<kc::BucketWin>();
             a.meta = meta;
-            a.table = c->table.as<kc::Slot1>();
+            a.table = c->table.p;
             a.k = c->cfg.k;
             a.lo = min_freq;
             a.hi = max_freq;
             a.gh = d;
             a.extra = d + bins;
-            const uint64_t grid = std::min<uint64_t>(c->n_wins, (uint64_t)c->sm_count * 3);
-            kc::hist_window<<<grid, kc::WIN_THREADS, kc::window_smem_bytes(), c->stream>>>(a);
+            const uint64_t grid = std::min<uint64_t>(c->n_wins, (uint64_t)c->sm_count * kc::Win<NW>::HIST_CTAS);
+            kc::hist_window<NW><<<grid, kc::WIN_THREADS, kc::hist_window_smem<NW>(), c->stream>>>(a);
             CK(cudaGetLastError());
             if (a.spill_seg >= a.nsegs) return KC_OK;  // nothing spilled
             prefix = a.prefix;
@@ -2749,7 +2823,10 @@ route_again:
     if constexpr (NW == 1) {
         if (windowed) {
             CK(cudaMemcpyAsync(d_key0, set_key0.data(), n_sets * sizeof(uint64_t), cudaMemcpyHostToDevice, c->stream));
-            if ((rc = window_count(c, n_keys, (uint32_t)nbk, kc::SetSpan{d_key0, n_sets}))) return rc;
+            if ((rc = window_count<1>(c, n_keys, (uint32_t)nbk, kc::SetSpan{d_key0, n_sets}))) {
+                // (routed2 was sized above)
+                return rc == NO_WINDOWS ? fail(KC_ERR_DEVICE, "no memory for the sub-routed keys") : rc;
+            }
             c->win_ready = false;
             nsegs = n_keys / SEG;
             kc::set_window_segs<<<std::max<uint64_t>(1, ceil_div(n_sets, 256)), 256, 0, c->stream>>>(

@@ -1279,8 +1279,11 @@ constexpr int CNT_SEGS_PER_WARP = 8;
 // adds follow.  Outputs are compacted IN PLACE into the warp's own segment
 // (only this warp reads it; __syncwarp orders reads before writes): first
 // occurrences at the front, keys that met a full table at the back.
-template <int NW>
+// CELLS2: 128-bit keys whose filter words are fields of the table cells (a run
+// counted in windows; its spilled, retried and later keys come here).
+template <int NW, bool CELLS2 = false>
 __global__ void __launch_bounds__(CNT_THREADS, count_min_ctas<NW>()) count_routed(CountArgs a) {
+    static_assert(!CELLS2 || NW == 2, "128-bit keys only");
     using K = typename KeyOf<NW>::T;
     using S = typename SlotOf<NW>::T;
     // first table slot read ahead of the filter result (not for 256-bit keys,
@@ -1416,7 +1419,10 @@ __global__ void __launch_bounds__(CNT_THREADS, count_min_ctas<NW>()) count_route
                         seen[j] = __ldcg(&slot->key);
                     }
                 } else {
-                    if (a.use_filter) old[j] = __ldcg(a.bloom + m.bloom_off + (h[j] & m.bloom_mask));
+                    if constexpr (CELLS2)
+                        old[j] = __ldcg(&(table + m.bloom_off + ((h[j] >> 17) & m.bloom_mask))->pad[0]);
+                    else if (a.use_filter)
+                        old[j] = __ldcg(a.bloom + m.bloom_off + (h[j] & m.bloom_mask));
                     if constexpr (NW == 2) seen[j] = __ldcg(reinterpret_cast<const ulonglong2*>(slot));
                     else seen[j] = 0;
                 }
@@ -1427,7 +1433,7 @@ __global__ void __launch_bounds__(CNT_THREADS, count_min_ctas<NW>()) count_route
             // every item's filter atomic is issued before any old value is
             // tested (old[j] is replaced by the atomic's return value; an item
             // whose bits were all set already keeps its read value)
-            bool in_table = false;
+            bool in_table = CELLS2;
             if constexpr (NW == 1) in_table = a.filter_in_table != 0;
             uint32_t issued = 0;
 #pragma unroll
@@ -1444,6 +1450,9 @@ __global__ void __launch_bounds__(CNT_THREADS, count_min_ctas<NW>()) count_route
                                 old[j] = atomicOr(reinterpret_cast<unsigned long long*>(a.bloom + m.bloom_off +
                                                                                         (h[j] & m.bloom_mask)),
                                                   bits);
+                        } else if constexpr (CELLS2) {
+                            old[j] = atomicOr(&(table + m.bloom_off + ((h[j] >> 17) & m.bloom_mask))->pad[0],
+                                              (uint32_t)bits);
                         } else {
                             old[j] = atomicOr(
                                 reinterpret_cast<unsigned long long*>(a.bloom + m.bloom_off + (h[j] & m.bloom_mask)), bits);

@@ -1,5 +1,5 @@
-// Windowed count of 64-bit keys: first-occurrence filter and repeat table in
-// shared memory.
+// Windowed count of 64- and 128-bit keys (k <= 63): first-occurrence filter and
+// repeat table in shared memory.
 //
 // The count_routed kernel works on a bucket-sorted key array against the
 // bucket's filter + table cells in global memory: every key costs a cell
@@ -38,6 +38,11 @@
 //                     low.bin keys looked up in its staged cells     low.bin)
 // Small batches, and a batch whose spill area overflows, take exact window
 // counts (every chunk) instead: exact ranges, no spill.
+//
+// 128-bit keys (one device pass, 6 M reads at k = 63, 4096 buckets, 496 M keys;
+// before: the global count, an initialisation beside the extraction, global
+// histogram lookups): sub-routing 5.6 + count 5.7 ms against 12.1, extraction
+// 5.4 -> 4.7, histogram 4.4 -> 2.8; count + histogram 25.0 -> 22.2.
 #pragma once
 
 #include <cstdint>
@@ -47,12 +52,22 @@
 
 namespace kc {
 
-constexpr int WIN_Z = 4096;                        // cells owned by one window
-constexpr int WIN_HALO = PROBE_LIMIT;              // cells staged after it
-constexpr int WIN_CELLS = WIN_Z + WIN_HALO;        // staged per CTA (16 B each: 73.7 KB)
-constexpr uint32_t WIN_ZSHIFT = 12;                // log2(WIN_Z)
+constexpr int WIN_HALO = PROBE_LIMIT;              // cells staged after a window's own
 constexpr uint32_t WIN_SINGLE = 63;                // zshift of a one-window bucket
-constexpr int WIN_THREADS = 512;
+template <int NW>
+struct Win {
+    static constexpr uint32_t ZSHIFT = NW == 1 ? 12 : 11;     // log2(Z)
+    static constexpr int Z = 1 << ZSHIFT;                     // cells owned by one window
+    static constexpr int CELLS = Z + WIN_HALO;                // staged per CTA
+    static constexpr int CELL_BYTES = 8 * NW + 8;             // key, count, filter word: 73.7 / 61.4 KB a CTA
+    // count_window: 128-bit keys take 56 registers; 6 M reads at k = 63 count
+    // in 5.7 ms so, 6.1 with 2 CTAs of 512 threads, 6.9 with 3 of 512 (spills)
+    static constexpr int THREADS = NW == 1 ? 512 : 384;
+    static constexpr int CTAS = 3;                            // of count_window per SM
+    static constexpr int HIST_CTAS = NW == 1 ? 3 : 2;         // of hist_window (whole cells: 73.7 / 81.9 KB)
+    static constexpr int SCAT_ITEMS = NW == 1 ? 8 : 4;        // keys per thread of subroute_scatter
+};
+constexpr int WIN_THREADS = 512;                   // hist_window
 constexpr int WIN_SEG = 64;                        // count_seg<1>(): output segment of 64 keys
 constexpr int WIN_GROUP = 1;                       // segments a warp loads at once
 constexpr int SUB_THREADS = 256;
@@ -78,9 +93,33 @@ struct WinCache {
     BucketWin w;
     uint64_t mask;
 };
-__device__ __forceinline__ uint32_t window_of(uint64_t key, uint32_t bucket_shift, const WinCache& c,
+__device__ __forceinline__ bool key_empty(uint64_t k) { return k == EMPTY; }
+__device__ __forceinline__ bool key_empty(const Key2& k) { return k.w0 == EMPTY && k.w1 == EMPTY; }
+template <int NW>
+__device__ __forceinline__ typename KeyOf<NW>::T empty_key() {
+    if constexpr (NW == 1) return EMPTY;
+    else return Key2{EMPTY, EMPTY};
+}
+// A routed key, read once.
+__device__ __forceinline__ uint64_t stream_key(const uint64_t* p) { return __ldcs(p); }
+__device__ __forceinline__ Key2 stream_key(const Key2* p) {
+    const ulonglong2 v = __ldcs(reinterpret_cast<const ulonglong2*>(p));
+    return Key2{v.x, v.y};
+}
+__device__ __forceinline__ uint64_t load_key(const uint64_t* p) { return *p; }
+__device__ __forceinline__ Key2 load_key(const Key2* p) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+    return Key2{v.x, v.y};
+}
+__device__ __forceinline__ void put_key(uint64_t* p, uint64_t k) { *p = k; }
+__device__ __forceinline__ void put_key(Key2* p, const Key2& k) {
+    *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(k.w0, k.w1);
+}
+
+template <class K>
+__device__ __forceinline__ uint32_t window_of(const K& key, uint32_t bucket_shift, const WinCache& c,
                                               const BucketMeta* __restrict__ meta, const BucketWin* __restrict__ bw) {
-    const uint32_t b = (uint32_t)(key >> bucket_shift);
+    const uint32_t b = (uint32_t)(key_hi(key) >> bucket_shift);
     BucketWin w = c.w;
     uint64_t m = c.mask;
     if (b != c.bucket) {
@@ -108,12 +147,13 @@ __device__ __forceinline__ uint32_t first_bucket(const SetSpan& sets, uint64_t i
 }
 
 // Smallest bucket of the chunk's keys (EMPTY keys skipped); 0xFFFFFFFF if none.
-__device__ __forceinline__ uint32_t chunk_min_bucket(const uint64_t (&k)[SUB_ITEMS], uint32_t bucket_shift,
+template <class K>
+__device__ __forceinline__ uint32_t chunk_min_bucket(const K (&k)[SUB_ITEMS], uint32_t bucket_shift,
                                                      uint32_t* s_min) {
     uint32_t m = 0xFFFFFFFFu;
 #pragma unroll
     for (int j = 0; j < SUB_ITEMS; ++j)
-        if (k[j] != EMPTY) m = min(m, (uint32_t)(k[j] >> bucket_shift));
+        if (!key_empty(k[j])) m = min(m, (uint32_t)(key_hi(k[j]) >> bucket_shift));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) atomicMin(s_min, m);
@@ -126,21 +166,24 @@ __device__ __forceinline__ uint32_t chunk_min_bucket(const uint64_t (&k)[SUB_ITE
 // window of the chunk's smallest bucket; windows out of that span (keys of
 // the extraction's overflow area, or a chunk spanning many tiny buckets) go
 // to global atomics.
-__global__ void __launch_bounds__(SUB_THREADS) subroute_count(const uint64_t* __restrict__ keys, uint64_t n,
+template <int NW>
+__global__ void __launch_bounds__(SUB_THREADS) subroute_count(const typename KeyOf<NW>::T* __restrict__ keys, uint64_t n,
                                                              const BucketMeta* __restrict__ meta,
                                                              const BucketWin* __restrict__ bw, uint32_t bucket_shift,
                                                              uint32_t chunk_stride, SetSpan sets,
                                                              uint32_t* __restrict__ win_count) {
+    using K = typename KeyOf<NW>::T;
     __shared__ uint32_t hist[SUB_BINS];
     __shared__ uint32_t s_min;
     const uint64_t c0 = (uint64_t)blockIdx.x * chunk_stride * SUB_CHUNK;
     for (int i = threadIdx.x; i < SUB_BINS; i += SUB_THREADS) hist[i] = 0;
     if (threadIdx.x == 0) s_min = 0xFFFFFFFFu;
-    uint64_t k[SUB_ITEMS];
+    K k[SUB_ITEMS];
 #pragma unroll
     for (int j = 0; j < SUB_ITEMS; ++j) {
         const uint64_t i = c0 + (uint64_t)j * SUB_THREADS + threadIdx.x;
-        k[j] = i < n ? __ldcs(keys + i) : EMPTY;
+        k[j] = empty_key<NW>();
+        if (i < n) k[j] = stream_key(keys + i);
     }
     bool split = false;  // a chunk that lies in several sets: every key by itself
     if (sets.n) {
@@ -156,8 +199,9 @@ __global__ void __launch_bounds__(SUB_THREADS) subroute_count(const uint64_t* __
 #pragma unroll 1
         for (int j = 0; j < SUB_ITEMS; ++j) {
             const uint64_t i = c0 + (uint64_t)j * SUB_THREADS + threadIdx.x;
-            const uint64_t key = i < n ? keys[i] : EMPTY;
-            if (key == EMPTY) continue;
+            if (i >= n) continue;
+            const K key = stream_key(keys + i);
+            if (key_empty(key)) continue;
             const uint32_t b = first_bucket(sets, i);
             atomicAdd(&win_count[window_of(key, bucket_shift, WinCache{0xFFFFFFFFu, {}, 0}, meta + b, bw + b)], 1u);
         }
@@ -169,7 +213,7 @@ __global__ void __launch_bounds__(SUB_THREADS) subroute_count(const uint64_t* __
     const uint32_t r0 = wc.w.range_base;
 #pragma unroll
     for (int j = 0; j < SUB_ITEMS; ++j) {
-        if (k[j] == EMPTY) continue;
+        if (key_empty(k[j])) continue;
         const uint32_t r = window_of(k[j], bucket_shift, wc, meta, bw);
         if (r - r0 < (uint32_t)SUB_BINS) atomicAdd(&hist[r - r0], 1u);
         else atomicAdd(&win_count[r], 1u);
@@ -212,17 +256,20 @@ __global__ void window_bounds(const uint64_t* __restrict__ start, const uint32_t
 }
 
 constexpr int SCAT_THREADS = 512;
-constexpr int SCAT_ITEMS = 8;
-constexpr int SCAT_CHUNK = SCAT_THREADS * SCAT_ITEMS;  // 4096 keys
 constexpr int SCAT_BINS = 1024;                         // windows staged in shared memory
 constexpr int SCAT_WARPS = SCAT_THREADS / 32;
+template <int NW>
+constexpr int scat_chunk() {  // 4096 keys of 64 bits, 2048 of 128
+    return SCAT_THREADS * Win<NW>::SCAT_ITEMS;
+}
 // dynamic shared memory of subroute_scatter
+template <int NW>
 constexpr size_t scatter_smem_bytes() {
-    return (size_t)SCAT_CHUNK * 8 + (size_t)SCAT_BINS * (8 + 8 + 4 + 4) + (size_t)SCAT_CHUNK * 2;
+    return (size_t)scat_chunk<NW>() * 8 * NW + (size_t)SCAT_BINS * (8 + 8 + 4 + 4) + (size_t)scat_chunk<NW>() * 2;
 }
 
 struct ScatterArgs {
-    const uint64_t* keys;
+    const void* keys;
     uint64_t n;
     const BucketMeta* meta;
     const BucketWin* bw;
@@ -232,7 +279,7 @@ struct ScatterArgs {
     unsigned long long* spill_cursor;
     uint64_t spill_end;
     uint32_t* spill_full;            // set when the spill area overflowed
-    uint64_t* out;
+    void* out;
     SetSpan sets;
 };
 
@@ -251,11 +298,15 @@ struct ScatterArgs {
 // genome shape (1163 M keys, 18.6 GB): 6.84 -> 5.94 ms, 0.48 of the copy
 // bandwidth, by the 32-bit window, five barriers instead of eight and one
 // addition per key written.
-template <bool SETS>
+template <int NW, bool SETS>
 __global__ void __launch_bounds__(SCAT_THREADS, 3) subroute_scatter(ScatterArgs a) {
     extern __shared__ __align__(16) uint8_t sc_smem[];
-    uint64_t* stage = reinterpret_cast<uint64_t*>(sc_smem);
-    uint64_t* gdelta = stage + SCAT_CHUNK;   // window l: staged place i goes to out[gdelta[l] + i],
+    using K = typename KeyOf<NW>::T;
+    constexpr int SCAT_ITEMS = Win<NW>::SCAT_ITEMS, SCAT_CHUNK = scat_chunk<NW>();
+    const K* in = static_cast<const K*>(a.keys);
+    K* out = static_cast<K*>(a.out);
+    K* stage = reinterpret_cast<K*>(sc_smem);
+    uint64_t* gdelta = reinterpret_cast<uint64_t*>(stage + SCAT_CHUNK);  // window l: staged place i goes to out[gdelta[l] + i],
     uint64_t* sdelta = gdelta + SCAT_BINS;   //   or, from limit[l] on, to the spill area at sdelta[l] + i
     uint32_t* hist = reinterpret_cast<uint32_t*>(sdelta + SCAT_BINS);  // counts, then staging offsets
     uint32_t* limit = hist + SCAT_BINS;
@@ -264,11 +315,12 @@ __global__ void __launch_bounds__(SCAT_THREADS, 3) subroute_scatter(ScatterArgs 
     __shared__ __align__(16) uint32_t s_tot[SCAT_WARPS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t c0 = (uint64_t)blockIdx.x * SCAT_CHUNK;
-    uint64_t k[SCAT_ITEMS];
+    K k[SCAT_ITEMS];
 #pragma unroll
     for (int j = 0; j < SCAT_ITEMS; ++j) {
         const uint64_t i = c0 + (uint64_t)j * SCAT_THREADS + tid;
-        k[j] = i < a.n ? __ldcs(a.keys + i) : EMPTY;
+        k[j] = empty_key<NW>();
+        if (i < a.n) k[j] = stream_key(in + i);
     }
     for (int i = tid; i < SCAT_BINS; i += SCAT_THREADS) hist[i] = 0;
     if (tid == 0) {
@@ -282,7 +334,7 @@ __global__ void __launch_bounds__(SCAT_THREADS, 3) subroute_scatter(ScatterArgs 
         uint32_t lo = 0xFFFFFFFFu, hi = 0;
 #pragma unroll
         for (int j = 0; j < SCAT_ITEMS; ++j) {
-            const uint32_t t = (uint32_t)(k[j] >> 32);
+            const uint32_t t = (uint32_t)(key_hi(k[j]) >> 32);
             lo = min(lo, t);
             hi = max(hi, t);
         }
@@ -309,7 +361,7 @@ __global__ void __launch_bounds__(SCAT_THREADS, 3) subroute_scatter(ScatterArgs 
     const uint64_t bmask = __ldg(&meta[bmin].tab_mask);
     const uint32_t r0 = bwin.range_base;
     const WinCache wc{split ? 0xFFFFFFFFu : bmin, bwin, bmask};
-    auto general_window = [&](uint64_t key, int j) {
+    auto general_window = [&](const K& key, int j) {
         if (!SETS || !split) return window_of(key, a.bucket_shift, wc, meta, bw);
         const uint32_t b = first_bucket(a.sets, c0 + (uint64_t)j * SCAT_THREADS + tid);
         return window_of(key, a.bucket_shift, wc, a.meta + b, a.bw + b);
@@ -323,17 +375,17 @@ __global__ void __launch_bounds__(SCAT_THREADS, 3) subroute_scatter(ScatterArgs 
     if (uniform) {
         // windows of at most 2^32 cells: 32-bit arithmetic
         const uint32_t wmask = bwin.zshift >= WIN_SINGLE ? 0u : (uint32_t)bmask;
-        bins = min((uint32_t)SCAT_BINS, (wmask >> WIN_ZSHIFT) + 1);
+        bins = min((uint32_t)SCAT_BINS, (wmask >> Win<NW>::ZSHIFT) + 1);
 #pragma unroll
         for (int j = 0; j < SCAT_ITEMS; ++j) {
-            const uint32_t l = ((uint32_t)(hash_key(k[j]) >> 17) & wmask) >> WIN_ZSHIFT;
+            const uint32_t l = ((uint32_t)(hash_key(k[j]) >> 17) & wmask) >> Win<NW>::ZSHIFT;
             slot[j] = l < (uint32_t)SCAT_BINS ? (l << 16) | atomicAdd(&hist[l], 1u) : FAR;
         }
     } else {
 #pragma unroll
         for (int j = 0; j < SCAT_ITEMS; ++j) {
             slot[j] = FAR;
-            if (k[j] == EMPTY) continue;
+            if (key_empty(k[j])) continue;
             const uint32_t l = general_window(k[j], j) - r0;
             if (l < (uint32_t)SCAT_BINS) slot[j] = (l << 16) | atomicAdd(&hist[l], 1u);
         }
@@ -384,16 +436,16 @@ __global__ void __launch_bounds__(SCAT_THREADS, 3) subroute_scatter(ScatterArgs 
         if (slot[j] != FAR) {
             const uint32_t l = slot[j] >> 16;
             const uint32_t pos = hist[l] + (slot[j] & 0xFFFFu);
-            stage[pos] = k[j];
+            put_key(stage + pos, k[j]);
             stage_bin[pos] = (uint16_t)l;
-        } else if (k[j] != EMPTY) {  // far window: one key at a time
+        } else if (!key_empty(k[j])) {  // far window: one key at a time
             const uint32_t w = general_window(k[j], j);
             const unsigned long long g = atomicAdd(&a.win_cursor[w], 1ull);
             if (g < a.win_end[w]) {
-                a.out[g] = k[j];
+                put_key(out + g, k[j]);
             } else {
                 const unsigned long long sp = atomicAdd(a.spill_cursor, 1ull);
-                if (sp < a.spill_end) a.out[sp] = k[j];
+                if (sp < a.spill_end) put_key(out + sp, k[j]);
                 else atomicOr(a.spill_full, 1u);
             }
         }
@@ -401,18 +453,18 @@ __global__ void __launch_bounds__(SCAT_THREADS, 3) subroute_scatter(ScatterArgs 
     __syncthreads();
     for (uint32_t i = tid; i < staged; i += SCAT_THREADS) {
         const uint32_t l = stage_bin[i];
-        const uint64_t key = stage[i];
+        const K key = load_key(stage + i);
         if (i < limit[l]) {
-            a.out[gdelta[l] + i] = key;
+            put_key(out + gdelta[l] + i, key);
         } else {
             const uint64_t sp = sdelta[l] + i;
-            if (sp < a.spill_end) a.out[sp] = key;
+            if (sp < a.spill_end) put_key(out + sp, key);
         }
     }
 }
 
 struct WindowArgs {
-    uint64_t* keys;                  // window-grouped keys (subroute_scatter's output)
+    void* keys;                      // window-grouped keys (subroute_scatter's output)
     const uint64_t* win_start;       // first key of each window (multiple of WIN_SEG)
     const unsigned long long* win_fill;  // place after the last key the scatter put there
     const uint32_t* win_cap;         // capacity (multiple of WIN_SEG) of each window
@@ -421,7 +473,7 @@ struct WindowArgs {
     uint32_t order_base;             // this launch's first entry of `order`
     const BucketWin* bw;
     const BucketMeta* meta;
-    Slot1* table;                    // filter words in the cells' pad fields
+    void* table;                     // filter words in the cells' pad fields
     uint32_t* seg_low;               // per 64-key segment, as count_routed
     uint32_t* seg_fail;
     uint32_t* bucket_overflow;
@@ -448,10 +500,16 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // EMPTY: no initialisation pass and hardly a cell read.  Half-size genome
 // shape (299 M cells): count 7.67 -> 7.31 ms, and the extraction that the
 // initialisation (1.6 ms) ran beside 7.58 -> 7.05.
-__global__ void __launch_bounds__(WIN_THREADS, 3) count_window(WindowArgs a) {
+template <int NW>
+__global__ void __launch_bounds__(Win<NW>::THREADS, Win<NW>::CTAS) count_window(WindowArgs a) {
+    using K = typename KeyOf<NW>::T;
+    using S = typename SlotOf<NW>::T;
+    constexpr int WIN_Z = Win<NW>::Z, WIN_CELLS = Win<NW>::CELLS, WIN_THREADS = Win<NW>::THREADS;
+    K* const keys = static_cast<K*>(a.keys);
     extern __shared__ __align__(16) uint8_t win_smem[];
     unsigned long long* s_key = reinterpret_cast<unsigned long long*>(win_smem);
-    uint32_t* s_cnt = reinterpret_cast<uint32_t*>(win_smem + (size_t)WIN_CELLS * 8);
+    unsigned long long* s_key1 = s_key + WIN_CELLS;  // 128-bit keys: their second words
+    uint32_t* s_cnt = reinterpret_cast<uint32_t*>(win_smem + (size_t)WIN_CELLS * 8 * NW);
     uint32_t* s_pad = s_cnt + WIN_CELLS;
     __shared__ uint32_t s_full;  // a key of this window has met a full probe window
     if (threadIdx.x == 0) s_full = 0;
@@ -473,7 +531,7 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) count_window(WindowArgs a) {
     }
     if (cnt == 0 && !a.fresh) return;  // block-uniform; the window's cells are left as they are
     const uint64_t M = a.meta[wi.bucket].tab_mask;
-    Slot1* tab = a.table + a.meta[wi.bucket].tab_off;
+    S* tab = static_cast<S*>(a.table) + a.meta[wi.bucket].tab_off;
     const uint64_t base = single ? 0 : ((uint64_t)wi.sub << bw.zshift);
     const uint32_t W = single ? (uint32_t)(M + 1) : (uint32_t)WIN_CELLS;
 
@@ -483,14 +541,15 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) count_window(WindowArgs a) {
     // a warp's keys of segment group g (EMPTY past the window's keys); the
     // loads of the next group are issued before the current one is counted,
     // the first group's before the window's cells are staged
-    auto load_group = [&](uint32_t g, uint64_t (&dst)[ITEMS]) {
+    auto load_group = [&](uint32_t g, K (&dst)[ITEMS]) {
 #pragma unroll
         for (int j = 0; j < ITEMS; ++j) {
             const uint32_t idx = (g + j / 2) * WIN_SEG + (j & 1) * 32 + lane;
-            dst[j] = (g < nseg && idx < cnt) ? __ldcs(a.keys + k0 + idx) : EMPTY;
+            dst[j] = empty_key<NW>();
+            if (g < nseg && idx < cnt) dst[j] = stream_key(keys + k0 + idx);
         }
     };
-    uint64_t nxt[ITEMS];
+    K nxt[ITEMS];
     load_group((uint32_t)warp * WIN_GROUP, nxt);
 
     // stage the window (wrapping at the table's end: the last window's
@@ -501,12 +560,19 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) count_window(WindowArgs a) {
     const uint32_t lead = a.fresh ? (a.phase ? (uint32_t)WIN_HALO : 0u) : W;
     for (uint32_t i = threadIdx.x; i < W; i += WIN_THREADS) {
         if (i < lead || (a.fresh && a.phase && i >= (uint32_t)WIN_Z)) {
-            const Slot1* src = tab + ((base + i) & M);
-            cp_async8(&s_key[i], &src->key);
+            const S* src = tab + ((base + i) & M);
+            if constexpr (NW == 1) {
+                cp_async8(&s_key[i], &src->key);
+                cp_async4(&s_pad[i], &src->pad);
+            } else {
+                cp_async8(&s_key[i], &src->w0);
+                cp_async8(&s_key1[i], &src->w1);
+                cp_async4(&s_pad[i], &src->pad[0]);
+            }
             cp_async4(&s_cnt[i], &src->count);
-            cp_async4(&s_pad[i], &src->pad);
         } else {
             s_key[i] = EMPTY;
+            if (NW == 2) s_key1[i] = EMPTY;
             s_cnt[i] = 0;
             s_pad[i] = 0;
         }
@@ -517,7 +583,7 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) count_window(WindowArgs a) {
     const uint32_t lt = (1u << lane) - 1u;
     const uint32_t limit = (uint32_t)min((uint64_t)PROBE_LIMIT, M + 1);
     for (uint32_t g = (uint32_t)warp * WIN_GROUP; g < nseg; g += GSTEP) {
-        uint64_t it[ITEMS];
+        K it[ITEMS];
         uint32_t mult[ITEMS];
 #pragma unroll
         for (int j = 0; j < ITEMS; ++j) {
@@ -531,11 +597,21 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) count_window(WindowArgs a) {
         // shared-memory atomics of a run are one per distinct key
 #pragma unroll
         for (int j = 0; j < ITEMS; ++j) {
-            const uint64_t nx = __shfl_down_sync(0xffffffffu, it[j], 1);
-            if (!__any_sync(0xffffffffu, nx == it[j] && lane < 31 && mult[j] != 0)) continue;
+            bool eq_next;
+            if constexpr (NW == 1) {
+                const uint64_t nx = __shfl_down_sync(0xffffffffu, it[j], 1);
+                eq_next = nx == it[j];
+            } else {
+                const uint64_t n0 = __shfl_down_sync(0xffffffffu, it[j].w0, 1);
+                const uint64_t n1 = __shfl_down_sync(0xffffffffu, it[j].w1, 1);
+                eq_next = n0 == it[j].w0 && n1 == it[j].w1;
+            }
+            if (!__any_sync(0xffffffffu, eq_next && lane < 31 && mult[j] != 0)) continue;
             const uint32_t active = __ballot_sync(0xffffffffu, mult[j] != 0);
             if (mult[j]) {
-                const uint32_t same = __match_any_sync(active, it[j]);
+                uint32_t same;
+                if constexpr (NW == 1) same = __match_any_sync(active, it[j]);
+                else same = __match_any_sync(active, it[j].w0) & __match_any_sync(active, it[j].w1);
                 mult[j] = ((__ffs(same) - 1) == lane) ? (uint32_t)__popc(same) : 0u;
             }
         }
@@ -557,15 +633,39 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) count_window(WindowArgs a) {
             for (uint32_t p = 0; p < limit; ++p) {
                 if (p && p % PROBE_CHECK == 0 && *reinterpret_cast<volatile uint32_t*>(&s_full)) break;
                 const uint32_t c = single ? (uint32_t)((local + p) & M) : local + p;
-                unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&s_key[c]);
-                if (cur == EMPTY) {
-                    cur = atomicCAS(&s_key[c], EMPTY, (unsigned long long)it[j]);
-                    if (cur == EMPTY) cur = it[j];
-                }
-                if (cur == it[j]) {
-                    atomicAdd(&s_cnt[c], reps);
-                    done = true;
-                    break;
+                if constexpr (NW == 1) {
+                    unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&s_key[c]);
+                    if (cur == EMPTY) {
+                        cur = atomicCAS(&s_key[c], EMPTY, (unsigned long long)it[j]);
+                        if (cur == EMPTY) cur = it[j];
+                    }
+                    if (cur == it[j]) {
+                        atomicAdd(&s_cnt[c], reps);
+                        done = true;
+                        break;
+                    }
+                } else {
+                    // a cell is claimed word by word: the first word decides
+                    // who may claim the second, the second whose cell it is;
+                    // a key that loses the second goes on to the next cell
+                    // (neither word of a key of k <= 63 is EMPTY)
+                    unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&s_key[c]);
+                    if (cur == EMPTY) {
+                        cur = atomicCAS(&s_key[c], EMPTY, (unsigned long long)it[j].w0);
+                        if (cur == EMPTY) cur = it[j].w0;
+                    }
+                    if (cur == it[j].w0) {
+                        cur = *reinterpret_cast<volatile unsigned long long*>(&s_key1[c]);
+                        if (cur == EMPTY) {
+                            cur = atomicCAS(&s_key1[c], EMPTY, (unsigned long long)it[j].w1);
+                            if (cur == EMPTY) cur = it[j].w1;
+                        }
+                        if (cur == it[j].w1) {
+                            atomicAdd(&s_cnt[c], reps);
+                            done = true;
+                            break;
+                        }
+                    }
                 }
             }
             if (!done) {
@@ -590,7 +690,7 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) count_window(WindowArgs a) {
                 const int j = 2 * s + q;
                 const bool first = (first_bits >> j) & 1u;
                 const uint32_t lm = __ballot_sync(0xffffffffu, first);
-                if (first) a.keys[s0 + n_low + __popc(lm & lt)] = it[j];
+                if (first) put_key(keys + s0 + n_low + __popc(lm & lt), it[j]);
                 n_low += __popc(lm);
             }
             if (__any_sync(0xffffffffu, ((fail_bits >> (2 * s)) & 3u) != 0)) {
@@ -606,7 +706,7 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) count_window(WindowArgs a) {
                     }
                     const uint32_t wtot = __shfl_sync(0xffffffffu, fsum, 31);
                     const uint32_t my0 = n_fail + fsum - f;
-                    for (uint32_t rr = 0; rr < f; ++rr) a.keys[s_end - 1 - (my0 + rr)] = it[j];
+                    for (uint32_t rr = 0; rr < f; ++rr) put_key(keys + s_end - 1 - (my0 + rr), it[j]);
                     n_fail += wtot;
                 }
             }
@@ -618,12 +718,21 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) count_window(WindowArgs a) {
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < W; i += WIN_THREADS) {
-        const ulonglong2 v = make_ulonglong2(s_key[i], (uint64_t)s_cnt[i] | ((uint64_t)s_pad[i] << 32));
-        __stcg(reinterpret_cast<ulonglong2*>(tab + ((base + i) & M)), v);
+        ulonglong2* cell = reinterpret_cast<ulonglong2*>(tab + ((base + i) & M));
+        const uint64_t cp = (uint64_t)s_cnt[i] | ((uint64_t)s_pad[i] << 32);
+        if constexpr (NW == 1) {
+            __stcg(cell, make_ulonglong2(s_key[i], cp));
+        } else {
+            __stcg(cell, make_ulonglong2(s_key[i], s_key1[i]));
+            __stcg(cell + 1, make_ulonglong2(cp, 0));
+        }
     }
 }
 
-constexpr size_t window_smem_bytes() { return (size_t)WIN_CELLS * 16; }
+template <int NW>
+constexpr size_t window_smem_bytes() {
+    return (size_t)Win<NW>::CELLS * Win<NW>::CELL_BYTES;
+}
 
 // ------------------------------------------------------ merged histogram
 //
@@ -649,26 +758,40 @@ struct HistWindowArgs {
     const WinInfo* wins;
     const BucketWin* bw;
     const BucketMeta* meta;
-    const Slot1* table;
+    const void* table;
     uint32_t k, lo, hi;
     unsigned long long* gh;
     unsigned long long* extra;   // += table keys - low.bin keys found
 };
 
+__device__ __forceinline__ uint64_t cell_key(const Slot1& c) { return c.key; }
+__device__ __forceinline__ Key2 cell_key(const Slot2& c) { return Key2{c.w0, c.w1}; }
+__device__ __forceinline__ uint32_t& mark_of(Slot1& c) { return c.pad; }
+__device__ __forceinline__ uint32_t& mark_of(Slot2& c) { return c.pad[0]; }
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 
-__global__ void __launch_bounds__(WIN_THREADS, 3) hist_window(HistWindowArgs a) {
+// dynamic shared memory of hist_window: whole cells
+template <int NW>
+constexpr size_t hist_window_smem() {
+    return (size_t)Win<NW>::CELLS * sizeof(typename SlotOf<NW>::T);
+}
+
+template <int NW>
+__global__ void __launch_bounds__(WIN_THREADS, Win<NW>::HIST_CTAS) hist_window(HistWindowArgs a) {
+    using K = typename KeyOf<NW>::T;
+    using S = typename SlotOf<NW>::T;
+    constexpr int WIN_Z = Win<NW>::Z, WIN_CELLS = Win<NW>::CELLS;
     extern __shared__ __align__(16) uint8_t win_smem[];
-    Slot1* s_cell = reinterpret_cast<Slot1*>(win_smem);
+    S* s_cell = reinterpret_cast<S*>(win_smem);
     __shared__ uint32_t sh[HIST_SMEM];
     __shared__ unsigned long long s_extra;
     for (int i = threadIdx.x; i < HIST_SMEM; i += WIN_THREADS) sh[i] = 0;
     if (threadIdx.x == 0) s_extra = 0;
     const uint32_t full = a.k / 32, tail_bytes = (2 * (a.k % 32) + 7) / 8, P = full * 8 + tail_bytes;
-    constexpr int IT = 4;  // low.bin keys a thread holds at once
+    constexpr int IT = 4 / NW;  // low.bin keys a thread holds at once
     long long extra = 0;
     uint32_t alone = 0;  // low.bin keys no table holds
     for (uint64_t r = blockIdx.x; r < a.n_wins; r += gridDim.x) {
@@ -676,47 +799,51 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) hist_window(HistWindowArgs a) 
         const BucketWin bw = a.bw[wi.bucket];
         const bool single = bw.zshift >= WIN_SINGLE;
         const uint64_t M = a.meta[wi.bucket].tab_mask;
-        const Slot1* tab = a.table + a.meta[wi.bucket].tab_off;
+        const S* tab = static_cast<const S*>(a.table) + a.meta[wi.bucket].tab_off;
         const uint64_t base = single ? 0 : ((uint64_t)wi.sub << bw.zshift);
         const uint32_t own = single ? (uint32_t)(M + 1) : (uint32_t)WIN_Z;
         const uint32_t W = single ? own : (uint32_t)WIN_CELLS;
-        for (uint32_t i = threadIdx.x; i < W; i += WIN_THREADS) cp_async16(&s_cell[i], tab + ((base + i) & M));
+        for (uint32_t i = threadIdx.x; i < W; i += WIN_THREADS) {
+            const S* src = tab + ((base + i) & M);
+            cp_async16(&s_cell[i], src);
+            if constexpr (NW == 2) cp_async16(reinterpret_cast<uint4*>(&s_cell[i]) + 1, reinterpret_cast<const uint4*>(src) + 1);
+        }
         const uint64_t l0 = low_at(a.prefix, a.nsegs, a.win_start[r] / WIN_SEG, a.n_low);
         const uint64_t l1 = low_at(a.prefix, a.nsegs, r + 1 < a.n_wins ? a.win_start[r + 1] / WIN_SEG : a.spill_seg,
                                    a.n_low);
         cp_async_wait_all();
         __syncthreads();
         // the pad field (the count's filter bits) becomes the cell's mark
-        for (uint32_t i = threadIdx.x; i < own; i += WIN_THREADS) s_cell[i].pad = 0;
+        for (uint32_t i = threadIdx.x; i < own; i += WIN_THREADS) mark_of(s_cell[i]) = 0;
         __syncthreads();
         const uint32_t limit = (uint32_t)min((uint64_t)PROBE_LIMIT, M + 1);
         for (uint64_t i0 = l0; i0 < l1; i0 += IT * WIN_THREADS) {
-            uint64_t key[IT];
+            K key[IT];
 #pragma unroll
             for (int j = 0; j < IT; ++j) {
                 const uint64_t i = i0 + j * WIN_THREADS + threadIdx.x;
-                key[j] = EMPTY;
-                if (i < l1) key[j] = load_low<1>(a.low, i, P, full, tail_bytes);
+                key[j] = empty_key<NW>();
+                if (i < l1) key[j] = load_low<NW>(a.low, i, P, full, tail_bytes);
             }
 #pragma unroll
             for (int j = 0; j < IT; ++j) {
-                if (key[j] == EMPTY) continue;
+                if (key_empty(key[j])) continue;
                 const uint64_t local64 = ((hash_key(key[j]) >> 17) & M) - base;
                 if (local64 >= own) continue;  // never: the window's own low.bin records
                 const uint32_t local = (uint32_t)local64;
                 uint32_t c = local;
-                uint64_t cur = s_cell[c].key;
-                for (uint32_t p = 1; p < limit && cur != key[j] && cur != EMPTY; ++p) {
+                K cur = cell_key(s_cell[c]);
+                for (uint32_t p = 1; p < limit && !same_key(cur, key[j]) && !key_empty(cur); ++p) {
                     c = single ? (uint32_t)((local + p) & M) : local + p;
-                    cur = s_cell[c].key;
+                    cur = cell_key(s_cell[c]);
                 }
-                if (cur != key[j]) {
+                if (!same_key(cur, key[j])) {
                     ++alone;
                     continue;
                 }
                 --extra;
                 if (c < own) {
-                    s_cell[c].pad = 1;
+                    mark_of(s_cell[c]) = 1;
                 } else {
                     const uint32_t n = s_cell[c].count;
                     hist_add(sh, a.gh, n, -1, a.lo, a.hi);
@@ -726,10 +853,9 @@ __global__ void __launch_bounds__(WIN_THREADS, 3) hist_window(HistWindowArgs a) 
         }
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < own; i += WIN_THREADS) {
-            const Slot1 c = s_cell[i];
-            if (c.key == EMPTY) continue;
+            if (key_empty(cell_key(s_cell[i]))) continue;
             ++extra;
-            hist_add(sh, a.gh, (uint64_t)c.count + c.pad, 1, a.lo, a.hi);
+            hist_add(sh, a.gh, (uint64_t)s_cell[i].count + mark_of(s_cell[i]), 1, a.lo, a.hi);
         }
         __syncthreads();  // the cells are overwritten by the next window's
     }
