@@ -556,12 +556,19 @@ bool windows2_fit(const kc_context* c, uint64_t slots, uint64_t keys, double sca
     return want <= (double)free_bytes + held - (double)total / 16;
 }
 
-// The global count of 128-bit keys comes in two forms.
+// The global count of 128- and 256-bit keys comes in two forms (halves: every
+// k <= 127).
 template <int NW>
-void count_routed(const kc_context* c, const kc::CountArgs& a, uint64_t tiles) {
+void count_routed(const kc_context* c, const kc::CountArgs& a, uint64_t tiles, bool halves) {
     if constexpr (NW == 2) {
         if (c->cells2) {
             kc::count_routed<2, true><<<tiles, kc::CNT_THREADS, 0, c->stream>>>(a);
+            return;
+        }
+    }
+    if constexpr (NW == 4) {
+        if (halves) {
+            kc::count_routed<4, false, true><<<tiles, kc::CNT_THREADS, 0, c->stream>>>(a);
             return;
         }
     }
@@ -705,7 +712,7 @@ int launch_count(kc_context* c, uint64_t n_keys, int use_filter) {
     a.use_filter = use_filter;
     a.filter_in_table = c->nw == 1;
     Stage st(c, use_filter ? KC_STAGE_COUNT_ROUTED : KC_STAGE_REHASH);
-    count_routed<NW>(c, a, tiles);
+    count_routed<NW>(c, a, tiles, c->cfg.k <= 127);
     CK(cudaGetLastError());
     return KC_OK;
 }
@@ -856,7 +863,7 @@ int launch_count_range(kc_context* c, uint64_t off, uint64_t n, int use_filter) 
     a.use_filter = use_filter;
     a.filter_in_table = c->nw == 1;
     Stage st(c, KC_STAGE_COUNT_ROUTED);
-    count_routed<NW>(c, a, tiles);
+    count_routed<NW>(c, a, tiles, c->cfg.k <= 127);
     CK(cudaGetLastError());
     return KC_OK;
 }
@@ -2659,6 +2666,7 @@ route_again:
     c->K = K;
     c->bloom_words = NW == 1 ? ts / 2 : bw;
     c->table_slots_used = ts;
+    c->cells2 = false;
     CK(c->bloom.ensure(bw * sizeof(uint64_t)));
     CK(c->table.ensure(ts * c->slot_bytes + ts * c->slot_bytes / 4));  // room for a few in-place growths
     CK(c->meta.ensure(nbk * sizeof(kc::BucketMeta)));
@@ -2741,6 +2749,7 @@ route_again:
     ca.set_buckets = NB;
     ca.use_filter = 1;
     ca.filter_in_table = NW == 1;
+    const bool halves = std::all_of(sets, sets + n_sets, [](const kc_set_desc& q) { return q.k <= 127; });
     ca.error = c->scalars.as<uint32_t>() + 13;
     uint64_t cgrid = ceil_div(n_keys, (uint64_t)CT * kc::CNT_SEGS_PER_WARP);
 
@@ -2764,7 +2773,7 @@ route_again:
                 c->region_end.as<unsigned long long>(), (uint32_t)nbk);
         // and after each set's keys (its overflow area's unused part, the alignment gap)
         kc::fill_set_gaps<NW><<<n_sets, 256, 0, c->stream>>>(c->routed.p, d_ovc, d_next, n_sets);
-        if (cgrid && !windowed) kc::count_routed<NW><<<cgrid, kc::CNT_THREADS, 0, c->stream>>>(ca);
+        if (cgrid && !windowed) count_routed<NW>(c, ca, cgrid, halves);
         const cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
         if (ce != cudaSuccess) return fail(KC_ERR_DEVICE, "graph capture failed: %s", cudaGetErrorString(ce));
         cudaError_t e = cudaSuccess;
@@ -2858,7 +2867,7 @@ route_again:
         ca.table = c->table.p;
         ca.use_filter = 0;
         Stage st(c, KC_STAGE_REHASH);
-        if (cgrid) kc::count_routed<NW><<<cgrid, kc::CNT_THREADS, 0, c->stream>>>(ca);
+        if (cgrid) count_routed<NW>(c, ca, cgrid, halves);
         CK(cudaGetLastError());
     }
 

@@ -133,10 +133,13 @@ struct __align__(16) Slot1 {
     uint32_t count;
     uint32_t pad;
 };
-// 256-bit keys have no CAS of their width: a slot is claimed by a CAS of
-// `state` (SLOT_EMPTY -> SLOT_WRITING); the owner writes the key and the first
-// count and publishes them with a release of state = SLOT_READY.  A thread
-// that meets a SLOT_WRITING slot waits for it (bounded) before comparing.
+// 256-bit keys have no CAS of their width.  For k <= 127 the count claims a
+// slot half by half (table_add4_halves).  At k = 128 a half can be all ones,
+// and a slot is claimed by a CAS of `state` (SLOT_EMPTY -> SLOT_WRITING): the
+// owner writes the key and the first count and publishes them with a release
+// of state = SLOT_READY.  A thread that meets a SLOT_WRITING slot waits for it
+// (bounded) before comparing.  Either way a used slot is SLOT_READY at the
+// kernel's end, and an unused one has EMPTY words.
 constexpr uint32_t SLOT_EMPTY = 0, SLOT_WRITING = 1, SLOT_READY = 2;
 constexpr uint32_t PUBLISH_WAIT_LIMIT = 1u << 22;  // polls before a wait counts as a device error
 struct __align__(16) Slot4 {
@@ -1039,6 +1042,25 @@ __device__ __forceinline__ uint32_t bloom_bits32(uint64_t h) {
     return (1u << (h & 31)) | (1u << ((h >> 5) & 31)) | (1u << ((h >> 10) & 31));
 }
 
+// Whether a cell reads empty (a 16-byte read may be torn while the cell is
+// claimed: any EMPTY word counts as empty and is settled by the CAS), and
+// whether it holds the key.
+__device__ __forceinline__ bool cell_empty(uint64_t v) { return v == EMPTY; }
+__device__ __forceinline__ bool cell_empty(const ulonglong2& v) { return v.x == EMPTY || v.y == EMPTY; }
+__device__ __forceinline__ bool cell_holds(uint64_t v, uint64_t key) { return v == key; }
+__device__ __forceinline__ bool cell_holds(const ulonglong2& v, const Key2& key) {
+    return v.x == key.w0 && v.y == key.w1;
+}
+// Claim a 16-byte cell (or half of one) that read empty: its value after the
+// CAS (the key's own when this thread claimed it).
+__device__ __forceinline__ ulonglong2 claim16(void* s, const Key2& key) {
+    const unsigned __int128 e = ~(unsigned __int128)0;
+    const unsigned __int128 kv = ((unsigned __int128)key.w1 << 64) | key.w0;
+    const unsigned __int128 old = atomicCAS(reinterpret_cast<unsigned __int128*>(s), e, kv);
+    const unsigned __int128 now = old == e ? kv : old;
+    return make_ulonglong2((uint64_t)now, (uint64_t)(now >> 64));
+}
+
 // Insert `add` occurrences of key into a bucket table starting at slot
 // (h >> 17) & mask; false = probe limit hit.  Linear probing; a slot goes
 // EMPTY -> key exactly once (CAS), counts only grow (atomicAdd).
@@ -1146,6 +1168,39 @@ static __device__ __noinline__ int table_add4(Slot4* __restrict__ tab, uint64_t 
     return 0;
 }
 
+// The same for k <= 127, where neither 16-byte half of a canonical key is all
+// ones (its first half would take 64 T in one orientation and 64 A in the
+// other, its last ends in unused zero bits): a slot is claimed half by half,
+// each with one 16-byte CAS.  The first half decides who may claim the second,
+// the second whose slot it is; a key that loses the second goes on to the next
+// slot.  No fence and no wait, of which the published state cost every warp
+// several in turn: 136 M keys of k = 101 counted in 3.74 ms, 6.59 before (the
+// table cell read beside the filter word as for shorter keys: no gain).
+// false = probe limit hit, or `overflowed` says that the bucket has.
+__device__ __forceinline__ bool table_add4_halves(Slot4* __restrict__ tab, uint64_t mask, uint64_t h, const Key4& key,
+                                                  uint32_t add, const uint32_t* overflowed) {
+    const uint64_t i = (h >> 17) & mask;
+    const uint32_t limit = (uint32_t)min((uint64_t)PROBE_LIMIT, mask + 1);
+    const Key2 k0{key.w0, key.w1}, k1{key.w2, key.w3};
+    for (uint32_t p = 0; p < limit; ++p) {
+        if (p && p % PROBE_CHECK == 0 && __ldcg(overflowed)) return false;
+        Slot4* s = tab + ((i + p) & mask);
+        ulonglong2* halves = reinterpret_cast<ulonglong2*>(s);
+        ulonglong2 a = __ldcg(halves), b = __ldcg(halves + 1);
+        // (a half that shows an EMPTY word may be torn: the CAS tells)
+        if (cell_empty(a)) a = claim16(halves, k0);
+        if (!cell_holds(a, k0)) continue;
+        if (cell_empty(b)) {
+            b = claim16(halves + 1, k1);
+            if (cell_holds(b, k1)) s->state = SLOT_READY;  // (all that get here store the same)
+        }
+        if (!cell_holds(b, k1)) continue;
+        atomicAdd(&s->count, add);
+        return true;
+    }
+    return false;
+}
+
 // Full insert (used by the table rehash).
 __device__ __forceinline__ bool table_add(Slot1* tab, uint64_t mask, uint64_t h, uint64_t key, uint32_t add) {
     return table_add_slow(tab, mask, h, key, add, 0);
@@ -1158,16 +1213,8 @@ __device__ __forceinline__ bool table_add(Slot4* tab, uint64_t mask, uint64_t h,
 }
 
 // Probe-round helpers of count_routed (64- and 128-bit keys): a cell's key
-// as read (16-byte reads of a 128-bit cell may be torn while it is claimed:
-// any EMPTY half counts as empty and is settled by the CAS), the claim of a
-// cell read empty (returns the cell's key after the CAS: `key` when this
-// thread claimed it), and the match test.
-__device__ __forceinline__ bool cell_empty(uint64_t v) { return v == EMPTY; }
-__device__ __forceinline__ bool cell_empty(const ulonglong2& v) { return v.x == EMPTY || v.y == EMPTY; }
-__device__ __forceinline__ bool cell_holds(uint64_t v, uint64_t key) { return v == key; }
-__device__ __forceinline__ bool cell_holds(const ulonglong2& v, const Key2& key) {
-    return v.x == key.w0 && v.y == key.w1;
-}
+// as read, and the claim of a cell read empty (returns the cell's key after
+// the CAS: `key` when this thread claimed it).
 __device__ __forceinline__ uint64_t read_cell(const Slot1* s) { return __ldcg(&s->key); }
 __device__ __forceinline__ ulonglong2 read_cell(const Slot2* s) {
     return __ldcg(reinterpret_cast<const ulonglong2*>(s));
@@ -1176,13 +1223,7 @@ __device__ __forceinline__ uint64_t claim_cell(Slot1* s, uint64_t key) {
     const uint64_t old = atomicCAS(reinterpret_cast<unsigned long long*>(&s->key), EMPTY, key);
     return old == EMPTY ? key : old;
 }
-__device__ __forceinline__ ulonglong2 claim_cell(Slot2* s, const Key2& key) {
-    const unsigned __int128 e = ~(unsigned __int128)0;
-    const unsigned __int128 kv = ((unsigned __int128)key.w1 << 64) | key.w0;
-    const unsigned __int128 old = atomicCAS(reinterpret_cast<unsigned __int128*>(s), e, kv);
-    const unsigned __int128 now = old == e ? kv : old;
-    return make_ulonglong2((uint64_t)now, (uint64_t)(now >> 64));
-}
+__device__ __forceinline__ ulonglong2 claim_cell(Slot2* s, const Key2& key) { return claim16(s, key); }
 
 // Whether the n cells from index `at` on (mod mask + 1) are all taken, read
 // by the whole warp at once (all lanes pass the same arguments).
@@ -1219,9 +1260,9 @@ template <int NW>
 __host__ __device__ constexpr int count_items() {
     return NW == 1 ? 2 : (NW == 2 ? 2 : 1);
 }
-template <int NW>
+template <int NW, bool HALVES = false>
 __host__ __device__ constexpr int count_min_ctas() {
-    return NW == 1 ? 6 : (NW == 2 ? 4 : 4);
+    return NW == 1 ? 6 : (NW == 2 ? 4 : (HALVES ? 6 : 4));
 }
 // Keys owned by one warp of the count kernel (a contiguous segment).
 template <int NW>
@@ -1281,9 +1322,11 @@ constexpr int CNT_SEGS_PER_WARP = 8;
 // occurrences at the front, keys that met a full table at the back.
 // CELLS2: 128-bit keys whose filter words are fields of the table cells (a run
 // counted in windows; its spilled, retried and later keys come here).
-template <int NW, bool CELLS2 = false>
-__global__ void __launch_bounds__(CNT_THREADS, count_min_ctas<NW>()) count_routed(CountArgs a) {
+// HALVES: 256-bit keys of k <= 127 (table_add4_halves).
+template <int NW, bool CELLS2 = false, bool HALVES = false>
+__global__ void __launch_bounds__(CNT_THREADS, count_min_ctas<NW, HALVES>()) count_routed(CountArgs a) {
     static_assert(!CELLS2 || NW == 2, "128-bit keys only");
+    static_assert(!HALVES || NW == 4, "256-bit keys only");
     using K = typename KeyOf<NW>::T;
     using S = typename SlotOf<NW>::T;
     // first table slot read ahead of the filter result (not for 256-bit keys,
@@ -1477,7 +1520,10 @@ __global__ void __launch_bounds__(CNT_THREADS, count_min_ctas<NW>()) count_route
                 if (mult[j] && reps) {
                     const uint32_t b = set_bucket0 + (uint32_t)(key_hi(it[j]) >> a.bucket_shift);
                     const MetaS m = meta_of(b);
-                    const int r = table_add4(table + m.tab_off, m.tab_mask, h[j], it[j], reps, a.bucket_overflow + b);
+                    int r;
+                    if constexpr (HALVES)
+                        r = table_add4_halves(table + m.tab_off, m.tab_mask, h[j], it[j], reps, a.bucket_overflow + b);
+                    else r = table_add4(table + m.tab_off, m.tab_mask, h[j], it[j], reps, a.bucket_overflow + b);
                     if (r < 0) atomicOr(a.error, 1u);  // a slot was never published: reported, not retried
                     if (r == 0) {
                         fail_bits |= 1u << j;
@@ -1636,7 +1682,7 @@ __device__ __forceinline__ void init_slot(typename SlotOf<NW>::T& s) {
         s.count = 0;
         s.pad[0] = s.pad[1] = s.pad[2] = 0;
     } else {
-        s.w0 = s.w1 = s.w2 = s.w3 = 0;
+        s.w0 = s.w1 = s.w2 = s.w3 = EMPTY;
         s.count = 0;
         s.state = SLOT_EMPTY;
         s.mark = 0;
@@ -1697,7 +1743,8 @@ __global__ void init_slots(void* tab, uint64_t n) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += (uint64_t)gridDim.x * blockDim.x) {
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if constexpr (NW == 1) v = make_uint4(~0u, ~0u, 0u, 0u);           // {key = EMPTY, count, pad}
-        else if constexpr (NW == 2) if ((i & 1) == 0) v = make_uint4(~0u, ~0u, ~0u, ~0u);  // {w0, w1} = EMPTY
+        else if constexpr (NW == 2) { if ((i & 1) == 0) v = make_uint4(~0u, ~0u, ~0u, ~0u); }  // {w0, w1} = EMPTY
+        else if (i % 3 != 2) v = make_uint4(~0u, ~0u, ~0u, ~0u);                               // {w0..w3} = EMPTY
         t[i] = v;
     }
 }
