@@ -334,7 +334,8 @@ def stage_rooflines(stage_ms, stats, F, k, hbm_gbs, P, rec, traffic=None):
       count            8N K + 8N L + 2 x 16 x cells x 9/8
                                          (windowed count) every key read, first occurrences
                                          written back, every table cell (16 B: key, count,
-                                         filter word) and its window's halo read and written;
+                                         filter word) and its window's halo read and written
+                                         (128-bit keys: 32 B cells, 5/4 with the halo);
                        64 K + 64 (K - L) (global count, no windows) one 32 B filter sector read
                                          + write per k-mer and one table sector per repeat
       pack_low         8N L + P L        first occurrences read, packed low.bin written
@@ -349,10 +350,11 @@ def stage_rooflines(stage_ms, stats, F, k, hbm_gbs, P, rec, traffic=None):
     S = {1: 16, 2: 32, 4: 48}[nw]
     W = stats.get("filter_words", 0) if nw > 1 else 0  # 64-bit keys keep the filter in the cells
     windowed = stage_ms.get("subroute", 0.0) > 0
+    halo, halo_rule = (9 / 8, "9/8") if nw == 1 else (5 / 4, "5/4")  # 512 cells past a window of 4096, 2048
     rules = {
         "extract_scatter": (F + 8 * nw * K, "F + 8N K"),
         "subroute": (2 * 8 * nw * K, "2 x 8N K"),
-        "count": ((8 * nw * K + 8 * nw * L + int(2 * 16 * cells * 9 / 8), "8N K + 8N L + 2 x 16 x cells x 9/8")
+        "count": ((8 * nw * K + 8 * nw * L + int(2 * S * cells * halo), f"8N K + 8N L + 2 x {S} x cells x {halo_rule}")
                   if windowed else (64 * K + 64 * (K - L), "64 K + 64 (K - L)")),
         "pack_low": (8 * nw * L + P * L, "8N L + P L"),
         "export": (S * cells + rec * R, f"{S} cells + rec R"),

@@ -1134,7 +1134,7 @@ static __device__ __noinline__ int table_add4(Slot4* __restrict__ tab, uint64_t 
         // a READY slot is that slot's, whenever they were read (its words are
         // written once); one that does not may have been read too early and is
         // read again behind a fence.  A fence per probe and a second round trip
-        // made the count of 136 M keys 7.56 ms; 6.62 now.
+        // made the count of 136 M keys (k = 101, counted here) 7.56 ms, 6.62 so.
         uint32_t st = *state;
         Key4 have = cell_key4(s);
         if (st == SLOT_READY && same_key(have, key)) {
