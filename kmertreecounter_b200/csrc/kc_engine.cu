@@ -530,6 +530,30 @@ int init_now(kc_context* c) {
     return KC_OK;
 }
 
+// Whether the device has room for the buffers (kc_needs_fit).
+bool needs_fit(const KcNeed* v, int n) {
+    if (kc_needs_fit(v, n, -1e30)) return true;  // all held: no question to the driver
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return kc_needs_fit(v, n, (double)free_bytes);
+}
+
+// An allocation that comes after the windowed count: the keys' first buffer
+// (routed2 by then) holds nothing any more and is given back for it.
+template <class F>
+cudaError_t or_shed(kc_context* c, F alloc) {
+    cudaError_t e = alloc();
+    if (e == cudaErrorMemoryAllocation && c->routed2.p) {
+        cudaGetLastError();
+        c->routed2.release();
+        e = alloc();
+    }
+    return e;
+}
+
 // Whether the device has room for 128-bit keys counted in windows: `slots`
 // cells with their growth share, the keys and their sub-routed copy, and all
 // of the input's keys packed (the buffers that the context holds already
@@ -738,8 +762,10 @@ int grow_buckets(kc_context* c, const std::vector<uint32_t>& buckets) {
             total += new_slots[i];
             max_slots = std::max<uint64_t>(max_slots, new_slots[i]);
         }
-        CK(c->table.grow_keep((c->table_slots_used + total) * c->slot_bytes, c->table_slots_used * c->slot_bytes,
-                              c->stream));
+        CK(or_shed(c, [&] {
+            return c->table.grow_keep((c->table_slots_used + total) * c->slot_bytes,
+                                      c->table_slots_used * c->slot_bytes, c->stream);
+        }));
         std::vector<kc::GrowJob> jobs(todo.size());
         for (size_t j = 0; j < todo.size(); ++j) {
             const kc::BucketMeta& m = c->h_meta[buckets[todo[j]]];
@@ -1352,7 +1378,7 @@ int count_and_pack(kc_context* c, uint64_t n_keys, const void* src) {
         if (need > c->low_packed.cap && c->expected_total_bytes > c->input_bytes && c->input_bytes > 0)
             need = std::max<uint64_t>(need, (uint64_t)((double)need * 1.1 * (double)c->expected_total_bytes /
                                                        (double)c->input_bytes));
-        CK(c->low_packed.grow_keep(need, low_before * c->packed_bytes, c->stream));
+        CK(or_shed(c, [&] { return c->low_packed.grow_keep(need, low_before * c->packed_bytes, c->stream); }));
         low_dst = c->low_packed.as<uint8_t>();
         low_base = low_before;
     }
@@ -1440,7 +1466,7 @@ int run_export(kc_context* c, const std::vector<kc::ExportChunk>& ch, uint64_t n
         c->end_recorded = true;
         return KC_OK;
     }
-    CK(c->roots.ensure(std::max<uint64_t>(R, 1) * c->record_bytes));
+    CK(or_shed(c, [&] { return c->roots.ensure(std::max<uint64_t>(R, 1) * c->record_bytes); }));
     if (nch && R) CKR(write());
     return KC_OK;
 }
@@ -2612,15 +2638,8 @@ route_again:
     // layout: each set's routed region starts on a segment boundary
     std::vector<uint64_t> start(nbk), rend(nbk), set_key0(n_sets), set_key1(n_sets), set_next(n_sets), set_seg(n_sets);
     std::vector<uint64_t> ovf_start(n_sets), ovf_end(n_sets);
-    uint64_t pos = 0;
-    c->h_meta.assign(nbk, kc::BucketMeta{});
-    uint64_t bw = 0, ts = 0, K = 0;
-    // learned sizing (kc_set_predicted_set_rates) when predictions for these
-    // n_sets sets were handed over: predicted rates x the bucket's exact
-    // k-mer total, 12 filter bits per distinct key, table keys with 15%
-    // headroom at the target load; else (and for a negative rate) the sampled
-    // rule on the exact per-bucket k-mer totals
-    const bool learned = g.sizing == KC_SIZING_LEARNED && c->set_pred_table.size() == nbk;
+    std::vector<uint64_t> kmers(nbk);  // per bucket (estimated for a sampled set)
+    uint64_t pos = 0, K = 0, low_bound = 0;
     for (uint32_t s = 0; s < n_sets; ++s) {
         pos = ceil_div(pos, SEG) * SEG;
         set_key0[s] = pos;
@@ -2635,26 +2654,9 @@ route_again:
             pos += cap;
             rend[(uint64_t)s * NB + b] = pos;
             set_cap += cap;
+            kmers[(uint64_t)s * NB + b] = kb;
             K += kb;
-            uint64_t words, slots;
-            const uint64_t q = (uint64_t)s * NB + b;
-            if (learned && c->set_pred_distinct[q] >= 0.0 && c->set_pred_table[q] >= 0.0) {
-                const double d = std::min(c->set_pred_distinct[q], 1.0) * (double)kb;
-                const double t = std::min(c->set_pred_table[q], 1.0) * (double)kb;
-                words = pow2_at_least(std::max<uint64_t>((uint64_t)(d * 12.0 / 64.0), 64));
-                slots = pow2_at_least(std::max<uint64_t>((uint64_t)(t * 1.15 / g.table_load), 64));
-            } else {
-                words = pow2_at_least(std::max<uint64_t>((uint64_t)(kb * g.bloom_bits / 64.0), 64));
-                slots = pow2_at_least(std::max<uint64_t>((uint64_t)(kb * g.repeat_ratio / g.table_load), 64));
-            }
-            if (NW == 1) {  // the filter words are the cells' pad fields, as for one input
-                slots = std::max<uint64_t>(slots, 2 * words);
-                c->h_meta[q] = kc::BucketMeta{ts, slots - 1, ts, slots - 1};
-            } else {
-                c->h_meta[q] = kc::BucketMeta{bw, words - 1, ts, slots - 1};
-                bw += words;
-            }
-            ts += slots;
+            low_bound += kb * kc_packed_bytes(sets[s].k);
         }
         ovf_start[s] = pos;
         if (sampled[s]) pos += std::max<uint64_t>(1ull << 16, set_cap / 32);
@@ -2664,29 +2666,82 @@ route_again:
     uint64_t n_keys = ceil_div(pos, SEG) * SEG;
     for (uint32_t s = 0; s < n_sets; ++s) set_next[s] = (s + 1 < n_sets) ? set_key0[s + 1] : n_keys;
     c->K = K;
-    c->bloom_words = NW == 1 ? ts / 2 : bw;
-    c->table_slots_used = ts;
     c->cells2 = false;
+    // filter and tables by learned sizing (kc_set_predicted_set_rates) when
+    // predictions for these n_sets sets were handed over: predicted rates x the
+    // bucket's exact k-mer total, 12 filter bits per distinct key, table keys
+    // with 15% headroom at the target load; else (and for a negative rate) by
+    // the sampled rule on the exact per-bucket k-mer totals
+    const bool learned = g.sizing == KC_SIZING_LEARNED && c->set_pred_table.size() == nbk;
+    uint64_t bw = 0, ts = 0;
+    auto place = [&](bool in_cells) {
+        c->h_meta.assign(nbk, kc::BucketMeta{});
+        bw = ts = 0;
+        for (uint64_t q = 0; q < nbk; ++q) {
+            const uint64_t kb = kmers[q];
+            uint64_t words, slots;
+            if (learned && c->set_pred_distinct[q] >= 0.0 && c->set_pred_table[q] >= 0.0) {
+                const double d = std::min(c->set_pred_distinct[q], 1.0) * (double)kb;
+                const double t = std::min(c->set_pred_table[q], 1.0) * (double)kb;
+                words = pow2_at_least(std::max<uint64_t>((uint64_t)(d * 12.0 / 64.0), 64));
+                slots = pow2_at_least(std::max<uint64_t>((uint64_t)(t * 1.15 / g.table_load), 64));
+            } else {
+                words = pow2_at_least(std::max<uint64_t>((uint64_t)(kb * g.bloom_bits / 64.0), 64));
+                slots = pow2_at_least(std::max<uint64_t>((uint64_t)(kb * g.repeat_ratio / g.table_load), 64));
+            }
+            if (in_cells) {  // the filter words are the cells' pad fields, as for one input
+                slots = std::max<uint64_t>(slots, 2 * words);
+                c->h_meta[q] = kc::BucketMeta{ts, slots - 1, ts, slots - 1};
+            } else {
+                c->h_meta[q] = kc::BucketMeta{bw, words - 1, ts, slots - 1};
+                bw += words;
+            }
+            ts += slots;
+        }
+        c->table_slots_used = ts;
+    };
+    // 64-bit keys of a large pass are counted in windows (the rule for one
+    // input; SETS_WINDOW_KEYS keys pay for the extra launches and the exact
+    // window counts): 48 sets of 10k-300k reads, 543 M k-mers, 34.6 ms by the
+    // global count, 22.3 in windows.  That takes a second key buffer, and the
+    // filter in the cells may take more than an array of its own: where the
+    // pass does not fit the device so, it does without the one, then without
+    // the other, so that it is refused for memory no sooner.
+    bool in_cells = NW == 1;
+    place(in_cells);
+    auto fits = [&](bool second) {
+        const double kb = (double)n_keys * sizeof(KeyT);
+        const KcNeed need[5] = {
+            {(double)ts * c->slot_bytes * 1.25, (double)c->table.cap},
+            {kb, (double)c->routed.cap},
+            {(double)low_bound, (double)c->low_packed.cap},
+            {(double)std::min(ts, K) * c->record_bytes, (double)c->roots.cap},
+            {kb + (double)c->n_wins * kc::WIN_SEG * sizeof(KeyT), (double)c->routed2.cap},
+        };
+        return needs_fit(need, second ? 5 : 4);
+    };
+    bool windowed = in_cells && n_keys >= SETS_WINDOW_KEYS && windows_pay(c, n_keys) &&
+                    build_windows(c, (uint32_t)nbk) && fits(true);
+    if (!windowed && !fits(false)) {
+        c->routed2.release();  // an earlier count's
+        if (in_cells && !fits(false)) place(in_cells = false);
+    }
+    c->bloom_words = in_cells ? ts / 2 : bw;
     CK(c->bloom.ensure(bw * sizeof(uint64_t)));
     CK(c->table.ensure(ts * c->slot_bytes + ts * c->slot_bytes / 4));  // room for a few in-place growths
     CK(c->meta.ensure(nbk * sizeof(kc::BucketMeta)));
     CK(c->overflow.ensure(nbk * sizeof(uint32_t)));
-    // 64-bit keys of a large pass are counted in windows (the rule for one
-    // input; SETS_WINDOW_KEYS keys pay for the extra launches and the exact
-    // window counts) while the second key buffer fits the device: 48 sets of
-    // 10k-300k reads, 543 M k-mers, 34.6 ms by the global count, 22.3 in windows
-    bool windowed = NW == 1 && n_keys >= SETS_WINDOW_KEYS && windows_pay(c, n_keys) && build_windows(c, (uint32_t)nbk);
+    uint64_t nsegs = n_keys / SEG;
+    CK(c->routed.ensure(std::max<uint64_t>(ceil_div(n_keys, CT) * CT, 1) * sizeof(KeyT)));
+    CK(c->tile_low.ensure(std::max<uint64_t>(nsegs, 1) * sizeof(uint32_t)));
+    CK(c->tile_fail.ensure(std::max<uint64_t>(nsegs, 1) * sizeof(uint32_t)));
+    CK(c->tile_low_prefix.ensure(std::max<uint64_t>(nsegs, 1) * sizeof(uint64_t)));
     if (windowed && c->routed2.ensure((n_keys + c->n_wins * kc::WIN_SEG) * sizeof(KeyT)) != cudaSuccess) {
         cudaGetLastError();
         windowed = false;
     }
     c->win_ready = false;
     c->init_deferred = windowed;
-    uint64_t nsegs = n_keys / SEG;
-    CK(c->routed.ensure(std::max<uint64_t>(ceil_div(n_keys, CT) * CT, 1) * sizeof(KeyT)));
-    CK(c->tile_low.ensure(std::max<uint64_t>(nsegs, 1) * sizeof(uint32_t)));
-    CK(c->tile_fail.ensure(std::max<uint64_t>(nsegs, 1) * sizeof(uint32_t)));
-    CK(c->tile_low_prefix.ensure(std::max<uint64_t>(nsegs, 1) * sizeof(uint64_t)));
     CK(c->set_info.ensure((size_t)n_sets * 10 * sizeof(uint64_t) + 64));
     uint64_t* d_key0 = c->set_info.as<uint64_t>();             // windows: set_key0[n_sets]
     uint64_t* d_seg = d_key0 + n_sets;                         // set_seg_start[n_sets]
@@ -2748,7 +2803,7 @@ route_again:
     ca.n_sets = n_sets;
     ca.set_buckets = NB;
     ca.use_filter = 1;
-    ca.filter_in_table = NW == 1;
+    ca.filter_in_table = in_cells;
     const bool halves = std::all_of(sets, sets + n_sets, [](const kc_set_desc& q) { return q.k <= 127; });
     ca.error = c->scalars.as<uint32_t>() + 13;
     uint64_t cgrid = ceil_div(n_keys, (uint64_t)CT * kc::CNT_SEGS_PER_WARP);
@@ -2894,7 +2949,7 @@ route_again:
         lb += lows[s] * kc_packed_bytes(sets[s].k);
     }
     CK(cudaMemcpyAsync(d_lowbase, lowbase.data(), n_sets * sizeof(uint64_t), cudaMemcpyHostToDevice, c->stream));
-    CK(c->low_packed.ensure(lb + 64));
+    CK(or_shed(c, [&] { return c->low_packed.ensure(lb + 64); }));
     if (nsegs) {
         Stage st(c, KC_STAGE_PACK_LOW);
         kc::pack_low_sets<NW><<<std::min<uint64_t>(ceil_div(nsegs, 8 * 32), (uint64_t)c->sm_count * 16), 256, 0,

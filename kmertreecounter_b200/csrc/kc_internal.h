@@ -28,6 +28,25 @@ const char* kc_sort_error();
 // kc_sort_scratch_bytes with record_bytes = 8 nw).
 int kc_sort_keys(void* keys, uint64_t n, uint32_t nw, uint32_t k, const KcSortScratch& w, cudaStream_t stream);
 
+// A device buffer that a run still needs (bytes) and what it holds already.
+struct KcNeed {
+    double bytes, held;
+};
+// Whether the buffers that have to grow find room in `free_bytes` of device
+// memory: each is given back before it is allocated anew, with an eighth to
+// spare; 64 MiB stay for the small arrays.
+inline bool kc_needs_fit(const KcNeed* v, int n, double free_bytes) {
+    double want = 0;
+    bool grow = false;
+    for (int i = 0; i < n; ++i)
+        if (v[i].bytes > v[i].held) {
+            want += v[i].bytes * 9 / 8;
+            free_bytes += v[i].held;
+            grow = true;
+        }
+    return !grow || want + (64 << 20) <= free_bytes;
+}
+
 int kc_internal_set_error(int code, const char* msg);
 uint64_t kc_internal_record_bytes(const kc_context* c);
 uint32_t kc_internal_k(const kc_context* c);
