@@ -1109,8 +1109,15 @@ static __device__ __noinline__ bool table_add_slow(Slot2* __restrict__ tab, uint
 
 __device__ __forceinline__ bool same_key(uint64_t a, uint64_t b) { return a == b; }
 __device__ __forceinline__ bool same_key(const Key2& a, const Key2& b) { return a.w0 == b.w0 && a.w1 == b.w1; }
-__device__ __forceinline__ bool same_key(const Key4& a, const Key4& b) {
+KC_HD bool same_key(const Key4& a, const Key4& b) {
     return a.w0 == b.w0 && a.w1 == b.w1 && a.w2 == b.w2 && a.w3 == b.w3;
+}
+// Whether a slot read without a fence while its key may be arriving holds
+// `key`: every word was EMPTY before it was written, once, so a read that
+// agrees in all words holds no unwritten one, unless the key itself has a word
+// of all ones (32 T's in its place).
+KC_HD bool holds_unfenced(const Key4& have, const Key4& key) {
+    return same_key(have, key) && key.w0 != EMPTY && key.w1 != EMPTY && key.w2 != EMPTY && key.w3 != EMPTY;
 }
 __device__ __forceinline__ Key4 cell_key4(const Slot4* s) {
     const ulonglong2 a = __ldcg(reinterpret_cast<const ulonglong2*>(s));
@@ -1130,14 +1137,15 @@ static __device__ __noinline__ int table_add4(Slot4* __restrict__ tab, uint64_t 
         if (p && p % PROBE_CHECK == 0 && overflowed && __ldcg(overflowed)) return 0;
         Slot4* s = tab + ((i + p) & mask);
         volatile uint32_t* state = &s->state;
-        // state and key in one round trip.  A key that agrees in all words of
-        // a READY slot is that slot's, whenever they were read (its words are
-        // written once); one that does not may have been read too early and is
-        // read again behind a fence.  A fence per probe and a second round trip
-        // made the count of 136 M keys (k = 101, counted here) 7.56 ms, 6.62 so.
+        // state and key in one round trip, with nothing that orders the two:
+        // the key words of a READY slot may still be the unwritten ones.  A
+        // match that cannot mix the two counts (holds_unfenced); anything else
+        // is read again behind a fence.  A fence per probe and a second round
+        // trip made the count of 136 M keys (k = 101, counted here) 7.56 ms,
+        // 6.62 so.
         uint32_t st = *state;
         Key4 have = cell_key4(s);
-        if (st == SLOT_READY && same_key(have, key)) {
+        if (st == SLOT_READY && holds_unfenced(have, key)) {
             atomicAdd(&s->count, add);
             return 1;
         }
