@@ -1233,13 +1233,20 @@ __device__ __forceinline__ uint64_t claim_cell(Slot1* s, uint64_t key) {
 }
 __device__ __forceinline__ ulonglong2 claim_cell(Slot2* s, const Key2& key) { return claim16(s, key); }
 
-// Whether the n cells from index `at` on (mod mask + 1) are all taken, read
-// by the whole warp at once (all lanes pass the same arguments).
-template <class S>
-static __device__ __noinline__ bool cells_full(const S* tab, uint32_t at, uint32_t mask, uint32_t n) {
-    bool empty = false;
-    for (uint32_t q = threadIdx.x & 31; q < n; q += 32) empty |= cell_empty(read_cell(tab + ((at + q) & mask)));
-    return !__any_sync(0xffffffffu, empty);
+// Whether the n cells from index `at` on (mod mask + 1) are all taken by other
+// keys, read by the whole warp at once (all lanes pass the same arguments).
+template <class S, class K>
+static __device__ __noinline__ bool cells_full(const S* tab, uint32_t at, uint32_t mask, uint32_t n, K key) {
+    bool open = false;
+    for (uint32_t q = threadIdx.x & 31; q < n; q += 32) {
+        const auto v = read_cell(tab + ((at + q) & mask));
+        open |= cell_empty(v) || cell_holds(v, key);
+    }
+    return !__any_sync(0xffffffffu, open);
+}
+__device__ __forceinline__ uint64_t key_of_lane(uint64_t k, int lane) { return __shfl_sync(0xffffffffu, k, lane); }
+__device__ __forceinline__ Key2 key_of_lane(const Key2& k, int lane) {
+    return Key2{__shfl_sync(0xffffffffu, k.w0, lane), __shfl_sync(0xffffffffu, k.w1, lane)};
 }
 
 template <int NW>
@@ -1581,8 +1588,9 @@ __global__ void __launch_bounds__(CNT_THREADS, count_min_ctas<NW, HALVES>()) cou
                 if (!__any_sync(0xffffffffu, todo != 0)) break;  // warp-uniform
                 if (p % PROBE_CHECK == PROBE_CHECK - 1) {
                     // a long probe sequence: the rest of one pending item's
-                    // window, read at once, tells whether its bucket overflows;
-                    // items of a bucket that does stop here
+                    // window, read at once, tells whether its bucket overflows
+                    // (it does not where the key lies further on); items of a
+                    // bucket that does stop here
 #pragma unroll
                     for (int j = 0; j < ITEMS; ++j) {
                         const uint32_t pend = __ballot_sync(0xffffffffu, (todo >> j) & 1u);
@@ -1591,10 +1599,11 @@ __global__ void __launch_bounds__(CNT_THREADS, count_min_ctas<NW, HALVES>()) cou
                         const uint32_t b = set_bucket0 + (uint32_t)(key_hi(it[j]) >> a.bucket_shift);
                         const uint32_t bs = __shfl_sync(0xffffffffu, b, src);
                         const uint32_t h17 = __shfl_sync(0xffffffffu, (uint32_t)(h[j] >> 17), src);
+                        const K key = key_of_lane(it[j], src);
                         const MetaS m = meta_of(bs);
                         const uint32_t limit = (uint32_t)min((uint64_t)PROBE_LIMIT, (uint64_t)m.tab_mask + 1);
-                        if (p + 1 < limit && cells_full(table + m.tab_off, h17 + p + 1, m.tab_mask, limit - (p + 1)) &&
-                            lane == 0)
+                        if (p + 1 < limit &&
+                            cells_full(table + m.tab_off, h17 + p + 1, m.tab_mask, limit - (p + 1), key) && lane == 0)
                             a.bucket_overflow[bs] = 1u;
                         __syncwarp();
                         if (((todo >> j) & 1u) && __ldcg(a.bucket_overflow + b)) {
