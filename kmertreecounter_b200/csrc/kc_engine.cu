@@ -223,6 +223,7 @@ struct kc_context {
     std::vector<kc::BucketWin> h_bucket_win;
     std::vector<kc::WinInfo> h_win_info;
     std::vector<uint32_t> h_win_order;  // windows in launch order: phase 0, then phase 1
+    bool keys_swapped = false;   // routed and routed2 have changed places (window_count)
     DevBuf routed2, bucket_win, win_info, win_order, win_count, win_padded, win_start, win_cursor, win_end;
     // the whole result was counted in windows in one batch and no table has
     // grown: window r's first occurrences are the low.bin records of its
@@ -1009,6 +1010,7 @@ int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets 
         break;
     }
     std::swap(c->routed, c->routed2);
+    c->keys_swapped = !c->keys_swapped;
     n_keys = spill_start + spill_used;
     c->win_result_spill_seg = spill_start / kc::WIN_SEG;
     CKR(join_init(c));
@@ -1087,6 +1089,15 @@ int launch_extract(kc_context* c, const uint8_t* buf, uint64_t n, int has_halo, 
     return KC_OK;
 }
 
+// Before new keys are routed: the two key buffers take their places again.
+// They differ in size by the windows' slack, and a call that found them
+// exchanged had to allocate one anew (k = 63: 30, 28.5, then 22.3 ms for the
+// first three calls).
+void place_key_buffers(kc_context* c) {
+    if (c->keys_swapped) std::swap(c->routed, c->routed2);
+    c->keys_swapped = false;
+}
+
 template <int NW>
 int count_and_pack(kc_context* c, uint64_t n_keys, const void* src = nullptr);
 
@@ -1098,6 +1109,7 @@ template <int NW>
 int process_batch(kc_context* c, const uint8_t* buf, uint64_t n, int has_halo, bool route_only = false) {
     if (reinterpret_cast<uintptr_t>(buf) % 16)
         return fail(KC_ERR_INVALID, "device FASTQ batch must be 16-byte aligned");
+    place_key_buffers(c);
     const uint32_t nb = c->n_buckets;
     const uint64_t tiles = ceil_div(n, kc::EXT_TILE);
     c->last_batch_low = 0;  // a batch without k-mers packs nothing
@@ -1719,6 +1731,7 @@ int run_batch(kc_context* c, const uint8_t* buf, uint64_t n, int has_halo) {
 // then filter, tables and packing as for a batch of FASTQ.
 template <int NW>
 int count_keys(kc_context* c, const void* d_keys, uint64_t n_keys, const uint64_t* counts) {
+    place_key_buffers(c);
     const uint32_t nb = c->n_buckets;
     const uint32_t per = nb / 256;  // table buckets per routing bucket (1 or 16)
     std::vector<uint64_t> kest(nb);
@@ -2546,6 +2559,7 @@ int count_sets_impl(kc_context* c, const uint8_t* buf, const kc_set_desc* sets, 
     const kc_config& g = c->cfg;
     const uint64_t nbk = (uint64_t)n_sets * NB;
     using KeyT = typename kc::KeyOf<NW>::T;
+    place_key_buffers(c);
 
     // tiles
     std::vector<kc::SetTile> tiles;
