@@ -557,28 +557,20 @@ cudaError_t or_shed(kc_context* c, F alloc) {
 
 // Whether the device has room for 128-bit keys counted in windows: `slots`
 // cells with their growth share, the keys and their sub-routed copy, and all
-// of the input's keys packed (the buffers that the context holds already
-// counted as free).  Where it has not, the filter gets its own array (1.5
-// bytes a key, not 8) and the keys no copy, so that an input is refused for
-// memory no sooner.
+// of the input's keys packed and exported.  Where it has not, the filter gets
+// its own array (1.5 bytes a key, not 8) and the keys no copy, so that an
+// input is refused for memory no sooner.
 bool windows2_fit(const kc_context* c, uint64_t slots, uint64_t keys, double scale) {
-    const double kb = (double)keys * sizeof(kc::Key2);
-    const double need[4] = {(double)slots * c->slot_bytes * 1.25, kb, kb * 17 / 16, (double)keys * scale * c->packed_bytes};
-    const size_t cap[4] = {c->table.cap, c->routed.cap, c->routed2.cap, c->low_packed.cap};
-    double want = 0, held = 0;
-    bool held_all = true;
-    for (int i = 0; i < 4; ++i) {
-        held_all = held_all && need[i] <= (double)cap[i];
-        want += need[i] * 9 / 8;  // as DevBuf::ensure allocates
-        held += (double)cap[i];
-    }
-    if (held_all) return true;
-    size_t free_bytes = 0, total = 0;
-    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return want <= (double)free_bytes + held - (double)total / 16;
+    const double kb = sizeof(kc::Key2), all = (double)keys * scale;
+    const double windows = std::max<double>((double)(slots >> kc::Win<2>::ZSHIFT), c->n_buckets);
+    const KcNeed need[5] = {
+        {(double)slots * c->slot_bytes * 1.25, (double)c->table.cap},
+        {(double)keys * kb, (double)c->routed.cap},
+        {kc_windowed_keys((double)keys, windows) * kb, (double)c->routed2.cap},
+        {all * c->packed_bytes, (double)c->low_packed.cap},
+        {std::min((double)slots, all) * c->record_bytes, (double)c->roots.cap},
+    };
+    return needs_fit(need, 5);
 }
 
 // The global count of 128- and 256-bit keys comes in two forms (halves: every
@@ -1571,7 +1563,7 @@ int finish_run(kc_context* c) {
     if (c->cfg.sort_output && c->root_total > 1) {
         uint64_t bt, bh, bo, bs;
         kc_sort_scratch_bytes(c->root_total, c->record_bytes, &bt, &bh, &bo, &bs);
-        CK(c->sort_tmp.ensure(bt));
+        CK(or_shed(c, [&] { return c->sort_tmp.ensure(bt); }));
         CK(c->sort_hist.ensure(bh));
         CK(c->sort_offs.ensure(bo));
         CK(c->sort_sums.ensure(bs));

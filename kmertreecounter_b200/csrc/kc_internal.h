@@ -1,6 +1,8 @@
 // Internal (non-ABI) declarations shared by the engine's translation units.
 #pragma once
 
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -45,6 +47,13 @@ inline bool kc_needs_fit(const KcNeed* v, int n, double free_bytes) {
             grow = true;
         }
     return !grow || want + (64 << 20) <= free_bytes;
+}
+// Places that sub-routing `keys` keys into `windows` windows takes at most:
+// every window's estimate x 1.1 + 4 sqrt(estimate) + 64, in whole segments of
+// 64 (window_caps), and the spill area's sixteenth (at least 65536).
+inline double kc_windowed_keys(double keys, double windows) {
+    const double ranges = keys * 1.1 + 4.0 * std::sqrt(keys * windows) + 128.0 * windows;
+    return ranges + std::max(ranges / 16 + 64, 65536.0);
 }
 
 int kc_internal_set_error(int code, const char* msg);
