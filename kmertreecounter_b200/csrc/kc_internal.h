@@ -21,10 +21,10 @@ void kc_sort_scratch_bytes(uint64_t n, uint64_t record_bytes, uint64_t* tmp, uin
                            uint64_t* sums);
 
 // Sort root records (ExportRecord<N>, record_bytes each, grouped by root id)
-// by key, keeping the grouping, in place on `stream` (asynchronous).
-// Returns 0 or a negative KC_ERR_* code.
+// by key, keeping the grouping, in place on `stream`; adds the kernels
+// launched to *launches.  Returns 0 or a negative KC_ERR_* code.
 int kc_sort_roots(void* records, uint64_t n, uint64_t record_bytes, uint32_t k, const KcSortScratch& w,
-                  cudaStream_t stream);
+                  cudaStream_t stream, uint64_t* launches);
 const char* kc_sort_error();
 // The same over bare keys of nw 64-bit words (scratch sizes from
 // kc_sort_scratch_bytes with record_bytes = 8 nw).

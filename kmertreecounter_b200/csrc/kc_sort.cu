@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_long_runs(Rec<W>* __restric
 }
 
 template <int NW, int W>
-int sort_impl(void* records, uint64_t n, uint32_t k, const KcSortScratch& w, cudaStream_t st) {
+int sort_impl(void* records, uint64_t n, uint32_t k, const KcSortScratch& w, cudaStream_t st, uint64_t* launches) {
     using R = Rec<W>;
     const uint32_t key_bits = 2 * k;
     const uint32_t lowbit = 64 * NW - key_bits;
@@ -291,6 +291,7 @@ int sort_impl(void* records, uint64_t n, uint32_t k, const KcSortScratch& w, cud
             kc::scan_apply<uint32_t, uint64_t><<<nb, kc::SCAN_BLOCK, 0, st>>>(hist, hn, sums, offs);
             downsweep<NW, W><<<n_tiles, SORT_THREADS, 0, st>>>(src, dst, n, bit, offs, n_tiles);
             std::swap(src, dst);
+            *launches += 5;
         }
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess && src != a) e = cudaMemcpyAsync(a, src, n * sizeof(R), cudaMemcpyDeviceToDevice, st);
@@ -312,6 +313,7 @@ int sort_impl(void* records, uint64_t n, uint32_t k, const KcSortScratch& w, cud
                            st>>>(a, n, 8 * lead, list);
         sort_warp_runs<NW, W><<<148 * 8, 128, 0, st>>>(a, n, 8 * lead, list);
         sort_long_runs<NW, W><<<148 * 2, SORT_THREADS, 0, st>>>(a, n, 8 * lead, list);
+        *launches += 3;
         unsigned long long head[3] = {0, 0, 0};
         if (e == cudaSuccess) e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpyAsync(head, list.count, sizeof head, cudaMemcpyDeviceToHost, st);
@@ -340,20 +342,21 @@ void kc_sort_scratch_bytes(uint64_t n, uint64_t record_bytes, uint64_t* tmp, uin
 }
 
 int kc_sort_roots(void* records, uint64_t n, uint64_t record_bytes, uint32_t k, const KcSortScratch& w,
-                  cudaStream_t stream) {
+                  cudaStream_t stream, uint64_t* launches) {
     if (n < 2) return KC_OK;
-    if (record_bytes == 16 && k <= 32) return sort_impl<1, 2>(records, n, k, w, stream);
-    if (record_bytes == 24 && k <= 64) return sort_impl<2, 3>(records, n, k, w, stream);
-    if (record_bytes == 40 && k <= 128) return sort_impl<4, 5>(records, n, k, w, stream);
+    if (record_bytes == 16 && k <= 32) return sort_impl<1, 2>(records, n, k, w, stream, launches);
+    if (record_bytes == 24 && k <= 64) return sort_impl<2, 3>(records, n, k, w, stream, launches);
+    if (record_bytes == 40 && k <= 128) return sort_impl<4, 5>(records, n, k, w, stream, launches);
     g_sort_err = "unsupported record layout";
     return KC_ERR_INVALID;
 }
 
 int kc_sort_keys(void* keys, uint64_t n, uint32_t nw, uint32_t k, const KcSortScratch& w, cudaStream_t stream) {
+    uint64_t launches = 0;
     if (n < 2) return KC_OK;
-    if (nw == 1 && k <= 32) return sort_impl<1, 1>(keys, n, k, w, stream);
-    if (nw == 2 && k <= 64) return sort_impl<2, 2>(keys, n, k, w, stream);
-    if (nw == 4 && k <= 128) return sort_impl<4, 4>(keys, n, k, w, stream);
+    if (nw == 1 && k <= 32) return sort_impl<1, 1>(keys, n, k, w, stream, &launches);
+    if (nw == 2 && k <= 64) return sort_impl<2, 2>(keys, n, k, w, stream, &launches);
+    if (nw == 4 && k <= 128) return sort_impl<4, 4>(keys, n, k, w, stream, &launches);
     g_sort_err = "unsupported key width";
     return KC_ERR_INVALID;
 }
