@@ -309,13 +309,15 @@ int sort_impl(void* records, uint64_t n, uint32_t k, const KcSortScratch& w, cud
         const RunList list{base + 8, reinterpret_cast<unsigned long long*>(hist), base};
         e = run(64 * NW - 8 * lead, lead);
         if (e == cudaSuccess) e = cudaMemsetAsync(list.count, 0, 8 * sizeof(*base), st);
-        sort_runs<NW, W><<<(uint32_t)std::min<uint64_t>((n + SORT_THREADS - 1) / SORT_THREADS, 148 * 8), SORT_THREADS, 0,
-                           st>>>(a, n, 8 * lead, list);
-        sort_warp_runs<NW, W><<<148 * 8, 128, 0, st>>>(a, n, 8 * lead, list);
-        sort_long_runs<NW, W><<<148 * 2, SORT_THREADS, 0, st>>>(a, n, 8 * lead, list);
-        *launches += 3;
+        if (e == cudaSuccess) {  // (the run kernels index by the counters)
+            sort_runs<NW, W><<<(uint32_t)std::min<uint64_t>((n + SORT_THREADS - 1) / SORT_THREADS, 148 * 8),
+                               SORT_THREADS, 0, st>>>(a, n, 8 * lead, list);
+            sort_warp_runs<NW, W><<<148 * 8, 128, 0, st>>>(a, n, 8 * lead, list);
+            sort_long_runs<NW, W><<<148 * 2, SORT_THREADS, 0, st>>>(a, n, 8 * lead, list);
+            *launches += 3;
+            e = cudaGetLastError();
+        }
         unsigned long long head[3] = {0, 0, 0};
-        if (e == cudaSuccess) e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpyAsync(head, list.count, sizeof head, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e == cudaSuccess && head[2]) e = run(lowbit, passes);
