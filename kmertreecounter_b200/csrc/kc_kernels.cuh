@@ -91,12 +91,13 @@ constexpr uint64_t EST_MIN_TILES = 4096;
 constexpr int CNT_THREADS = 256;                     // count CTA
 constexpr uint64_t EMPTY = ~0ull;                    // never a canonical key
 constexpr int PROBE_LIMIT = 512;                     // linear-probe bound before overflow
-// Probes between two looks at whether the bucket has overflowed already.  A
-// bucket that overflows is grown and its failed keys are inserted then, so
-// once one key has met a full probe window the others of the bucket need not
-// walk theirs to the end.  100,000 reads at 3x coverage, whose tables fill
-// up: count stage 5.6 ms with every key walking 512 cells, 0.76 ms now; 48
-// read sets with 1408 growths: 33.4 -> 26.4 ms.
+// Probes between two looks at whether the bucket has overflowed already, and
+// the lockstep rounds of count_routed after which a key's window is probed by
+// the whole warp (insert_far).  A bucket that overflows is grown and its failed
+// keys are inserted then, so once one key has met a full probe window the
+// others of the bucket need not walk theirs to the end.  100,000 reads at 3x
+// coverage, whose tables fill up: count stage 5.6 ms with every key walking 512
+// cells, 0.76 ms with an early end.
 constexpr uint32_t PROBE_CHECK = 32;
 
 // One 128-bit key word pair in the reference's kmer<2> order: w0 = data[0]
@@ -1233,20 +1234,66 @@ __device__ __forceinline__ uint64_t claim_cell(Slot1* s, uint64_t key) {
 }
 __device__ __forceinline__ ulonglong2 claim_cell(Slot2* s, const Key2& key) { return claim16(s, key); }
 
-// Whether the n cells from index `at` on (mod mask + 1) are all taken by other
-// keys, read by the whole warp at once (all lanes pass the same arguments).
-template <class S, class K>
-static __device__ __noinline__ bool cells_full(const S* tab, uint32_t at, uint32_t mask, uint32_t n, K key) {
-    bool open = false;
-    for (uint32_t q = threadIdx.x & 31; q < n; q += 32) {
-        const auto v = read_cell(tab + ((at + q) & mask));
-        open |= cell_empty(v) || cell_holds(v, key);
-    }
-    return !__any_sync(0xffffffffu, open);
-}
 __device__ __forceinline__ uint64_t key_of_lane(uint64_t k, int lane) { return __shfl_sync(0xffffffffu, k, lane); }
 __device__ __forceinline__ Key2 key_of_lane(const Key2& k, int lane) {
     return Key2{__shfl_sync(0xffffffffu, k.w0, lane), __shfl_sync(0xffffffffu, k.w1, lane)};
+}
+
+// Keys with long probe sequences: the n keys before `end` (a segment's back),
+// whose first PROBE_CHECK cells hold other keys, are inserted one after another
+// by the whole warp, 32 cells a round, of which those that hold the key or read
+// empty are settled in probe order.  Keys that find no room in their probe
+// window, or whose bucket has overflowed already, stay; returns their number.
+template <class S, class K>
+static __device__ __forceinline__ uint32_t insert_far(K* end, uint32_t n, uint32_t bucket0, S* __restrict__ table,
+                                                   const BucketMeta* __restrict__ meta, uint32_t bucket_shift,
+                                                   uint32_t* bucket_overflow) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t kept = 0;
+    for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+        const bool in = i0 + lane < n;
+        K own = *(end - 1 - (in ? i0 + lane : i0));
+        __syncwarp();  // every read precedes the writes below
+        uint32_t failed = 0;
+        for (uint32_t left = __ballot_sync(0xffffffffu, in); left;) {
+            const K key = key_of_lane(own, __ffs(left) - 1);
+            const uint32_t same = __ballot_sync(0xffffffffu, in && same_key(own, key));  // its occurrences
+            left &= ~same;
+            const uint32_t b = bucket0 + (uint32_t)(key_hi(key) >> bucket_shift);
+            S* tab = table + __ldg(&meta[b].tab_off);
+            const uint32_t mask = (uint32_t)__ldg(&meta[b].tab_mask);
+            const uint32_t limit = (uint32_t)min((uint64_t)PROBE_LIMIT, (uint64_t)mask + 1);
+            const uint32_t home = (uint32_t)(hash_key(key) >> 17);
+            bool added = false;
+            const bool full = __ldcg(bucket_overflow + b) != 0;
+            if (__any_sync(0xffffffffu, full)) {
+                failed |= same;
+                continue;
+            }
+            for (uint32_t p = PROBE_CHECK; p < limit && !added; p += 32) {
+                S* s = tab + ((home + p + lane) & mask);
+                auto v = read_cell(s);
+                uint32_t open = __ballot_sync(0xffffffffu, p + lane < limit && (cell_empty(v) || cell_holds(v, key)));
+                for (; open && !added; open &= open - 1) {
+                    bool mine = false;
+                    if (lane == __ffs(open) - 1) {
+                        if (cell_empty(v)) v = claim_cell(s, key);
+                        mine = cell_holds(v, key);
+                        if (mine) atomicAdd(&s->count, (uint32_t)__popc(same));
+                    }
+                    added = __any_sync(0xffffffffu, mine);
+                }
+            }
+            if (!added) {
+                failed |= same;
+                if (lane == 0) bucket_overflow[b] = 1u;
+            }
+        }
+        if ((failed >> lane) & 1u) *(end - 1 - (kept + __popc(failed & ((1u << lane) - 1u)))) = own;
+        kept += __popc(failed);
+        __syncwarp();
+    }
+    return kept;
 }
 
 template <int NW>
@@ -1375,6 +1422,18 @@ __global__ void __launch_bounds__(CNT_THREADS, count_min_ctas<NW, HALVES>()) cou
     // dispatched in blockIdx order, so the keys in flight stay within a narrow
     // window of the bucket-sorted array (one or two buckets' filter and table
     // lines live in L2 at a time).
+    auto bucket0_of = [&](uint64_t gw) {  // first bucket of the set that segment gw belongs to
+        if (!a.n_sets) return 0u;
+        uint32_t lo = 0, hi = a.n_sets;  // last set whose first segment <= gw
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) / 2;
+            if (a.set_seg_start[mid] <= gw) lo = mid;
+            else hi = mid;
+        }
+        return lo * a.set_buckets;
+    };
+    __shared__ uint32_t s_far[CNT_THREADS / 32];  // keys lie at the back of some of the warp's segments
+    if (NW <= 2 && lane == 0) s_far[threadIdx.x >> 5] = 0;
     const uint64_t cta_seg0 = (uint64_t)blockIdx.x * (CNT_THREADS / 32) * CNT_SEGS_PER_WARP;
     const uint64_t cta_seg1 = min(n_segs, cta_seg0 + (uint64_t)(CNT_THREADS / 32) * CNT_SEGS_PER_WARP);
     for (uint64_t gw = cta_seg0 + (threadIdx.x >> 5); gw < cta_seg1; gw += CNT_THREADS / 32) {
@@ -1389,16 +1448,7 @@ __global__ void __launch_bounds__(CNT_THREADS, count_min_ctas<NW, HALVES>()) cou
             n_in = nf;
         }
 
-        uint32_t set_bucket0 = 0;
-        if (a.n_sets) {
-            uint32_t lo = 0, hi = a.n_sets;  // last set whose first segment <= gw
-            while (hi - lo > 1) {
-                const uint32_t mid = (lo + hi) / 2;
-                if (a.set_seg_start[mid] <= gw) lo = mid;
-                else hi = mid;
-            }
-            set_bucket0 = lo * a.set_buckets;
-        }
+        const uint32_t set_bucket0 = bucket0_of(gw);
         K it[ITEMS];
         uint32_t mult[ITEMS];
 #pragma unroll
@@ -1586,32 +1636,9 @@ __global__ void __launch_bounds__(CNT_THREADS, count_min_ctas<NW, HALVES>()) cou
                     }
                 }
                 if (!__any_sync(0xffffffffu, todo != 0)) break;  // warp-uniform
-                if (p % PROBE_CHECK == PROBE_CHECK - 1) {
-                    // a long probe sequence: the rest of one pending item's
-                    // window, read at once, tells whether its bucket overflows
-                    // (it does not where the key lies further on); items of a
-                    // bucket that does stop here
-#pragma unroll
-                    for (int j = 0; j < ITEMS; ++j) {
-                        const uint32_t pend = __ballot_sync(0xffffffffu, (todo >> j) & 1u);
-                        if (!pend) continue;  // warp-uniform
-                        const int src = __ffs(pend) - 1;
-                        const uint32_t b = set_bucket0 + (uint32_t)(key_hi(it[j]) >> a.bucket_shift);
-                        const uint32_t bs = __shfl_sync(0xffffffffu, b, src);
-                        const uint32_t h17 = __shfl_sync(0xffffffffu, (uint32_t)(h[j] >> 17), src);
-                        const K key = key_of_lane(it[j], src);
-                        const MetaS m = meta_of(bs);
-                        const uint32_t limit = (uint32_t)min((uint64_t)PROBE_LIMIT, (uint64_t)m.tab_mask + 1);
-                        if (p + 1 < limit &&
-                            cells_full(table + m.tab_off, h17 + p + 1, m.tab_mask, limit - (p + 1), key) && lane == 0)
-                            a.bucket_overflow[bs] = 1u;
-                        __syncwarp();
-                        if (((todo >> j) & 1u) && __ldcg(a.bucket_overflow + b)) {
-                            fail_bits |= 1u << j;
-                            todo &= ~(1u << j);
-                        }
-                    }
-                    if (!__any_sync(0xffffffffu, todo != 0)) break;  // warp-uniform
+                if (p + 1 == PROBE_CHECK) {  // the rest by insert_far
+                    fail_bits |= todo;
+                    break;
                 }
 #pragma unroll
                 for (int j = 0; j < ITEMS; ++j) {
@@ -1647,10 +1674,25 @@ __global__ void __launch_bounds__(CNT_THREADS, count_min_ctas<NW, HALVES>()) cou
                 for (uint32_t r = 0; r < f; ++r) keys[s_end - 1 - (my0 + r)] = it[j];
                 n_fail += wtot;
             }
+            if (NW <= 2 && lane == 0) s_far[threadIdx.x >> 5] = 1;
         }
         if (lane == 0) {
             if (a.use_filter) a.seg_low[gw] = n_low;
             a.seg_fail[gw] = n_fail;
+        }
+    }
+    // Long probe sequences, once the warp's segments are through: looked into
+    // in the rounds above they cost the kernel 200 bytes of spills (10 M reads
+    // in five passes, 64-bit keys: count 4.6 ms without, 6.5 with).
+    if constexpr (NW <= 2) {
+        __syncwarp();
+        if (!s_far[threadIdx.x >> 5]) return;
+        for (uint64_t gw = cta_seg0 + (threadIdx.x >> 5); gw < cta_seg1; gw += CNT_THREADS / 32) {
+            const uint32_t nf = a.seg_fail[gw];
+            if (nf == 0) continue;  // warp-uniform
+            const uint32_t kept = insert_far(keys + min(a.n_keys, gw * SEG + SEG), nf, bucket0_of(gw), table, a.meta,
+                                             a.bucket_shift, a.bucket_overflow);
+            if (lane == 0) a.seg_fail[gw] = kept;
         }
     }
 }

@@ -47,9 +47,26 @@ def test_exactly_full_table_without_allocation(k):
     data = _reads(k, 64, 100, seed=k)
     keys, counts, _ = oracle.count(data, k)
     cfg = kc.default_config(k=k, repeat_ratio=1e-6, bloom_bits=0.1)
-    rc, st, low, roots = noalloc(cfg, torch.from_numpy(data).cuda(), data.size, 1 << 20, 1 << 20)
+    rc, st, low, roots = noalloc(cfg, torch.from_numpy(data.copy()).cuda(), data.size, 1 << 20, 1 << 20)
     assert rc == 0 and st.rehashes == 0 and st.table_keys == 64
     n = st.low_records * kc.packed_bytes(k)
     (mk, mc), _, _ = merged_from(low.cpu().numpy()[:n], roots.cpu().numpy()[:st.root_records * kc.record_bytes(k)], k,
                                  st.root_records)
     assert np.array_equal(mk, keys) and np.array_equal(mc, counts.astype(np.uint64))
+
+
+@pytest.mark.parametrize("k,slots", [(31, 512), (63, 256)])
+@pytest.mark.parametrize("over", [-40, 1, 60])
+def test_nearly_full_and_overfull_tables(monkeypatch, k, slots, over):
+    """Keys that end far from their first cell, several occurrences together in a segment's back."""
+    monkeypatch.setenv("KC_WINDOW_COUNT", "0")
+    data = _reads(k, slots + over, 30, seed=100 + k + over)
+    lines = data.tobytes().split(b"\n")[1::4]
+    hot = b"".join(b"@h\n%s\n+\n%s\n" % (s, b"I" * k) for s in lines[:slots + over] for _ in range(7))
+    data = np.concatenate([data, np.frombuffer(hot, np.uint8), data])
+    want = oracle.count(data, k)
+    with kc.Counter(k=k, repeat_ratio=1e-6, bloom_bits=0.1) as c:
+        for _ in range(2):
+            st = c.count_host(data)
+            parity.check_exact(c, data, k, want)
+            assert (st.rehashes > 0) == (over > 0)
