@@ -122,6 +122,10 @@ inline uint64_t pow2_at_least(uint64_t x) { return std::bit_ceil(std::max<uint64
 // Routed keys of a multi-set pass from which it is counted in windows.
 constexpr uint64_t SETS_WINDOW_KEYS = 4ull << 20;
 
+// Keys from which window capacities are estimated from every 16th chunk:
+// sampled ranges need enough sampled chunks per window to be worth it.
+constexpr uint64_t WINDOW_SAMPLE_KEYS = 64ull * 16 * kc::SUB_CHUNK;
+
 // A last batch whose keys (packed) and tables take at most this much is packed
 // and exported without waiting for its counts (count_and_pack): the bounds of
 // both outputs are allocated.  1000 reads: three waits of ~12 us in 260.
@@ -531,9 +535,12 @@ int init_now(kc_context* c) {
     return KC_OK;
 }
 
-// Whether the device has room for the buffers (kc_needs_fit).
-bool needs_fit(const KcNeed* v, int n) {
-    if (kc_needs_fit(v, n, -1e30)) return true;  // all held: no question to the driver
+// Whether the device has room for n buffers (kc_needs_fit).  A context that
+// holds the first `before` of them, which are allocated before the keys are
+// counted, asks the driver nothing (60 us a call): the others may take the
+// second key buffer's place (or_shed).
+bool needs_fit(const KcNeed* v, int before, int n) {
+    if (kc_needs_fit(v, before, -1e30)) return true;
     size_t free_bytes = 0, total = 0;
     if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
         cudaGetLastError();
@@ -566,11 +573,11 @@ bool windows2_fit(const kc_context* c, uint64_t slots, uint64_t keys, double sca
     const KcNeed need[5] = {
         {(double)slots * c->slot_bytes * 1.25, (double)c->table.cap},
         {(double)keys * kb, (double)c->routed.cap},
-        {kc_windowed_keys((double)keys, windows) * kb, (double)c->routed2.cap},
+        {kc_windowed_keys((double)keys, windows, keys >= WINDOW_SAMPLE_KEYS) * kb, (double)c->routed2.cap},
         {all * c->packed_bytes, (double)c->low_packed.cap},
         {std::min((double)slots, all) * c->record_bytes, (double)c->roots.cap},
     };
-    return needs_fit(need, 5);
+    return needs_fit(need, 3, 5);
 }
 
 // The global count of 128- and 256-bit keys comes in two forms (halves: every
@@ -928,8 +935,7 @@ int window_count(kc_context* c, uint64_t& n_keys, uint32_t nb, kc::SetSpan sets 
     const auto* bwin = c->bucket_win.as<kc::BucketWin>();
     const uint64_t cchunks = ceil_div(n_keys, kc::SUB_CHUNK);
     const uint64_t small_grid = std::min<uint64_t>(ceil_div(nw, 256), (uint64_t)c->sm_count * 8);
-    // sampled ranges need enough sampled chunks per window to be worth it
-    uint32_t stride = cchunks >= 64ull * 16 && !sets.n ? 16u : 1u;
+    uint32_t stride = n_keys >= WINDOW_SAMPLE_KEYS && !sets.n ? 16u : 1u;
     uint64_t total = 0, spill_start = 0, spill_used = 0;
     for (;;) {
         CKR(fill_dev(c, c->win_count.p, nw * sizeof(uint32_t), 0));
@@ -2644,26 +2650,59 @@ route_again:
     // layout: each set's routed region starts on a segment boundary
     std::vector<uint64_t> start(nbk), rend(nbk), set_key0(n_sets), set_key1(n_sets), set_next(n_sets), set_seg(n_sets);
     std::vector<uint64_t> ovf_start(n_sets), ovf_end(n_sets);
-    std::vector<uint64_t> kmers(nbk);  // per bucket (estimated for a sampled set)
-    uint64_t pos = 0, K = 0, low_bound = 0;
+    uint64_t pos = 0, K = 0, bw = 0, ts = 0, low_bound = 0;
+    c->h_meta.assign(nbk, kc::BucketMeta{});
+    // filter and tables by learned sizing (kc_set_predicted_set_rates) when
+    // predictions for these n_sets sets were handed over: predicted rates x the
+    // bucket's exact k-mer total, 12 filter bits per distinct key, table keys
+    // with 15% headroom at the target load; else (and for a negative rate) by
+    // the sampled rule on the exact per-bucket k-mer totals
+    const bool learned = g.sizing == KC_SIZING_LEARNED && c->set_pred_table.size() == nbk;
+    // bucket q of kb k-mers; in_cells: the filter words are the cells' pad
+    // fields, as for one input
+    auto place = [&](uint64_t q, uint64_t kb, bool in_cells) {
+        uint64_t words, slots;
+        if (learned && c->set_pred_distinct[q] >= 0.0 && c->set_pred_table[q] >= 0.0) {
+            const double d = std::min(c->set_pred_distinct[q], 1.0) * (double)kb;
+            const double t = std::min(c->set_pred_table[q], 1.0) * (double)kb;
+            words = pow2_at_least(std::max<uint64_t>((uint64_t)(d * 12.0 / 64.0), 64));
+            slots = pow2_at_least(std::max<uint64_t>((uint64_t)(t * 1.15 / g.table_load), 64));
+        } else {
+            words = pow2_at_least(std::max<uint64_t>((uint64_t)(kb * g.bloom_bits / 64.0), 64));
+            slots = pow2_at_least(std::max<uint64_t>((uint64_t)(kb * g.repeat_ratio / g.table_load), 64));
+        }
+        if (in_cells) {
+            slots = std::max<uint64_t>(slots, 2 * words);
+            c->h_meta[q] = kc::BucketMeta{ts, slots - 1, ts, slots - 1};
+        } else {
+            c->h_meta[q] = kc::BucketMeta{bw, words - 1, ts, slots - 1};
+            bw += words;
+        }
+        ts += slots;
+    };
+    auto kmers_of = [&](uint32_t s, uint32_t b) {  // (estimated for a sampled set)
+        const uint64_t n = cnt[(uint64_t)s * NB + b];
+        return sampled[s] ? (uint64_t)((double)n * factor[s]) : n;
+    };
     for (uint32_t s = 0; s < n_sets; ++s) {
         pos = ceil_div(pos, SEG) * SEG;
         set_key0[s] = pos;
         set_seg[s] = pos / SEG;
-        uint64_t set_cap = 0;
+        uint64_t set_cap = 0, set_kmers = 0;
         for (uint32_t b = 0; b < NB; ++b) {
-            // k-mers of the bucket (estimated for a sampled set) and its region
+            // k-mers of the bucket and its region
             const double e = (double)cnt[(uint64_t)s * NB + b] * factor[s];
-            const uint64_t kb = sampled[s] ? (uint64_t)e : cnt[(uint64_t)s * NB + b];
+            const uint64_t kb = kmers_of(s, b);
             const uint64_t cap = sampled[s] ? (uint64_t)(e * 1.02 + 4.0 * std::sqrt(e) + 256.0) : kb;
             start[(uint64_t)s * NB + b] = pos;
             pos += cap;
             rend[(uint64_t)s * NB + b] = pos;
             set_cap += cap;
-            kmers[(uint64_t)s * NB + b] = kb;
-            K += kb;
-            low_bound += kb * kc_packed_bytes(sets[s].k);
+            place((uint64_t)s * NB + b, kb, NW == 1);
+            set_kmers += kb;
         }
+        K += set_kmers;
+        low_bound += set_kmers * kc_packed_bytes(sets[s].k);
         ovf_start[s] = pos;
         if (sampled[s]) pos += std::max<uint64_t>(1ull << 16, set_cap / 32);
         ovf_end[s] = pos;
@@ -2673,39 +2712,6 @@ route_again:
     for (uint32_t s = 0; s < n_sets; ++s) set_next[s] = (s + 1 < n_sets) ? set_key0[s + 1] : n_keys;
     c->K = K;
     c->cells2 = false;
-    // filter and tables by learned sizing (kc_set_predicted_set_rates) when
-    // predictions for these n_sets sets were handed over: predicted rates x the
-    // bucket's exact k-mer total, 12 filter bits per distinct key, table keys
-    // with 15% headroom at the target load; else (and for a negative rate) by
-    // the sampled rule on the exact per-bucket k-mer totals
-    const bool learned = g.sizing == KC_SIZING_LEARNED && c->set_pred_table.size() == nbk;
-    uint64_t bw = 0, ts = 0;
-    auto place = [&](bool in_cells) {
-        c->h_meta.assign(nbk, kc::BucketMeta{});
-        bw = ts = 0;
-        for (uint64_t q = 0; q < nbk; ++q) {
-            const uint64_t kb = kmers[q];
-            uint64_t words, slots;
-            if (learned && c->set_pred_distinct[q] >= 0.0 && c->set_pred_table[q] >= 0.0) {
-                const double d = std::min(c->set_pred_distinct[q], 1.0) * (double)kb;
-                const double t = std::min(c->set_pred_table[q], 1.0) * (double)kb;
-                words = pow2_at_least(std::max<uint64_t>((uint64_t)(d * 12.0 / 64.0), 64));
-                slots = pow2_at_least(std::max<uint64_t>((uint64_t)(t * 1.15 / g.table_load), 64));
-            } else {
-                words = pow2_at_least(std::max<uint64_t>((uint64_t)(kb * g.bloom_bits / 64.0), 64));
-                slots = pow2_at_least(std::max<uint64_t>((uint64_t)(kb * g.repeat_ratio / g.table_load), 64));
-            }
-            if (in_cells) {  // the filter words are the cells' pad fields, as for one input
-                slots = std::max<uint64_t>(slots, 2 * words);
-                c->h_meta[q] = kc::BucketMeta{ts, slots - 1, ts, slots - 1};
-            } else {
-                c->h_meta[q] = kc::BucketMeta{bw, words - 1, ts, slots - 1};
-                bw += words;
-            }
-            ts += slots;
-        }
-        c->table_slots_used = ts;
-    };
     // 64-bit keys of a large pass are counted in windows (the rule for one
     // input; SETS_WINDOW_KEYS keys pay for the extra launches and the exact
     // window counts): 48 sets of 10k-300k reads, 543 M k-mers, 34.6 ms by the
@@ -2714,23 +2720,29 @@ route_again:
     // pass does not fit the device so, it does without the one, then without
     // the other, so that it is refused for memory no sooner.
     bool in_cells = NW == 1;
-    place(in_cells);
+    c->table_slots_used = ts;
     auto fits = [&](bool second) {
         const double kb = (double)n_keys * sizeof(KeyT);
         const KcNeed need[5] = {
+            {second ? kb + (double)c->n_wins * kc::WIN_SEG * sizeof(KeyT) : 0.0, (double)c->routed2.cap},
             {(double)ts * c->slot_bytes * 1.25, (double)c->table.cap},
             {kb, (double)c->routed.cap},
             {(double)low_bound, (double)c->low_packed.cap},
             {(double)std::min(ts, K) * c->record_bytes, (double)c->roots.cap},
-            {kb + (double)c->n_wins * kc::WIN_SEG * sizeof(KeyT), (double)c->routed2.cap},
         };
-        return needs_fit(need, second ? 5 : 4);
+        return needs_fit(need, 3, 5);
     };
     bool windowed = in_cells && n_keys >= SETS_WINDOW_KEYS && windows_pay(c, n_keys) &&
                     build_windows(c, (uint32_t)nbk) && fits(true);
     if (!windowed && !fits(false)) {
         c->routed2.release();  // an earlier count's
-        if (in_cells && !fits(false)) place(in_cells = false);
+        if (in_cells && !fits(false)) {
+            in_cells = false;
+            bw = ts = 0;
+            for (uint32_t s = 0; s < n_sets; ++s)
+                for (uint32_t b = 0; b < NB; ++b) place((uint64_t)s * NB + b, kmers_of(s, b), false);
+            c->table_slots_used = ts;
+        }
     }
     c->bloom_words = in_cells ? ts / 2 : bw;
     CK(c->bloom.ensure(bw * sizeof(uint64_t)));

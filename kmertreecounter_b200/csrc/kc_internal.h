@@ -48,10 +48,12 @@ inline bool kc_needs_fit(const KcNeed* v, int n, double free_bytes) {
         }
     return !grow || want + (64 << 20) <= free_bytes;
 }
-// Places that sub-routing `keys` keys into `windows` windows takes at most:
-// every window's estimate x 1.1 + 4 sqrt(estimate) + 64, in whole segments of
-// 64 (window_caps), and the spill area's sixteenth (at least 65536).
-inline double kc_windowed_keys(double keys, double windows) {
+// Places that sub-routing `keys` keys into `windows` windows takes at most, in
+// whole segments of 64: exact ranges, or (sampled) every window's estimate
+// x 1.1 + 4 sqrt(estimate) + 64 (window_caps) and the spill area's sixteenth
+// (at least 65536).
+inline double kc_windowed_keys(double keys, double windows, bool sampled) {
+    if (!sampled) return keys + 64.0 * windows;
     const double ranges = keys * 1.1 + 4.0 * std::sqrt(keys * windows) + 128.0 * windows;
     return ranges + std::max(ranges / 16 + 64, 65536.0);
 }

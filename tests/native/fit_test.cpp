@@ -22,6 +22,7 @@ int main() {
     const KcNeed mixed[2] = {{8 * G, 7 * G}, {4 * G, 50 * G}};
     check(kc_needs_fit(mixed, 2, 2.1 * G), true, "a buffer is given back before it grows");
     check(kc_needs_fit(mixed, 2, 2 * G), false, "a buffer that stays gives nothing back");
+    check(kc_windowed_keys(1e6, 512, false) == 1e6 + 64 * 512, true, "exact ranges");
     // the sub-routed keys' places against window_caps' sum over windows of
     // even, skewed and mostly empty contents
     for (int form = 0; form < 3; ++form)
@@ -35,9 +36,9 @@ int main() {
                     sum += std::ceil((est * 1.1 + 4 * std::sqrt(est) + 64) / 64) * 64;
                 }
                 sum += std::max(65536.0, sum / 16);
-                check(kc_windowed_keys(keys, windows) >= sum, true, "room for every window");
+                check(kc_windowed_keys(keys, windows, true) >= sum, true, "room for every window");
                 if (keys > 1e6 * windows)
-                    check(kc_windowed_keys(keys, windows) < 1.2 * keys, true, "no more than the windows' slack");
+                    check(kc_windowed_keys(keys, windows, true) < 1.2 * keys, true, "no more than the windows' slack");
             }
     if (!bad) std::printf("ok\n");
     return bad != 0;
