@@ -122,6 +122,13 @@ inline uint64_t pow2_at_least(uint64_t x) { return std::bit_ceil(std::max<uint64
 // Routed keys of a multi-set pass from which it is counted in windows.
 constexpr uint64_t SETS_WINDOW_KEYS = 4ull << 20;
 
+// 128-bit keys of a batch from which they are counted in windows: smaller
+// inputs leave the device's shared memory half empty (few windows, in two
+// phases).  k = 63, 150 bp at 10x, count alone, global against windowed: 50,000
+// reads 0.46 / 0.59 ms, 200,000 1.13 / 1.48, 400,000 (35 M keys) 1.95 / 2.00,
+// 600,000 2.81 / 2.75, 4 M 17.2 / 14.5.
+constexpr uint64_t WINDOW2_KEYS = 40ull << 20;
+
 // Keys from which window capacities are estimated from every 16th chunk:
 // sampled ranges need enough sampled chunks per window to be worth it.
 constexpr uint64_t WINDOW_SAMPLE_KEYS = 64ull * 16 * kc::SUB_CHUNK;
@@ -221,7 +228,9 @@ struct kc_context {
     uint64_t sets_instantiations = 0;         // times that graph had to be instantiated
     // windowed count of 64-bit keys (kc_window.cuh): window-grouped keys,
     // per-bucket window ids and per-window counts and key ranges
-    bool window_count = true;    // KC_WINDOW_COUNT=0 in the environment: count_routed only
+    // KC_WINDOW_COUNT in the environment: 0 = count_routed only, 1 = windows at
+    // every size, unset = by the sizes below which they are slower
+    bool window_count = true, window_always = false;
     bool win_ready = false;      // windows built for the current table layout
     uint64_t n_wins = 0, n_wins_phase0 = 0;
     std::vector<kc::BucketWin> h_bucket_win;
@@ -653,7 +662,7 @@ int size_structures(kc_context* c, const std::vector<uint64_t>& kb, double scale
     uint64_t batch_keys = 0;
     for (uint32_t b = 0; b < nb; ++b) batch_keys += kb[b];
     c->cells2 = false;
-    if (c->nw == 2 && g.k <= 63 && c->window_count) {
+    if (c->nw == 2 && g.k <= 63 && c->window_count && (c->window_always || batch_keys >= WINDOW2_KEYS)) {
         place(true);
         c->cells2 = batch_keys >= 2 * ts && windows2_fit(c, ts, batch_keys, scale);
         if (!c->cells2) place(false);
@@ -1858,7 +1867,10 @@ int kc_create(const kc_config* cfg, kc_context** out) {
         delete c;
         return fail(KC_ERR_DEVICE, "kernel attribute setup failed: %s", cudaGetErrorString(e));
     }
-    if (const char* w = std::getenv("KC_WINDOW_COUNT")) c->window_count = std::strcmp(w, "0") != 0;
+    if (const char* w = std::getenv("KC_WINDOW_COUNT")) {
+        c->window_count = std::strcmp(w, "0") != 0;
+        c->window_always = c->window_count;
+    }
     *out = c;
     return KC_OK;
 }

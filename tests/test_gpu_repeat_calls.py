@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("form,k", [("input", 31), ("input", 63), ("input", 101), ("sets", 31), ("routed", 63)])
-def test_second_call_allocates_nothing(form, k):
+def test_second_call_allocates_nothing(monkeypatch, form, k):
+    monkeypatch.setenv("KC_WINDOW_COUNT", "1")  # windows wherever the key width has them
     data = synth.fastq(synth.params(seed=k, genome_len=1_500_000, n_reads=400_000, read_len=(150, 150)))
     pad = np.full(-data.size % 16, ord("\n"), np.uint8)
     d = torch.from_numpy(np.concatenate([data, pad])).cuda()
