@@ -52,3 +52,27 @@ def test_many_windows_per_bucket(monkeypatch, k, reads, buckets):
             assert _windowed(c) == (env == "1")
             assert st.max_bucket_table_slots > (4096 if k <= 32 else 2048)  # the cells of one window
             parity.check_exact(c, data, k, want)
+
+
+@pytest.mark.parametrize("sets,reads,by_size", [(400, 400, False), (6, 60_000, True)])
+def test_read_sets(monkeypatch, sets, reads, by_size):
+    """A pass of many small sets has few keys for each window."""
+    one = _reads(reads, genome=max(2000, reads))
+    pad = np.full(-one.size % 16, ord("\n"), np.uint8)
+    part = torch.from_numpy(np.concatenate([one, pad])).cuda()
+    buf = part.repeat(sets)
+    desc = [(i * part.numel(), one.size, 31) for i in range(sets)]
+    keys, counts, K = oracle.count(one, 31)
+    assert K * sets > 4 << 20
+    for env, want in ((None, by_size), ("0", False)):
+        monkeypatch.delenv("KC_WINDOW_COUNT", raising=False)
+        if env:
+            monkeypatch.setenv("KC_WINDOW_COUNT", env)
+        with kc.Counter(k=31) as c:
+            res = c.count_sets(buf.data_ptr(), desc)
+            assert _windowed(c) == want, env
+            low_all, (roots_all, _) = c.low_bytes(), c.root_records()
+            for r in (res[0], res[sets // 2], res[-1]):
+                low = oracle.unpack(low_all[r.low_offset:r.low_offset + r.low_bytes], 31)
+                mk, mc = parity.merged(low, roots_all[r.root_offset:r.root_offset + r.root_records], 31)
+                assert r.total_kmers == K and np.array_equal(mk, keys) and np.array_equal(mc, counts.astype(np.uint64))
