@@ -2357,6 +2357,17 @@ void loads_kernels(kc_context* c, unsigned long long* dd) {
 
 }  // namespace
 
+namespace {
+
+// A streamed count hands its packed first occurrences to the sink and keeps
+// none of them: calls that read them are refused.
+int low_kept(const kc_context* c) {
+    if (c->low_total && !c->low_packed.p) return fail(KC_ERR_STATE, "streamed results are not kept on the device");
+    return KC_OK;
+}
+
+}  // namespace
+
 extern "C" {
 
 // Merged count histogram and distinct keys of the last device-held result.
@@ -2364,7 +2375,7 @@ int kc_histogram(kc_context* c, uint32_t min_freq, uint32_t max_freq, uint64_t* 
     if (!c) return fail(KC_ERR_INVALID, "null context");
     if (!c->have_result) return fail(KC_ERR_STATE, "no result: run a count first");
     if (c->batch_result) return fail(KC_ERR_STATE, "a multi-set result has one histogram per set; not supported");
-    if (c->stream_low) return fail(KC_ERR_STATE, "streamed results are not kept on the device");
+    CKR(low_kept(c));
     if (max_freq < min_freq || min_freq == 0) return fail(KC_ERR_INVALID, "need 1 <= min_freq <= max_freq");
     const uint64_t bins = (uint64_t)max_freq - min_freq + 1;
     if (bins > (1ull << 26)) return fail(KC_ERR_INVALID, "histogram range too large");
@@ -2409,6 +2420,7 @@ int kc_copy_low(kc_context* c, uint8_t* dst, uint64_t cap) {
     if (cap < bytes) return fail(KC_ERR_INVALID, "destination too small: %llu < %llu", (unsigned long long)cap,
                                  (unsigned long long)bytes);
     if (bytes) {
+        CKR(low_kept(c));
         CK(cudaMemcpyAsync(dst, c->low_packed.p, bytes, cudaMemcpyDefault, c->stream));
         CK(cudaStreamSynchronize(c->stream));
     }
@@ -2474,7 +2486,7 @@ extern "C" int kc_bucket_loads(kc_context* c, uint64_t* distinct, uint64_t* tabl
     if (!c) return fail(KC_ERR_INVALID, "null context");
     if (!c->have_result) return fail(KC_ERR_STATE, "no result: run a count first");
     if (c->batch_result) return fail(KC_ERR_STATE, "not available for a multi-set result");
-    if (c->stream_low) return fail(KC_ERR_STATE, "streamed results are not kept on the device");
+    CKR(low_kept(c));
     CK(c->loads.ensure(3 * KC_MODEL_BUCKETS * sizeof(unsigned long long)));
     unsigned long long* dd = c->loads.as<unsigned long long>();
     CK(cudaMemsetAsync(dd, 0, 3 * KC_MODEL_BUCKETS * sizeof(unsigned long long), c->stream));

@@ -329,6 +329,7 @@ int kc_post_process(kc_context* ctx, const char* out_dir, kc_post_stats* stats) 
     uint64_t low_bytes = 0, R = 0;
     int rc = kc_device_results(ctx, &d_low, &low_bytes, &d_roots, &R);
     if (rc) return rc;
+    if (low_bytes && !d_low) return pfail(KC_ERR_STATE, "streamed results are not kept on the device");
     const uint32_t k = kc_internal_k(ctx);
     const uint64_t P = kc_packed_bytes(k), rec = kc_record_bytes(k);
     cudaStream_t st = static_cast<cudaStream_t>(kc_stream(ctx));
