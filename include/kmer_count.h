@@ -226,6 +226,9 @@ int kc_count_sets(kc_context* ctx, const uint8_t* d_fastq, const kc_set_desc* se
 /* Graph instantiations kc_count_sets has made on this context (a diagnostic:
  * later calls with a shape seen before update and replay its graph). */
 uint64_t kc_sets_graph_instantiations(const kc_context* ctx);
+/* Keys of the last count that left their shared-memory window's estimated range
+ * and were counted by the global kernel (a diagnostic). */
+uint64_t kc_window_spill(const kc_context* ctx);
 
 /* Sizes of the last result: packed low.bin bytes, number of root records,
  * and per-root record counts (256 entries, may be NULL). */

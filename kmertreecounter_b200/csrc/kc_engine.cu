@@ -3158,6 +3158,8 @@ extern "C" int kc_set_prefix_kmers(kc_context* c, const uint8_t* d_fastq, const 
 
 extern "C" uint64_t kc_sets_graph_instantiations(const kc_context* c) { return c ? c->sets_instantiations : 0; }
 
+extern "C" uint64_t kc_window_spill(const kc_context* c) { return c ? c->window_spill : 0; }
+
 extern "C" int kc_set_sizing_callback(kc_context* c, kc_sizing_fn fn, void* user) {
     if (!c) return fail(KC_ERR_INVALID, "null context");
     c->sizing_cb = fn;
