@@ -63,21 +63,22 @@ int fail(int code, const char* fmt, ...) {
 struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
-    // Grow to at least `bytes` (contents not kept).
+    // Grow to at least `bytes` (contents not kept), with an eighth to spare, or a
+    // 64th where the device has no more: sizes that differ a little from call to
+    // call (root records: which keys the filter lets through) find room again.
     cudaError_t ensure(size_t bytes) {
         if (bytes <= cap && p) return cudaSuccess;
-        if (p) cudaFree(p);
-        p = nullptr;
-        cap = 0;
-        size_t want = std::max<size_t>(bytes + bytes / 8, 4096);
-        cudaError_t e = cudaMalloc(&p, want);
-        if (e != cudaSuccess) {
+        release();
+        cudaError_t e = cudaSuccess;
+        for (const size_t spare : {bytes / 8, bytes / 64, (size_t)0}) {
+            const size_t want = std::max<size_t>(bytes + spare, 4096);
+            if ((e = cudaMalloc(&p, want)) == cudaSuccess) {
+                cap = want;
+                return e;
+            }
             cudaGetLastError();
-            e = cudaMalloc(&p, bytes);
-            want = bytes;
+            p = nullptr;
         }
-        if (e == cudaSuccess) cap = want;
-        else p = nullptr;
         return e;
     }
     // Grow keeping the first `keep` bytes.
