@@ -18,14 +18,17 @@
 // 4 of 8 passes for 12 M keys of k = 31, 4 of 16 for k = 63), and the few runs
 // of records that agree in all of those are sorted by the rest of the key
 // where they lie: short runs by a thread, runs up to WARP_RUN by a warp and up
-// to LONG_RUN by a block in shared memory.  Keys with longer runs (many
-// distinct keys behind one long common prefix) take the passes over all digits
-// after all.  11.7 M records of k = 31: 2.20 ms over all digits, 1.35 over four
+// to LONG_RUN by a block in shared memory.  Longer runs (many distinct keys
+// behind one long common prefix, as poly-A tails make) are put together and
+// take the passes over all digits by themselves; where they are many or hold
+// half of the records, all records do.  11.7 M records of k = 31: 2.20 ms over all digits, 1.35 over four
 // and the runs (high-coverage repeats with errors make ~100,000 of them).
 
 #include <algorithm>
 #include <cstdint>
 #include <string>
+#include <utility>
+#include <vector>
 
 #include <cuda_runtime.h>
 
@@ -133,6 +136,8 @@ __global__ void __launch_bounds__(SORT_THREADS) downsweep(const Rec<W>* __restri
 constexpr uint32_t SHORT_RUN = 16;     // records a thread sorts in place
 constexpr uint32_t WARP_RUN = 128;     // records a warp sorts in shared memory
 constexpr uint32_t LONG_RUN = 1024;    // records a block sorts in shared memory
+constexpr uint64_t LONG_LIST = 256;    // longer runs that are sorted apart, one for every 2^16 records at most:
+                                       // a run's two copies cost as much as the passes over so many
 constexpr uint64_t PREFIX_MIN = 1ull << 16;  // smaller sorts are a few launches either way
 
 template <int NW>
@@ -149,7 +154,8 @@ __device__ __forceinline__ bool key_less(const uint64_t* a, const uint64_t* b) {
 struct RunList {
     unsigned long long* warp;   // runs longer than SHORT_RUN, by first record
     unsigned long long* block;  // of these, runs longer than WARP_RUN
-    unsigned long long* count;  // [0], [1]: entries of the lists; [2]: set when a run is longer than LONG_RUN
+    unsigned long long* longer;  // runs longer than LONG_RUN: first record, length (LONG_LIST pairs)
+    unsigned long long* count;   // [0], [1], [2]: entries of the lists ([2] may exceed LONG_LIST)
 };
 
 template <int NW, int W>
@@ -250,7 +256,19 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_long_runs(Rec<W>* __restric
         const uint32_t len = s_len;
         __syncthreads();
         if (len > LONG_RUN) {  // block-uniform
-            if (threadIdx.x == 0) list.count[2] = 1;
+            if (threadIdx.x == 0) {
+                uint64_t lo = i + LONG_RUN, hi = n;  // the last record of the run lies in [lo, hi)
+                while (hi - lo > 1) {
+                    const uint64_t mid = lo + (hi - lo) / 2;
+                    if (r[mid].w[0] >> drop == top) lo = mid;
+                    else hi = mid;
+                }
+                const unsigned long long at = atomicAdd(list.count + 2, 1ull);
+                if (at < LONG_LIST) {
+                    list.longer[2 * at] = i;
+                    list.longer[2 * at + 1] = lo + 1 - i;
+                }
+            }
             continue;
         }
         uint32_t size = 32;
@@ -274,27 +292,54 @@ int sort_impl(void* records, uint64_t n, uint32_t k, const KcSortScratch& w, cud
     const uint32_t lowbit = 64 * NW - key_bits;
     const uint32_t passes = (key_bits + 7) / 8;
     const uint64_t n_tiles = (n + SORT_TILE - 1) / SORT_TILE;
-    const uint64_t hn = (uint64_t)RADIX * n_tiles;
     R* a = static_cast<R*>(records);
     R* tmp = static_cast<R*>(w.tmp);
     uint32_t* hist = static_cast<uint32_t*>(w.hist);
     uint64_t* offs = static_cast<uint64_t*>(w.offs);
     uint64_t* sums = static_cast<uint64_t*>(w.sums);
-    // `count` passes over the digits from bit `bit` on; the result is in `a`
-    auto run = [&](uint32_t bit, uint32_t count) {
-        R *src = a, *dst = tmp;
+    // `count` passes over the digits of `len` records from bit `bit` on; the
+    // result is in `at` (`other`: as many records of scratch)
+    auto run = [&](R* at, R* other, uint64_t len, uint32_t bit, uint32_t count) {
+        const uint64_t tiles = (len + SORT_TILE - 1) / SORT_TILE, hn = (uint64_t)RADIX * tiles;
+        R *src = at, *dst = other;
         for (uint32_t p = 0; p < count; ++p, bit += 8) {
-            upsweep<NW, W><<<n_tiles, SORT_THREADS, 0, st>>>(src, n, bit, hist, n_tiles);
+            upsweep<NW, W><<<tiles, SORT_THREADS, 0, st>>>(src, len, bit, hist, tiles);
             const uint64_t nb = (hn + kc::SCAN_TILE - 1) / kc::SCAN_TILE;
             kc::scan_reduce<uint32_t><<<nb, kc::SCAN_BLOCK, 0, st>>>(hist, hn, sums);
             kc::scan_sums<<<1, kc::SCAN_BLOCK, 0, st>>>(sums, nb, 0, nullptr);
             kc::scan_apply<uint32_t, uint64_t><<<nb, kc::SCAN_BLOCK, 0, st>>>(hist, hn, sums, offs);
-            downsweep<NW, W><<<n_tiles, SORT_THREADS, 0, st>>>(src, dst, n, bit, offs, n_tiles);
+            downsweep<NW, W><<<tiles, SORT_THREADS, 0, st>>>(src, dst, len, bit, offs, tiles);
             std::swap(src, dst);
             *launches += 5;
         }
         cudaError_t e = cudaGetLastError();
-        if (e == cudaSuccess && src != a) e = cudaMemcpyAsync(a, src, n * sizeof(R), cudaMemcpyDeviceToDevice, st);
+        if (e == cudaSuccess && src != at) e = cudaMemcpyAsync(at, src, len * sizeof(R), cudaMemcpyDeviceToDevice, st);
+        return e;
+    };
+    // the listed long runs by the passes over all digits: they lie in the order
+    // of their prefixes, so sorted together each is in its place
+    auto run_longer = [&](const unsigned long long* list, uint64_t count) {
+        std::vector<std::pair<uint64_t, uint64_t>> runs(count);
+        cudaError_t e = cudaMemcpyAsync(runs.data(), list, count * 16, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess) return e;
+        std::sort(runs.begin(), runs.end());
+        uint64_t m = 0;
+        for (const auto& q : runs) m += q.second;
+        if (2 * m > n) return run(a, tmp, n, lowbit, passes);
+        uint64_t at = 0;
+        for (const auto& q : runs) {
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(tmp + at, a + q.first, q.second * sizeof(R), cudaMemcpyDeviceToDevice, st);
+            at += q.second;
+        }
+        if (e == cudaSuccess) e = run(tmp, tmp + m, m, lowbit, passes);
+        at = 0;
+        for (const auto& q : runs) {
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(a + q.first, tmp + at, q.second * sizeof(R), cudaMemcpyDeviceToDevice, st);
+            at += q.second;
+        }
         return e;
     };
     uint32_t need = 8;
@@ -304,10 +349,11 @@ int sort_impl(void* records, uint64_t n, uint32_t k, const KcSortScratch& w, cud
     if (n >= PREFIX_MIN && lead <= 8 && lead < passes) {
         // the lists take the place of the offsets (256 n_tiles words: at most
         // n / 17 runs after the counters) and of the digit counts (128 n_tiles
-        // words: n / 129)
+        // words: n / 129, the longer runs from the middle on)
         unsigned long long* base = reinterpret_cast<unsigned long long*>(offs);
-        const RunList list{base + 8, reinterpret_cast<unsigned long long*>(hist), base};
-        e = run(64 * NW - 8 * lead, lead);
+        unsigned long long* base2 = reinterpret_cast<unsigned long long*>(hist);
+        const RunList list{base + 8, base2, base2 + 64 * n_tiles, base};
+        e = run(a, tmp, n, 64 * NW - 8 * lead, lead);
         if (e == cudaSuccess) e = cudaMemsetAsync(list.count, 0, 8 * sizeof(*base), st);
         if (e == cudaSuccess) {  // (the run kernels index by the counters)
             sort_runs<NW, W><<<(uint32_t)std::min<uint64_t>((n + SORT_THREADS - 1) / SORT_THREADS, 148 * 8),
@@ -320,9 +366,10 @@ int sort_impl(void* records, uint64_t n, uint32_t k, const KcSortScratch& w, cud
         unsigned long long head[3] = {0, 0, 0};
         if (e == cudaSuccess) e = cudaMemcpyAsync(head, list.count, sizeof head, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (e == cudaSuccess && head[2]) e = run(lowbit, passes);
+        if (e == cudaSuccess && head[2])
+            e = head[2] <= std::min(LONG_LIST, n >> 16) ? run_longer(list.longer, head[2]) : run(a, tmp, n, lowbit, passes);
     } else {
-        e = run(lowbit, passes);
+        e = run(a, tmp, n, lowbit, passes);
     }
     if (e != cudaSuccess) {
         g_sort_err = cudaGetErrorString(e);
