@@ -1163,6 +1163,13 @@ def run_reference(args):
     rank, world, _ = dist_env()
     if rank != 0:
         return
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import oracle
+    if not os.path.exists(oracle.REF_TREE):
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "the reference's Tree is not built (oracle/_ref): its sources were absent"}),
+              flush=True)
+        return
     with tempfile.TemporaryDirectory() as wd:
         path, data, k, bases, info = cpu_sample(args.workload, args.sample_scale, wd)
         res, kind, cores = time_reference(path, data, k, bases, max(args.warmup, 0) + args.steps, wd)
