@@ -231,7 +231,7 @@ struct kc_context {
     int sets_exec_key[SETS_EXECS] = {};
     int sets_exec_next = 0;                   // slot a new shape replaces
     uint64_t sets_instantiations = 0;         // times that graph had to be instantiated
-    // windowed count of 64-bit keys (kc_window.cuh): window-grouped keys,
+    // windowed count of 64- and 128-bit keys (kc_window.cuh): window-grouped keys,
     // per-bucket window ids and per-window counts and key ranges
     // KC_WINDOW_COUNT in the environment: 0 = count_routed only, 1 = windows at
     // every size, unset = by the sizes below which they are slower
@@ -685,7 +685,7 @@ int size_structures(kc_context* c, const std::vector<uint64_t>& kb, double scale
         // ~0.33 GB of FASTQ per ms, the initialisation 2-5 GB per ms) it runs
         // on the side stream, two CTAs per SM, after the work already queued
         // on `stream` (a previous count may still read the table), beside
-        // the extraction, which is bound by instruction issue, not by HBM;
+        // the extraction, which is bound by shared memory, not by HBM;
         // the count joins it.  Otherwise it runs first at full width: 48 GB
         // of 128-bit tables behind a 2 GiB batch slowed that batch's
         // extraction and still held up the count.

@@ -193,13 +193,6 @@ KC_HD uint64_t rev_bases(uint64_t x) {
     return ((x >> 1) & 0x5555555555555555ull) | ((x & 0x5555555555555555ull) << 1);
 }
 
-// 2-bit code of an ASCII base: A/a=0 C/c=1 G/g=2 T/t/U/u=3 (src/GetKmer.h:22-37).
-__device__ __forceinline__ uint32_t base_code(uint32_t c) { return ((c >> 1) ^ (c >> 2)) & 3u; }
-__device__ __forceinline__ bool is_base(uint32_t c) {
-    const uint32_t u = c & 0xDFu;  // fold lowercase, as src/FastqParser.h:211-230
-    return u == 'A' || u == 'C' || u == 'G' || u == 'T' || u == 'U';
-}
-
 template <int NW>
 struct KeyOf;
 template <>
@@ -782,8 +775,8 @@ KC_HD void key_of_window(const uint32_t* sw, const StreamPos& p, uint32_t k, uin
 //   (Staging 128-bit keys in 48 KB held 2048 of the 2300 keys of a tile of
 //   150 bp reads at k = 63; the tiles that did not fit built every key twice.)
 //
-// The kernel is bound by instruction issue (the integer pipe), not by its
-// bytes.  Before, each key came from 64-bit shifts and bit reversals of its
+// The kernel is bound by shared memory (l1tex 83%, the integer pipe 65%), not by
+// its bytes.  Before, bound by the integer pipe, each key came from 64-bit shifts and bit reversals of its
 // segment's codes, and tiles walked all their segments: 10 M reads of 150 bp
 // at k = 31 9.5 -> 7.6 ms, 6 M at k = 63 10.4 -> 5.4, 1 M of 250 bp at
 // k = 101 5.2 -> 2.2.

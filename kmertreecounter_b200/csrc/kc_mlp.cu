@@ -1,7 +1,7 @@
 // Sizing model: a small MLP with BF16 weights and FP32 accumulation,
 // trained and run by the project's own kernels.
 //
-//   x (4102 features) -> W1 + b1 -> ReLU -> W2 (512x512) + b2 -> ReLU
+//   x (4104 features) -> W1 + b1 -> ReLU -> W2 (512x512) + b2 -> ReLU
 //   -> W3 (512x8192) + b3 -> y (log1p of predicted distinct keys and table keys
 //   for 4096 buckets)
 //
