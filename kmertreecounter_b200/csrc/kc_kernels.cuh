@@ -97,7 +97,7 @@ constexpr int PROBE_LIMIT = 512;                     // linear-probe bound befor
 // keys are inserted then, so once one key has met a full probe window the
 // others of the bucket need not walk theirs to the end.  100,000 reads at 3x
 // coverage, whose tables fill up: count stage 5.6 ms with every key walking 512
-// cells, 0.76 ms with an early end.
+// cells, 0.70 ms in windows and 0.79 by count_routed with an early end.
 constexpr uint32_t PROBE_CHECK = 32;
 
 // One 128-bit key word pair in the reference's kmer<2> order: w0 = data[0]

@@ -42,7 +42,8 @@
 // 128-bit keys (one device pass, 6 M reads at k = 63, 4096 buckets, 496 M keys;
 // before: the global count, an initialisation beside the extraction, global
 // histogram lookups): sub-routing 5.6 + count 5.7 ms against 12.1, extraction
-// 5.4 -> 4.7, histogram 4.4 -> 2.8; count + histogram 25.0 -> 22.2.
+// 5.4 -> 4.7, histogram 4.4 -> 2.8; count + histogram 25.0 -> 22.2.  Small inputs
+// make too few windows of them: the engine takes them from 42 M keys on.
 #pragma once
 
 #include <cstdint>
